@@ -4,11 +4,13 @@
 // one hash table holds them all.  The lookup hash is GF(2)-linear, so the bucket of a target
 // (p << 40) | (s ^ x) is h(row key) ^ h(x): the probe loop of a row is the single-problem one,
 // only the row's group range, x = 0 group and sector filter come from its problem.
+#include <algorithm>
 #include <string>
 #include <vector>
 
 #include "rq_common.cuh"
 #include "rq_host.h"
+#include "rq_rows.cuh"
 
 namespace rq {
 
@@ -85,19 +87,6 @@ __global__ void k_batch_diag(const uint64_t *__restrict__ keys, int64_t D, const
         }
         out[i] = d;
     }
-}
-
-template <typename R>
-__device__ __forceinline__ cx<R> bgroup_diag(const rq_terms_t &T, int g, uint64_t s) {
-    CAcc<R> d;
-    const int k1 = __ldg(T.toff + g + 1);
-    for (int k = __ldg(T.toff + g); k < k1; ++k) {
-        const R re = (R)__ldg(T.coef + 2 * k), im = (R)__ldg(T.coef + 2 * k + 1);
-        if (re == (R)0 && im == (R)0) break;
-        if (__popcll(s & __ldg(T.zmask + k)) & 1) d.add({-re, -im});
-        else d.add({re, im});
-    }
-    return d.get();
 }
 
 // Line filter of a batch, per problem p (block p): the prefix shift lshift[p] from the highest
@@ -311,7 +300,7 @@ k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
         }
         const uint64_t s = key & kStateMask;
         batch_row_hits(B, htab, act, key, err, [&](int g, int m) {
-            acc.add(cmul(bgroup_diag<R>(B.terms, g, s), VT<V>::ld(x, m)));
+            acc.add(cmul(group_diag<R>(B.terms, g, s), VT<V>::ld(x, m)));
         });
         if (act) VT<V>::st(y, i, acc.get());
     }
@@ -355,23 +344,27 @@ k_batch_conn_fill(const rq_batch_t B, const int64_t *__restrict__ rowptr, int32_
 
 template <typename V>
 __global__ void __launch_bounds__(kThreads)
-k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y,
+k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y, int rows,
                     const int *gate, int64_t gstride, const int *gate2) {
+    using RT = RowTerm<V>;
     using R = typename VT<V>::R;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < B.D;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t key = __ldg(B.keys + i);
-        if (!gate_open(gate, gstride, gate2, problem_of(key))) continue;
-        const uint64_t s = key & kStateMask;
-        CAcc<R> acc;
-        const cx<R> xi = VT<V>::ld(x, i);
-        const R dv = (R)B.diag0[i];
-        acc.add({dv * xi.re, dv * xi.im});
-        const int64_t e1 = B.rowptr[i + 1];
-        for (int64_t e = B.rowptr[i]; e < e1; ++e)
-            acc.add(cmul(bgroup_diag<R>(B.terms, __ldg(B.grp + e), s),
-                         VT<V>::ld(x, __ldg(B.col + e))));
-        VT<V>::st(y, i, acc.get());
+    for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < B.D; r0 += (int64_t)gridDim.x * rows) {
+        const int nr = (int)min((int64_t)rows, B.D - r0);
+        // a tile within one problem that is closed is passed over (every thread sees the same)
+        const int p0 = problem_of(__ldg(B.keys + r0)), p1 = problem_of(__ldg(B.keys + r0 + nr - 1));
+        if (p0 == p1 && !gate_open(gate, gstride, gate2, p0)) continue;
+        tile_product<V>(
+            B.rowptr, r0, nr,
+            [&](int64_t e) {
+                const int m = __ldg(B.col + e), g = __ldg(B.grp + e);
+                const uint64_t key = __ldg(B.keys + m);
+                if (p0 != p1 && !gate_open(gate, gstride, gate2, problem_of(key))) return typename RT::P{};
+                return RT::product(B.terms, g, (key ^ __ldg(B.terms.xmask + g)) & kStateMask, x, m);
+            },
+            [&](int64_t i, typename RT::A &acc) { acc.add(RT::scaled((R)B.diag0[i], x, i)); },
+            [&](int64_t i, const typename RT::A &acc) {
+                if (p0 == p1 || gate_open(gate, gstride, gate2, problem_of(__ldg(B.keys + i)))) RT::store(y, i, acc);
+            });
     }
 }
 
@@ -389,8 +382,10 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
     } else if (B.mode == RQ_MODE_CONN) {
         if (!B.rowptr || (B.nnz > 0 && (!B.col || !B.grp)))
             return fail(RQ_E_ARG, "rq_batch_matvec: RQ_MODE_CONN needs rowptr, col and grp");
-        k_batch_matvec_conn<V><<<grid_rows(B.D), kThreads, 0, st>>>(
-            B, static_cast<const V *>(x), static_cast<V *>(y), gate, gstride, gate2);
+        const int rows = tile_rows<V>(B.D, B.nnz, sm_count());
+        const int64_t tiles = (B.D + rows - 1) / rows, cap = (int64_t)sm_count() * 8;
+        k_batch_matvec_conn<V><<<(int)std::min(tiles, cap), kThreads, 0, st>>>(
+            B, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gstride, gate2);
     } else {
         return fail(RQ_E_ARG, "rq_batch_matvec: mode must be RQ_MODE_FREE or RQ_MODE_CONN");
     }

@@ -640,39 +640,85 @@ __global__ void k_scan_add(int64_t *v, int64_t n, const int64_t *boff) {
     }
 }
 
+int grid_rows(int64_t n) {
+    int64_t g = (n + kThreads - 1) / kThreads;
+    const int64_t cap = (int64_t)sm_count() * 8;
+    return (int)(g > cap ? cap : (g < 1 ? 1 : g));
+}
+
+// blocks of the tiled cached products: 8 resident per SM (17 KB of shared memory, 32 registers)
+int grid_tiles(int64_t D, int rows) {
+    const int64_t g = (D + rows - 1) / rows, cap = (int64_t)sm_count() * 8;
+    return (int)(g > cap ? cap : g);
+}
+
 // ------------------------------------------------------------------------------------------
 // CONN and CSR modes
 // ------------------------------------------------------------------------------------------
+// Element e of group g with source row m belongs to the row of state S[m] ^ x_g, so an element
+// needs no search for its row.
 template <typename V>
 __global__ void __launch_bounds__(kThreads)
-k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, const int *gate,
+k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int rows, const int *gate,
               const int *gate2) {
-    d_matvec_conn<V>(op, x, y, gate, gate2);
+    using RT = RowTerm<V>;
+    using R = typename VT<V>::R;
+    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
+    const rq_terms_t &T = op.terms;
+    const int64_t D = op.sub.D;
+    for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
+        tile_product<V>(
+            op.rowptr, r0, (int)min((int64_t)rows, D - r0),
+            [&](int64_t e) {
+                const int m = __ldg(op.col + e), g = __ldg(op.grp + e);
+                return RT::product(T, g, __ldg(op.sub.states + m) ^ __ldg(T.xmask + g), x, m);
+            },
+            [&](int64_t i, typename RT::A &acc) {
+                if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+                else if (T.diag_group >= 0) acc.add(RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
+            },
+            [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); });
 }
 
 // VV: storage type of the element values (converted to the vector's precision on load)
 template <typename V, typename VV>
 __global__ void __launch_bounds__(kThreads)
-k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, const int *gate,
+k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int rows, const int *gate,
              const int *gate2) {
-    d_matvec_csr<V, VV>(op, x, y, gate, gate2);
+    using RT = RowTerm<V>;
+    using R = typename VT<V>::R;
+    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
+    const VV *val = reinterpret_cast<const VV *>(op.val);
+    const int64_t D = op.sub.D;
+    for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
+        tile_product<V>(
+            op.rowptr, r0, (int)min((int64_t)rows, D - r0),
+            [&](int64_t e) {
+                const auto v = VT<VV>::ld(val, e);
+                return RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e));
+            },
+            [&](int64_t i, typename RT::A &acc) {
+                if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+            },
+            [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); });
 }
 
 template <typename V>
-int launch_csr(const rq_operator_t &op, const void *x, void *y, cudaStream_t st, const int *gate,
-               const int *gate2, int grid) {
+int launch_csr(const rq_operator_t &op, const void *x, void *y, cudaStream_t st, const int *gate, const int *gate2) {
     const V *xx = static_cast<const V *>(x);
     V *yy = static_cast<V *>(y);
+    const int rows = tile_rows<V>(op.sub.D, op.nnz, sm_count());
+    const int grid = grid_tiles(op.sub.D, rows);
     switch (op.val_vtype) {
-        case RQ_F32: k_matvec_csr<V, float><<<grid, kThreads, 0, st>>>(op, xx, yy, gate, gate2); break;
-        case RQ_F64: k_matvec_csr<V, double><<<grid, kThreads, 0, st>>>(op, xx, yy, gate, gate2); break;
+        case RQ_F32: k_matvec_csr<V, float><<<grid, kThreads, 0, st>>>(op, xx, yy, rows, gate, gate2); break;
+        case RQ_F64: k_matvec_csr<V, double><<<grid, kThreads, 0, st>>>(op, xx, yy, rows, gate, gate2); break;
         case RQ_C64:
             if (!VT<V>::kComplex) return fail(RQ_E_ARG, "rq_matvec: complex CSR values need complex vectors");
-            k_matvec_csr<V, float2><<<grid, kThreads, 0, st>>>(op, xx, yy, gate, gate2);
+            k_matvec_csr<V, float2><<<grid, kThreads, 0, st>>>(op, xx, yy, rows, gate, gate2);
             break;
         case RQ_C128:
             if (!VT<V>::kComplex) return fail(RQ_E_ARG, "rq_matvec: complex CSR values need complex vectors");
-            k_matvec_csr<V, double2><<<grid, kThreads, 0, st>>>(op, xx, yy, gate, gate2);
+            k_matvec_csr<V, double2><<<grid, kThreads, 0, st>>>(op, xx, yy, rows, gate, gate2);
             break;
         default: return fail(RQ_E_ARG, "rq_matvec: bad val_vtype");
     }
@@ -744,12 +790,6 @@ int launch_free(const rq_operator_t &op, const void *x, void *y, int stop_at_zer
     return RQ_OK;
 }
 
-int grid_rows(int64_t n) {
-    int64_t g = (n + kThreads - 1) / kThreads;
-    const int64_t cap = (int64_t)sm_count() * 8;
-    return (int)(g > cap ? cap : (g < 1 ? 1 : g));
-}
-
 template <typename V>
 int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch, cudaStream_t st,
                  const int *gate, const int *gate2) {
@@ -782,8 +822,11 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
         case RQ_MODE_CONN:
             if (!op.rowptr || (op.nnz > 0 && (!op.col || !op.grp)))
                 return fail(RQ_E_ARG, "rq_matvec: RQ_MODE_CONN needs rowptr, col and grp");
-            k_matvec_conn<V><<<grid_rows(op.sub.D), kThreads, 0, st>>>(
-                op, static_cast<const V *>(x), static_cast<V *>(y), gate, gate2);
+            {
+                const int rows = tile_rows<V>(op.sub.D, op.nnz, sm_count());
+                k_matvec_conn<V><<<grid_tiles(op.sub.D, rows), kThreads, 0, st>>>(
+                    op, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gate2);
+            }
             RQ_CUDA(cudaGetLastError());
             return RQ_OK;
         case RQ_MODE_CSR:
@@ -791,7 +834,7 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
                 return fail(RQ_E_ARG, "rq_matvec: RQ_MODE_CSR needs rowptr, col and val");
             if (op.terms.diag_group >= 0 && !op.diag0)
                 return fail(RQ_E_ARG, "rq_matvec: RQ_MODE_CSR needs diag0 when a diagonal group exists");
-            return launch_csr<V>(op, x, y, st, gate, gate2, grid_rows(op.sub.D));
+            return launch_csr<V>(op, x, y, st, gate, gate2);
         default:
             return fail(RQ_E_ARG, "rq_matvec: unknown mode");
     }

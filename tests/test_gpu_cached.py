@@ -1,0 +1,59 @@
+"""The tiled cached products (CONN, CSR): the same additions in the same order as the matrix-free
+product, so the same bits, at the edges of the tiles (rows per block, products per pass)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module', autouse=True)
+def built():
+    from rqutils_gb300._build import build
+    build()
+
+
+def _operators(n, K, D, real, seed):
+    from rqutils_gb300 import workloads
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    from rqutils_gb300.sqd import SQDProblem
+    rng = np.random.default_rng(seed)
+    labels, coeffs = workloads.random_pauli_masks(rng, n, K, locality=(1, n))
+    if real:  # an even number of Y per term
+        labels = [s if s.count('Y') % 2 == 0 else s.replace('Y', 'X') for s in labels]
+    ham = PauliSumXZ.from_paulisum((labels, coeffs), force_real=True, add_padding=True)
+    S = np.sort(rng.choice(1 << n, size=D, replace=False)).astype(np.uint64)
+    return [SQDProblem(ham, S, cache_level=c).op for c in ((0, 0), (1, 0), (1, 2))]
+
+
+# D around the tile heights (16 to 256 rows), row lists from empty (sparse subspace) to several
+# passes over the product buffer (a 10-qubit space with 900 groups: ~900 elements per row)
+@pytest.mark.parametrize('n,K,D', [(1, 2, 1), (3, 5, 7), (10, 1500, 1024), (12, 200, 15), (12, 200, 17),
+                                   (14, 300, 4863), (14, 300, 4864), (14, 300, 4865), (30, 60, 5000),
+                                   (18, 400, 200001)])
+@pytest.mark.parametrize('dtype', ['float32', 'float64', 'complex64', 'complex128'])
+def test_cached_products_equal_matrix_free_bits(n, K, D, dtype):
+    import torch
+    free, conn, csr = _operators(n, K, D, dtype.startswith('float'), 100 * n + D % 97)
+    x = torch.randn(D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(D))
+    y = free.matvec(x)
+    assert torch.equal(conn.matvec(x), y)
+    # cached elements are computed in 64 bits; a 32-bit vector rounds them after their sum
+    z = csr.matvec(x)
+    if dtype in ('float64', 'complex128'):
+        assert torch.equal(z, y)
+    else:
+        ref = csr.matvec(x.to(torch.float64 if dtype == 'float32' else torch.complex128))
+        assert torch.linalg.vector_norm(z - ref) <= 1e-6 * torch.linalg.vector_norm(ref)
+
+
+@pytest.mark.parametrize('mode', [1, 2])
+def test_cached_products_keep_infinities_and_nan(mode):
+    """Non-finite entries reach the rows connected to them and no others."""
+    import torch
+    ops = _operators(12, 80, 700, True, 5)
+    x = torch.randn(700, dtype=torch.float64, device='cuda', generator=torch.Generator('cuda').manual_seed(1))
+    x[3], x[10] = float('inf'), float('nan')
+    y, z = ops[0].matvec(x), ops[mode].matvec(x)
+    assert torch.equal(torch.isfinite(y), torch.isfinite(z))
+    ok = torch.isfinite(y)
+    assert torch.equal(y[ok], z[ok])
