@@ -348,7 +348,7 @@ __device__ __forceinline__ cdf cdf_zero() { return {{0.f, 0.f}, {0.f, 0.f}}; }
 __device__ __forceinline__ float4 cdf_pack(cdf a) { return make_float4(a.re.hi, a.re.lo, a.im.hi, a.im.lo); }
 __device__ __forceinline__ cdf cdf_unpack(float4 v) { return {{v.x, v.y}, {v.z, v.w}}; }
 
-// Block-wide sums of NV <= 8 values, left in tot[0..NV) (shared memory) for every thread.
+// Block-wide sums of NV <= 16 values, left in tot[0..NV) (shared memory) for every thread.
 // Within a warp the values are reduce-scattered: at each of the first log2(P) butterfly steps
 // (P = NV rounded up to a power of two) a lane keeps half of its values and receives the
 // partner's partial sums of that half, so a lane adds P - 1 + (5 - log2 P) pairs instead of
@@ -357,8 +357,8 @@ __device__ __forceinline__ cdf cdf_unpack(float4 v) { return {{v.x, v.y}, {v.z, 
 // the same inputs.
 template <int NV>
 __device__ __forceinline__ void block_sum_all(cdf (&w)[NV], cdf *tot, cdf (*red)[NV]) {
-    static_assert(NV >= 1 && NV <= 8, "block_sum_all: at most 8 values");
-    constexpr int L = NV <= 1 ? 0 : NV <= 2 ? 1 : NV <= 4 ? 2 : 3;  // halving steps
+    static_assert(NV >= 1 && NV <= 16, "block_sum_all: at most 16 values");
+    constexpr int L = NV <= 1 ? 0 : NV <= 2 ? 1 : NV <= 4 ? 2 : NV <= 8 ? 3 : 4;  // halving steps
     constexpr int P = 1 << L;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarp = (blockDim.x + 31) >> 5;

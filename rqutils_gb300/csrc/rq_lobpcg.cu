@@ -745,6 +745,43 @@ __global__ void __launch_bounds__(kThreads) k_convert(int64_t D, const VS *a, VD
     for (int p_ = first; p_ < (P); p_ += step)                                     \
         for (State *st = (states) + p_; st != nullptr && st->active; st = nullptr)
 
+// ------------------------------------------------------------------------------------------
+// scalars of the 3x3 problem: double for real vectors, double2 for complex ones
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ double s_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ double2 s_mul(double2 a, double2 b) {
+    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double s_add(double a, double b) { return a + b; }
+__device__ __forceinline__ double2 s_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double s_scale(double f, double a) { return f * a; }
+__device__ __forceinline__ double2 s_scale(double f, double2 a) { return make_double2(f * a.x, f * a.y); }
+__device__ __forceinline__ double s_conj(double a) { return a; }
+__device__ __forceinline__ double2 s_conj(double2 a) { return make_double2(a.x, -a.y); }
+__device__ __forceinline__ double s_re(double a) { return a; }
+__device__ __forceinline__ double s_re(double2 a) { return a.x; }
+__device__ __forceinline__ double s_abs2(double a) { return a * a; }
+__device__ __forceinline__ double s_abs2(double2 a) { return a.x * a.x + a.y * a.y; }
+// Re(conj(a) b)
+__device__ __forceinline__ double s_rdot(double a, double b) { return a * b; }
+__device__ __forceinline__ double s_rdot(double2 a, double2 b) { return a.x * b.x + a.y * b.y; }
+__device__ __forceinline__ double2 s_pair(double a) { return make_double2(a, 0.); }
+__device__ __forceinline__ double2 s_pair(double2 a) { return a; }
+template <typename R>
+__device__ __forceinline__ double s_round(double a) { return (double)(R)a; }
+template <typename R>
+__device__ __forceinline__ double2 s_round(double2 a) { return make_double2((double)(R)a.x, (double)(R)a.y); }
+template <typename R>
+__device__ __forceinline__ cx<R> s_coef(double a) { return {(R)a, (R)0}; }
+template <typename R>
+__device__ __forceinline__ cx<R> s_coef(double2 a) { return {(R)a.x, (R)a.y}; }
+template <typename S>
+__device__ __forceinline__ S s_of(double re);
+template <>
+__device__ __forceinline__ double s_of<double>(double re) { return re; }
+template <>
+__device__ __forceinline__ double2 s_of<double2>(double re) { return make_double2(re, 0.); }
+
 // Lowest eigenpair of a Hermitian 3x3 given by its strict lower triangle (m10, m20, m21) and its
 // diagonal (complex values, real part used as in ground_locg.py:446); Cardano (Kopp 2008).
 // Smallest root of lambda^3 + c2 lambda^2 + c1 lambda + c0 (three real roots) without FP64
@@ -791,20 +828,18 @@ __device__ __forceinline__ bool cubic_min_root_fast(double c2, double c1, double
     return false;
 }
 
-__device__ void eig3(double2 m10, double2 m20, double2 m21, double2 m00, double2 m11, double2 m22,
-                     double &lam, double2 (&v)[3], bool guard = false, bool fast = false) {
-    const double d0 = m00.x, d1 = m11.x, d2 = m22.x;
-    const double a10 = m10.x * m10.x + m10.y * m10.y;
-    const double a20 = m20.x * m20.x + m20.y * m20.y;
-    const double a21 = m21.x * m21.x + m21.y * m21.y;
+template <typename S>
+__device__ void eig3(S m10, S m20, S m21, S m00, S m11, S m22, double &lam, S (&v)[3], bool guard = false,
+                     bool fast = false) {
+    const double d0 = s_re(m00), d1 = s_re(m11), d2 = s_re(m22);
+    const double a10 = s_abs2(m10), a20 = s_abs2(m20), a21 = s_abs2(m21);
     const double c2 = -(d0 + d1 + d2);
     const double c1 = (d0 * d2 + d1 * d0 + d2 * d1) - (a10 + a20 + a21);
     double c0 = d0 * a21 + d1 * a20 + d2 * a10;
     c0 -= d0 * d1 * d2;
     // Re(m02 m10 m21) with m02 = conj(m20)
-    const double2 m02 = make_double2(m20.x, -m20.y);
-    const double2 t = make_double2(m02.x * m10.x - m02.y * m10.y, m02.x * m10.y + m02.y * m10.x);
-    c0 -= 2. * (t.x * m21.x - t.y * m21.y);
+    const S m02 = s_conj(m20);
+    c0 -= 2. * s_re(s_mul(s_mul(m02, m10), m21));
     const double p = c2 * c2 - 3. * c1;
     const double q = -13.5 * c0 - c2 * c2 * c2 + 4.5 * c2 * c1;
     // divisions by 3 as products with 1/3 (GB300 runs an FP64 division as a long FP64 sequence
@@ -821,36 +856,32 @@ __device__ void eig3(double2 m10, double2 m20, double2 m21, double2 m00, double2
         lam = sqrt(p) * kThird * xmin - c2 * kThird;
     }
     // columns 1 and 2 of (A - lambda I): a = (m01, m11 - l, m21), b = (m02, m12, m22 - l)
-    const double2 a0 = make_double2(m10.x, -m10.y), a1 = make_double2(m11.x - lam, m11.y), a2 = m21;
-    const double2 b0 = m02, b1 = make_double2(m21.x, -m21.y), b2 = make_double2(m22.x - lam, m22.y);
-    auto mul = [](double2 u, double2 w) {
-        return make_double2(u.x * w.x - u.y * w.y, u.x * w.y + u.y * w.x);
-    };
-    auto sub = [](double2 u, double2 w) { return make_double2(u.x - w.x, u.y - w.y); };
-    double2 c[3] = {sub(mul(a1, b2), mul(a2, b1)), sub(mul(a2, b0), mul(a0, b2)),
-                    sub(mul(a0, b1), mul(a1, b0))};
+    const S ml = s_of<S>(-lam);
+    const S a0 = s_conj(m10), a1 = s_add(m11, ml), a2 = m21;
+    const S b0 = m02, b1 = s_conj(m21), b2 = s_add(m22, ml);
+    auto cross = [](S u, S w, S t, S z) { return s_add(s_mul(u, w), s_scale(-1., s_mul(t, z))); };  // u w - t z
+    S c[3] = {cross(a1, b2, a2, b1), cross(a2, b0, a0, b2), cross(a0, b1, a1, b0)};
     double nrm = 0.;
     for (int k = 0; k < 3; ++k) {
-        c[k].y = -c[k].y;  // conjugate
-        nrm += c[k].x * c[k].x + c[k].y * c[k].y;
+        c[k] = s_conj(c[k]);
+        nrm += s_abs2(c[k]);
     }
     nrm = sqrt(nrm);
     if (guard && !(nrm > 0. && isfinite(nrm)) && isfinite(lam)) {
         // columns 1 and 2 of (A - lambda I) are parallel (or zero): the eigenvector is
         // orthogonal to the other column pairs; take the larger of their cross products
-        const double2 z0 = make_double2(m00.x - lam, m00.y);
-        const double2 col0[3] = {z0, m10, m20};
-        const double2 col1[3] = {a0, a1, a2};
-        const double2 col2[3] = {b0, b1, b2};
+        const S z0 = s_add(m00, ml);
+        const S col0[3] = {z0, m10, m20};
+        const S col1[3] = {a0, a1, a2};
+        const S col2[3] = {b0, b1, b2};
         double best = 0.;
         for (int pair = 0; pair < 2; ++pair) {
-            const double2 *u = col0, *w = pair == 0 ? col1 : col2;
-            double2 e[3] = {sub(mul(u[1], w[2]), mul(u[2], w[1])), sub(mul(u[2], w[0]), mul(u[0], w[2])),
-                            sub(mul(u[0], w[1]), mul(u[1], w[0]))};
+            const S *u = col0, *w = pair == 0 ? col1 : col2;
+            S e[3] = {cross(u[1], w[2], u[2], w[1]), cross(u[2], w[0], u[0], w[2]), cross(u[0], w[1], u[1], w[0])};
             double n2 = 0.;
             for (int k = 0; k < 3; ++k) {
-                e[k].y = -e[k].y;
-                n2 += e[k].x * e[k].x + e[k].y * e[k].y;
+                e[k] = s_conj(e[k]);
+                n2 += s_abs2(e[k]);
             }
             if (n2 > best && isfinite(n2)) {
                 best = n2;
@@ -859,13 +890,13 @@ __device__ void eig3(double2 m10, double2 m20, double2 m21, double2 m00, double2
         }
         nrm = sqrt(best);
         if (!(nrm > 0.)) {  // A = lambda I on the span: any vector; keep x
-            c[0] = make_double2(1., 0.);
-            c[1] = c[2] = make_double2(0., 0.);
+            c[0] = s_of<S>(1.);
+            c[1] = c[2] = s_of<S>(0.);
             nrm = 1.;
         }
     }
     const double inv = 1. / nrm;
-    for (int k = 0; k < 3; ++k) v[k] = make_double2(c[k].x * inv, c[k].y * inv);
+    for (int k = 0; k < 3; ++k) v[k] = s_scale(inv, c[k]);
 }
 
 __device__ __forceinline__ void d_rr3(State *states, int P, int first, int step) {
@@ -916,12 +947,9 @@ __global__ void k_clear_slot(State *states, int P, int slot) {
 
 // iteration 0: rho = Re <x, Ax> into red[kMisc] (already there from k_dots); nothing else.
 
-// Convergence test of ground_locg.py:329-334 and phase bookkeeping; a problem that stops
-// decrements the count of active problems.
-__device__ __forceinline__ void d_check(State *states, int P, int *nactive, int first, int step) {
-    FOR_ACTIVE_PROBLEMS(states, P, st) {
-    const double rn = sqrt(st->red[kRn].x);
-    const double an = sqrt(st->red[kAxn].x);
+// Convergence test of ground_locg.py:329-334 and phase bookkeeping on rn = |r|, an = |Ax|; a problem
+// that stops decrements the count of active problems.
+__device__ __forceinline__ void check_state(State *st, double rn, double an, int *nactive) {
     const double th = st->theta;
     st->resnorm = rn;
     st->axnorm = an;
@@ -961,7 +989,11 @@ __device__ __forceinline__ void d_check(State *states, int P, int *nactive, int 
         st->active = 0;
         if (nactive) atomicSub(nactive, 1);
     }
-    break;
+}
+__device__ __forceinline__ void d_check(State *states, int P, int *nactive, int first, int step) {
+    FOR_ACTIVE_PROBLEMS(states, P, st) {
+        check_state(st, sqrt(st->red[kRn].x), sqrt(st->red[kAxn].x), nactive);
+        break;
     }
 }
 __global__ void k_check(State *states, int P, int *nactive) {
@@ -1316,368 +1348,61 @@ int run_loop(PH &ph, int variant, bool use_graph, int chunk, cudaStream_t s, int
     return rc;
 }
 
-// ------------------------------------------------------------------------------------------
-// Persistent LOBPCG: one cooperative launch runs a phase's iterations to convergence.  The passes
-// are the same device bodies as the kernels above, separated by a grid barrier instead of a
-// kernel boundary (a launch and its drain cost more than the work of a pass at D <= 2^20).
-// ------------------------------------------------------------------------------------------
-constexpr long long kBarrierCycles = 4000000000LL;  // ~2 s at 2 GHz: a barrier that waits longer aborts
+#include "rq_persist.cuh"
 
-// Grid barrier on a counter that only grows: each block adds 1 without waiting for the old value
-// (the adds pipeline in L2 instead of queueing for their results) and waits until the counter
-// reaches (barriers passed) x (blocks); `passed` is the block's own count, kept in shared
-// memory.  Every wait is bounded; a block that gives up raises `abort`, which releases every
-// other waiter at once.  Returns false after an abort.
-__device__ bool group_sync(GridBar *b, unsigned int *passed, unsigned int nblocks) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned int target = (*passed + 1u) * nblocks;
-        *passed += 1u;
-        volatile unsigned int *count = &b->count;
-        volatile int *abort = &b->abort;
-        __threadfence();
-        atomicAdd(&b->count, 1u);
-        const long long t0 = clock64();
-        while ((int)(*count - target) < 0) {
-            if (*abort) {
-                ok = 0;
-                break;
-            }
-            if (clock64() - t0 > kBarrierCycles) {
-                atomicExch(&b->abort, 1);
-                ok = 0;
-                break;
-            }
-        }
-        __threadfence();
-        if (*abort) ok = 0;
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s != 0;
+constexpr size_t kPersistMaxDyn = 212 * 1024;       // of the SM's 227 KB, beside the static part
+constexpr size_t kPersistBatchDyn = 96 * 1024;      // two blocks per SM
+
+// Blocks of a single problem: one per SM, fewer when a block would have less than 1024 list elements
+// (a row counting for 8): the barriers of a small problem cost more than its work.
+int persist_grid(int64_t D, int64_t nnz) {
+    const int64_t g = (nnz + 8 * D + 1023) / 1024;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(g, std::min(sm_count(), kMaxReduceBlocks / 4)));
 }
 
-// Barrier over the whole grid.
-__device__ __forceinline__ bool grid_sync(GridBar *b, unsigned int *passed) {
-    return group_sync(b, passed, gridDim.x);
-}
-
-// One problem inside the persistent kernel: every block holds its own copy of the solver state
-// in shared memory.  A reduction writes the block's partial sums, crosses one grid barrier and
-// then every block adds all partials itself in the same order, so the copies stay identical
-// without a second barrier; scalar steps run on each block's thread 0.  Element i is always
-// handled by the same thread, so passes that only touch a thread's own elements need no barrier.
-struct SegPersist {
-    State *st;      // this block's shared-memory copy
-    int64_t D;
-    float4 *part;   // [2][gridDim.x * kMaxReduce] partial sums, alternate reductions alternate
-                    // halves (a block may write the next sums while another still reads these)
-    GridBar *bar;
-    int *flip;      // shared: which half the next reduction uses
-    unsigned int *passed;  // shared: barriers this block has passed
-    __device__ __forceinline__ State *state() const { return st; }
-    __device__ __forceinline__ int64_t begin() const {
-        return blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+template <typename V, bool FAST>
+int launch_persist(const PersistArgs<V> &args, int grid, size_t dyn, cudaStream_t s, bool *fits) {
+    thread_local KernelLaunchCache table[kMaxCachedDevices];
+    KernelLaunchCache *c = nullptr;
+    RQ_TRY(cache_slot(table, &c));
+    auto kern = k_persist<V, FAST>;
+    if (dyn > c->configured) {
+        RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+        c->configured = dyn;
     }
-    __device__ __forceinline__ int64_t end() const { return D; }
-    __device__ __forceinline__ int64_t stride() const { return (int64_t)gridDim.x * blockDim.x; }
-    template <int NV>
-    __device__ void reduce(cdf (&v)[NV], int slot) const {
-        __shared__ cdf red[kThreads / 32][NV];
-        __shared__ cdf tot[NV];
-        cdf w[NV];
-        float4 *pb = part + (size_t)(*flip) * gridDim.x * kMaxReduce;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) w[k] = v[k];
-        block_sum_all<NV>(w, tot, red);
-        if (threadIdx.x < NV) {
-            pb[(size_t)blockIdx.x * kMaxReduce + threadIdx.x] = cdf_pack(tot[threadIdx.x]);
-            __threadfence();
-        }
-        if (!grid_sync(bar, passed)) {
-            if (threadIdx.x == 0) st->active = 0;  // aborted: every block stops
-            __syncthreads();
-            return;
-        }
-        partials_sum<NV>(pb, (int)gridDim.x, kMaxReduce, tot);
-        if (threadIdx.x < NV) st->red[slot + threadIdx.x] = cdf_val(tot[threadIdx.x]);
-        if (threadIdx.x == 0) *flip ^= 1;
-        __syncthreads();
-    }
-};
-
-// One problem of a batch inside the persistent batched kernel: blocks [b0, b0 + nb) of the grid
-// (this block is number lb of them) own the problem's rows [r0, r1), reduce into the problem's
-// own partial sums and cross the problem's own barrier; otherwise as SegPersist.
-struct SegPersistB {
-    State *st;
-    int64_t r0, r1;
-    int lb, nb;
-    float4 *part;           // [2][nb * kMaxReduce]
-    GridBar *bar;
-    int *flip;
-    unsigned int *passed;
-    __device__ __forceinline__ State *state() const { return st; }
-    __device__ __forceinline__ int64_t begin() const {
-        return r0 + (int64_t)lb * blockDim.x + threadIdx.x;
-    }
-    __device__ __forceinline__ int64_t end() const { return r1; }
-    __device__ __forceinline__ int64_t stride() const { return (int64_t)nb * blockDim.x; }
-    template <int NV>
-    __device__ void reduce(cdf (&v)[NV], int slot) const {
-        __shared__ cdf red[kThreads / 32][NV];
-        __shared__ cdf tot[NV];
-        cdf w[NV];
-        float4 *pb = part + (size_t)(*flip) * nb * kMaxReduce;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) w[k] = v[k];
-        block_sum_all<NV>(w, tot, red);
-        if (threadIdx.x < NV) {
-            pb[(size_t)lb * kMaxReduce + threadIdx.x] = cdf_pack(tot[threadIdx.x]);
-            __threadfence();
-        }
-        if (!group_sync(bar, passed, (unsigned int)nb)) {
-            if (threadIdx.x == 0) st->active = 0;
-            __syncthreads();
-            return;
-        }
-        partials_sum<NV>(pb, nb, kMaxReduce, tot);
-        if (threadIdx.x < NV) st->red[slot + threadIdx.x] = cdf_val(tot[threadIdx.x]);
-        if (threadIdx.x == 0) *flip ^= 1;
-        __syncthreads();
-    }
-};
-
-template <typename V>
-struct PersistArgs {
-    State *st;      // global state (read at start, written back by block 0 at the end)
-    int64_t D;
-    float4 *part;
-    rq_operator_t op;
-    Vecs<V> v;
-    int variant;
-    int jacobi;
-    const double *diag;
-    GridBar *bar;
-};
-
-// MVK 0: cached connectivity, 1: CSR with values of type V
-template <typename V, int MVK>
-__device__ __forceinline__ void persist_mv(const PersistArgs<V> &a, State *st, const V *in, V *out,
-                                           const int *gate2) {
-    if (MVK == 0)
-        d_matvec_conn<V>(a.op, in, out, &st->active, gate2);
-    else
-        d_matvec_csr<V, V>(a.op, in, out, &st->active, gate2);
-}
-
-// The iterations of one phase inside a persistent kernel (ground_locg.py:288-341): the passes
-// of Phase::iteration, separated by barriers of the segment instead of kernel boundaries.
-// mv(in, out, gate2) forms a product over the segment's rows; sync() crosses the segment's
-// barrier and returns false after an abort; the loop also ends at iteration stop_iter.  Element
-// i is always handled by the same thread, so passes that only touch a thread's own elements need
-// no barrier; barriers stand before the products (which gather rows of other blocks) and inside
-// every reduction.
-template <typename V, typename SEG, typename MVF, typename SYNC>
-__device__ __forceinline__ void persist_loop(const SEG &seg, State *st, const Vecs<V> &v,
-                                             int variant, int jacobi, const double *diag, MVF &mv,
-                                             SYNC &sync, int stop_iter) {
-    constexpr int kOnce = 1 << 30;  // step of the scalar loops: thread 0 only
-    auto scalar_done = [&]() { __syncthreads(); };
-    while (st->active && st->iter < stop_iter) {
-        V *src = v.r;
-        if (jacobi) {
-            d_jacobi<V, SEG>(seg, diag, v.r, v.w);
-            src = v.w;
-        }
-        // project_out((x, y), src) -> p
-        if (variant == RQ_LOBPCG_FAST) {
-            Pairs<V, 6> g{{v.x, v.y, v.x, v.x, v.y, src}, {src, src, v.x, v.y, v.y, src}};
-            d_dots<V, 6, SEG>(seg, g, kG10);
-            if (threadIdx.x == 0) d_proj_coef(st, 1, 0, kOnce);
-            scalar_done();
-            d_sub2_scale<V, SEG>(seg, v.x, v.y, src, v.p);
-        } else {
-            Pairs<V, 2> pr{{v.x, v.y}, {src, src}};
-            d_dots<V, 2, SEG>(seg, pr, kIp0);
-            d_sub2_norm<V, SEG>(seg, v.x, v.y, src);
-            d_scale_dots2<V, SEG>(seg, v.x, v.y, src, 1);
-            d_sub2_norm<V, SEG>(seg, v.x, v.y, src);
-            d_scale_dots2<V, SEG>(seg, v.x, v.y, src, 1);
-            d_sub2_norm<V, SEG>(seg, v.x, v.y, src);
-            d_scale_dots2<V, SEG>(seg, v.x, v.y, src, 0);
-            d_sub2_norm<V, SEG>(seg, v.x, v.y, src);
-            d_mask<V, SEG>(seg, src, v.p);
-        }
-        if (!sync()) break;  // the products gather p (and x, y) from every block's rows
-        if (variant == RQ_LOBPCG_REFERENCE) {
-            mv(v.x, v.ax, nullptr);
-            mv(v.y, v.ay, nullptr);
-        }
-        mv(v.p, v.ap, nullptr);
-        d_gram3<V, SEG>(seg, v.x, v.y, v.p, v.ax, v.ay, v.ap);
-        if (threadIdx.x == 0) d_rr3(st, 1, 0, kOnce);
-        scalar_done();
-        if (variant == RQ_LOBPCG_FAST) {
-            d_upd_stu<V, SEG>(seg, v.x, v.y, v.p);
-            if (threadIdx.x == 0) d_stu_coef(st, 1, 0, kOnce);
-            scalar_done();
-        } else {
-            d_upd_s<V, SEG>(seg, v.y, v.p);
-            d_upd_tu<V, SEG>(seg, v.x, v.y, v.p);
-        }
-        if (variant == RQ_LOBPCG_REFERENCE) {
-            d_upd_xy<V, false, SEG>(seg, v.x, v.y, v.p, nullptr, nullptr, nullptr);
-            if (!sync()) break;
-            mv(v.x, v.ax, nullptr);
-        } else {
-            d_upd_xy<V, true, SEG>(seg, v.x, v.y, v.p, v.ax, v.ay, v.ap);
-            if (st->want_refresh) {
-                if (!sync()) break;
-                mv(v.x, v.ax, &st->want_refresh);
-                mv(v.y, v.ay, &st->want_refresh);
-                if (threadIdx.x == 0) d_refresh_mark(st, 1, 0, kOnce);
-                scalar_done();
-            }
-        }
-        d_resid<V, SEG>(seg, v.ax, v.x, v.r, 0);
-        if (threadIdx.x == 0) d_check(st, 1, nullptr, 0, kOnce);
-        scalar_done();
-    }
-}
-
-template <typename V, int MVK>
-__global__ void __launch_bounds__(kThreads) k_persist(const PersistArgs<V> a) {
-    __shared__ State sst;
-    __shared__ int flip;
-    __shared__ unsigned int passed;
-    if (threadIdx.x == 0) {
-        flip = 0;
-        passed = 0u;
-    }
-    {
-        const int n = (int)(sizeof(State) / sizeof(int));
-        for (int k = threadIdx.x; k < n; k += blockDim.x)
-            reinterpret_cast<int *>(&sst)[k] = reinterpret_cast<const int *>(a.st)[k];
-    }
-    __syncthreads();
-    State *st = &sst;
-    const SegPersist seg{st, a.D, a.part, a.bar, &flip, &passed};
-    auto sync = [&]() -> bool {
-        if (grid_sync(a.bar, &passed)) return true;
-        if (threadIdx.x == 0) st->active = 0;
-        __syncthreads();
-        return false;
-    };
-    auto mv = [&](const V *in, V *out, const int *gate2) { persist_mv<V, MVK>(a, st, in, out, gate2); };
-    persist_loop<V, SegPersist>(seg, st, a.v, a.variant, a.jacobi, a.diag, mv, sync, INT_MAX);
-    // the copies are identical; block 0 publishes its own
-    if (blockIdx.x == 0) {
-        const int n = (int)(sizeof(State) / sizeof(int));
-        for (int k = threadIdx.x; k < n; k += blockDim.x)
-            reinterpret_cast<int *>(a.st)[k] = reinterpret_cast<const int *>(&sst)[k];
-    }
-}
-
-// The batched cached-connectivity product over one problem's rows (the batch matvec's CONN form
-// restricted to the segment): y[i] = diag0[i] x[i] + the row's cached (source, group) terms.
-template <typename V>
-__device__ __forceinline__ void d_batch_conn_seg(const rq_batch_t &B, const SegPersistB &seg,
-                                                 const V *x, V *y, const int *gate2) {
-    using R = typename VT<V>::R;
-    if (!seg.st->active || (gate2 && *gate2 == 0)) return;
-    constexpr uint64_t kMask = (1ULL << RQ_BATCH_STATE_BITS) - 1ULL;
-    SEG_LOOP(i) {
-        const uint64_t s = __ldg(B.keys + i) & kMask;
-        CAcc<R> acc;
-        const cx<R> xi = VT<V>::ld(x, i);
-        const R dv = (R)B.diag0[i];
-        acc.add({dv * xi.re, dv * xi.im});
-        const int64_t e1 = B.rowptr[i + 1];
-        for (int64_t e = B.rowptr[i]; e < e1; ++e)
-            acc.add(cmul(group_diag<R>(B.terms, __ldg(B.grp + e), s), VT<V>::ld(x, __ldg(B.col + e))));
-        VT<V>::st(y, i, acc.get());
-    }
-}
-
-template <typename V>
-struct PersistBatchArgs {
-    State *states;          // [P], read at start, written back by each problem's first block
-    rq_batch_t B;
-    Vecs<V> v;
-    int variant, jacobi;
-    const double *diag;
-    int iter_cap;           // iterations per problem in this launch
-    const int32_t *bprob;   // [grid] problem of each block
-    const int32_t *bfirst;  // [P] first block of each problem
-    const int32_t *nblk;    // [P] blocks of each problem
-    const int64_t *poff;    // [P] first float4 of each problem's partial sums
-    float4 *part;
-    GridBar *bars;          // [P]
-};
-
-// Many problems in one cooperative launch: each problem owns a group of blocks and runs
-// persist_loop on its own rows with its own reductions and barrier (blocks of different problems
-// never wait for each other), at most iter_cap iterations, after which the host re-plans the
-// block groups over the problems still active.
-template <typename V>
-__global__ void __launch_bounds__(kThreads, 2) k_persist_batch(const PersistBatchArgs<V> a) {
-    __shared__ State sst;
-    __shared__ int flip;
-    __shared__ unsigned int passed;
-    const int q = a.bprob[blockIdx.x];
-    if (threadIdx.x == 0) {
-        flip = 0;
-        passed = 0u;
-    }
-    {
-        const int n = (int)(sizeof(State) / sizeof(int));
-        for (int k = threadIdx.x; k < n; k += blockDim.x)
-            reinterpret_cast<int *>(&sst)[k] = reinterpret_cast<const int *>(a.states + q)[k];
-    }
-    __syncthreads();
-    State *st = &sst;
-    const int nb = a.nblk[q], lb = blockIdx.x - a.bfirst[q];
-    const SegPersistB seg{st, a.B.prow[q], a.B.prow[q + 1], lb, nb, a.part + a.poff[q],
-                          a.bars + q, &flip, &passed};
-    auto sync = [&]() -> bool {
-        if (group_sync(a.bars + q, &passed, (unsigned int)nb)) return true;
-        if (threadIdx.x == 0) st->active = 0;
-        __syncthreads();
-        return false;
-    };
-    auto mv = [&](const V *in, V *out, const int *gate2) { d_batch_conn_seg<V>(a.B, seg, in, out, gate2); };
-    const int stop = sst.iter + a.iter_cap;
-    persist_loop<V, SegPersistB>(seg, st, a.v, a.variant, a.jacobi, a.diag, mv, sync, stop);
-    if (lb == 0) {
-        const int n = (int)(sizeof(State) / sizeof(int));
-        for (int k = threadIdx.x; k < n; k += blockDim.x)
-            reinterpret_cast<int *>(a.states + q)[k] = reinterpret_cast<const int *>(&sst)[k];
-    }
+    int per = 0;
+    RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPersistThreads, dyn));
+    *fits = per >= 1;
+    if (!*fits) return RQ_OK;
+    PersistArgs<V> a = args;
+    void *ptr[] = {&a};
+    RQ_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kPersistThreads), ptr, dyn, s));
+    return RQ_OK;
 }
 
 template <typename PH>
 int run_persist(PH &ph, int variant, cudaStream_t s) {
     using V = typename std::remove_pointer<decltype(ph.v.x)>::type;
     const rq_operator_t &op = *ph.pop;
-    const void *kern = op.mode == RQ_MODE_CONN ? (const void *)k_persist<V, 0> : (const void *)k_persist<V, 1>;
-    int per = 0;
-    RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kThreads, 0));
-    if (per < 1) return run_loop(ph, variant, true, kChunk, s);
-    // as many blocks as the phase's kernels use, within the co-resident limit (the element-wise
-    // FP64 work needs every SM; fewer, longer threads measured slower at D = 2^16)
-    int grid = ph.grid;
-    if (grid > per * sm_count()) grid = per * sm_count();
-    if (grid > kMaxReduceBlocks / 2) grid = kMaxReduceBlocks / 2;  // two halves of partial sums
+    const bool csr = op.mode == RQ_MODE_CSR;
+    const int64_t D = ph.seg.D;
+    const int grid = persist_grid(D, op.nnz);
+    // shared memory for the average block's lists and a quarter more; the rest stays L1
+    const double avg = ((double)op.nnz * (4 + sizeof(typename ListVal<V>::T)) + 4. * (double)D) / grid;
+    const size_t dyn = std::min(kPersistMaxDyn, ((size_t)(1.25 * avg) + 4096) & ~size_t(1023));
     // partial sums in the phase's reduction scratch (its counter slot stays unused)
     float4 *part = reinterpret_cast<float4 *>(static_cast<char *>(ph.seg.red) + 16);
-    PersistArgs<V> a{ph.states, ph.seg.D, part, op, ph.v, variant, ph.jacobi ? 1 : 0, ph.diag,
-                     ph.bar};
+    const PersistArgs<V> a{ph.states, D, part,
+                           ListOp{op.rowptr, op.col, op.grp, csr ? op.val : nullptr, op.sub.states, ~0ULL,
+                                  op.diag0, op.terms},
+                           ph.v, ph.bar, (int)dyn};
     RQ_CUDA(cudaMemsetAsync(ph.bar, 0, sizeof(GridBar), s));
-    void *args[] = {&a};
-    RQ_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, 0, s));
+    bool fits = false;
+    if (variant == RQ_LOBPCG_FAST)
+        RQ_TRY((launch_persist<V, true>(a, grid, dyn, s, &fits)));
+    else
+        RQ_TRY((launch_persist<V, false>(a, grid, dyn, s, &fits)));
+    if (!fits) return run_loop(ph, variant, true, kChunk, s);
     GridBar h{};
     RQ_CUDA(cudaMemcpyAsync(&h, ph.bar, sizeof(GridBar), cudaMemcpyDeviceToHost, s));
     RQ_CUDA(cudaStreamSynchronize(s));
@@ -1710,8 +1435,11 @@ int run_persist_batch(PH &ph, int variant, cudaStream_t s) {
     using V = typename std::remove_pointer<decltype(ph.v.x)>::type;
     BatchPersist &bp = *ph.bp;
     const int P = ph.P;
+    const bool fast = variant == RQ_LOBPCG_FAST;
+    const void *kern = fast ? (const void *)k_persist_batch<V, true> : (const void *)k_persist_batch<V, false>;
+    RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistBatchDyn));
     int per = 0;
-    RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_persist_batch<V>, kThreads, 0));
+    RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPersistBatchThreads, kPersistBatchDyn));
     int G = per * sm_count();
     if (G > kMaxPersistBlocks) G = kMaxPersistBlocks;
     std::vector<State> h(P);
@@ -1749,7 +1477,7 @@ int run_persist_batch(PH &ph, int variant, cudaStream_t s) {
             const int64_t n = 1 + (int64_t)((double)extra * (double)r / (double)rows);
             nblk[q] = (int32_t)std::min(n, cap);
             for (int k = 0; k < nblk[q]; ++k) bprob.push_back(q);
-            pos += 2 * (int64_t)nblk[q] * kMaxReduce;
+            pos += 2 * (int64_t)nblk[q] * kPartStride;
         }
         const int grid = (int)bprob.size();
         RQ_CUDA(cudaMemcpyAsync(bp.bprob, bprob.data(), sizeof(int32_t) * grid, cudaMemcpyHostToDevice, s));
@@ -1757,12 +1485,14 @@ int run_persist_batch(PH &ph, int variant, cudaStream_t s) {
         RQ_CUDA(cudaMemcpyAsync(bp.nblk, nblk.data(), sizeof(int32_t) * P, cudaMemcpyHostToDevice, s));
         RQ_CUDA(cudaMemcpyAsync(bp.poff, poff.data(), sizeof(int64_t) * P, cudaMemcpyHostToDevice, s));
         RQ_CUDA(cudaMemsetAsync(bp.bars, 0, sizeof(GridBar) * P, s));
-        PersistBatchArgs<V> a{ph.states, *bp.b, ph.v, variant, ph.jacobi ? 1 : 0, ph.diag,
-                              kPersistIterCap, bp.bprob, bp.bfirst, bp.nblk, bp.poff, bp.part,
-                              bp.bars};
+        const rq_batch_t &B = *bp.b;
+        PersistBatchArgs<V> a{ph.states, B.prow,
+                              ListOp{B.rowptr, B.col, B.grp, nullptr, B.keys, (1ULL << RQ_BATCH_STATE_BITS) - 1ULL,
+                                     B.diag0, B.terms},
+                              ph.v, kPersistIterCap, bp.bprob, bp.bfirst, bp.nblk, bp.poff, bp.part, bp.bars,
+                              (int)kPersistBatchDyn};
         void *args[] = {&a};
-        RQ_CUDA(cudaLaunchCooperativeKernel((const void *)k_persist_batch<V>, dim3(grid),
-                                            dim3(kThreads), args, 0, s));
+        RQ_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kPersistBatchThreads), args, kPersistBatchDyn, s));
         RQ_CUDA(cudaMemcpyAsync(bars.data(), bp.bars, sizeof(GridBar) * P, cudaMemcpyDeviceToHost, s));
         RQ_CUDA(cudaStreamSynchronize(s));  // (the host vectors above are read by the copies)
         for (int q = 0; q < P; ++q)
@@ -2192,7 +1922,7 @@ int plan_batch(const rq_batch_t &b, const rq_lobpcg_params_t &p, BatchPlan &pl) 
     pl.pb_nblk = take(sizeof(int32_t) * P);
     pl.pb_poff = take(sizeof(int64_t) * P);
     pl.pb_bars = take(sizeof(GridBar) * P);
-    pl.pb_part = take(sizeof(float4) * 2 * kMaxPersistBlocks * kMaxReduce);
+    pl.pb_part = take(sizeof(float4) * 2 * kMaxPersistBlocks * kPartStride);
     pl.hi_bytes = (size_t)b.D * vtype_size(p.vtype);
     pl.lo_bytes = (size_t)b.D * vtype_size(lo_type(p.vtype));
     pl.vec_hi = take(8 * ((pl.hi_bytes + 255) & ~size_t(255)));

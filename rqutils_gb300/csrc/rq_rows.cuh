@@ -1,8 +1,5 @@
-// Row products shared by the matvec launches and the persistent LOBPCG kernel: the diagonal of
-// one X group on a row, and the cached-connectivity (CONN) and cached-element (CSR) row sums.
-// The vectors are plain pointers (no __restrict__): inside the persistent kernel they are
-// written by other blocks between grid barriers, so they must not be read through the
-// non-coherent path.
+// Row products shared by the single-problem and the batched matvec launches and the persistent
+// LOBPCG kernel: the diagonal of one X group on a row, and the tiled cached products.
 #pragma once
 
 #include "rq_common.cuh"
@@ -133,55 +130,6 @@ __device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, 
     }
     if (own) done(r0 + threadIdx.x, acc);
     __syncthreads();  // rp is read by every thread of the tile before the next one overwrites it
-}
-
-// y[i] = diag0[i] x[i] + sum over the row's cached (source, group) pairs; gated like the kernels
-template <typename V>
-__device__ __forceinline__ void d_matvec_conn(const rq_operator_t &op, const V *x, V *y,
-                                              const int *gate, const int *gate2) {
-    using R = typename VT<V>::R;
-    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
-    const rq_terms_t &T = op.terms;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < op.sub.D;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t s = __ldg(op.sub.states + i);
-        CAcc<R> acc;
-        const cx<R> xi = VT<V>::ld(x, i);
-        if (op.diag0) {
-            const R dv = (R)op.diag0[i];
-            acc.add({dv * xi.re, dv * xi.im});
-        } else if (T.diag_group >= 0) {
-            acc.add(cmul(group_diag<R>(T, T.diag_group, s), xi));
-        }
-        const int64_t e1 = op.rowptr[i + 1];
-        for (int64_t e = op.rowptr[i]; e < e1; ++e)
-            acc.add(cmul(group_diag<R>(T, __ldg(op.grp + e), s), VT<V>::ld(x, __ldg(op.col + e))));
-        VT<V>::st(y, i, acc.get());
-    }
-}
-
-// y[i] = diag0[i] x[i] + sum over the row's cached elements (value type VV)
-template <typename V, typename VV>
-__device__ __forceinline__ void d_matvec_csr(const rq_operator_t &op, const V *x, V *y,
-                                             const int *gate, const int *gate2) {
-    using R = typename VT<V>::R;
-    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
-    const VV *val = reinterpret_cast<const VV *>(op.val);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < op.sub.D;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        CAcc<R> acc;
-        if (op.diag0) {
-            const R dv = (R)op.diag0[i];
-            const cx<R> xi = VT<V>::ld(x, i);
-            acc.add({dv * xi.re, dv * xi.im});
-        }
-        const int64_t e1 = op.rowptr[i + 1];
-        for (int64_t e = op.rowptr[i]; e < e1; ++e) {
-            const auto v = VT<VV>::ld(val, e);
-            acc.add(cmul(cx<R>{(R)v.re, (R)v.im}, VT<V>::ld(x, __ldg(op.col + e))));
-        }
-        VT<V>::st(y, i, acc.get());
-    }
 }
 
 }  // namespace
