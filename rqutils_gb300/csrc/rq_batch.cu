@@ -97,11 +97,11 @@ __global__ void __launch_bounds__(kThreads)
 k_batch_line_prep(const uint64_t *__restrict__ keys, const int64_t *__restrict__ prow,
                   const uint64_t *__restrict__ xmask, const int32_t *__restrict__ gofs, int lwbits,
                   int32_t *__restrict__ lshift, uint32_t *__restrict__ xline) {
-    __shared__ uint32_t T[kHashTableWords];
+    __shared__ __align__(16) uint32_t T[kHashTableWords];
     __shared__ unsigned int hist[64];
     __shared__ int shift_s;
     const int p = blockIdx.x;
-    init_hash_tables(T, 8);
+    copy_hash_tables(T, 8);
     if (threadIdx.x < 64) hist[threadIdx.x] = 0u;
     __syncthreads();
     const int64_t r0 = prow[p], r1 = prow[p + 1];
@@ -132,8 +132,8 @@ k_batch_line_prep(const uint64_t *__restrict__ keys, const int64_t *__restrict__
 __global__ void __launch_bounds__(kThreads)
 k_batch_line_build(const uint64_t *__restrict__ keys, int64_t D, const int32_t *__restrict__ lshift,
                    uint32_t *__restrict__ lmap, int lbits, int lwbits) {
-    __shared__ uint32_t T[kHashTableWords];
-    init_hash_tables(T, 8);
+    __shared__ __align__(16) uint32_t T[kHashTableWords];
+    copy_hash_tables(T, 8);
     __syncthreads();
     const uint32_t bmask = (1u << lwbits) - 1u;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x) {
@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(kThreads, 4)
 k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y, int *err,
                     const int *gate, int64_t gstride, const int *gate2) {
     using R = typename VT<V>::R;
-    __shared__ uint32_t htab[kHashTableWords];
-    init_hash_tables(htab, 8);
+    __shared__ __align__(16) uint32_t htab[kHashTableWords];
+    copy_hash_tables(htab, 8);
     __syncthreads();
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < B.D;
          base += (int64_t)gridDim.x * blockDim.x) {
@@ -308,8 +308,8 @@ k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
 
 __global__ void __launch_bounds__(kThreads)
 k_batch_conn_count(const rq_batch_t B, int64_t *__restrict__ rowcnt, int *err) {
-    __shared__ uint32_t htab[kHashTableWords];
-    init_hash_tables(htab, 8);
+    __shared__ __align__(16) uint32_t htab[kHashTableWords];
+    copy_hash_tables(htab, 8);
     __syncthreads();
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < B.D;
          base += (int64_t)gridDim.x * blockDim.x) {
@@ -325,8 +325,8 @@ k_batch_conn_count(const rq_batch_t B, int64_t *__restrict__ rowcnt, int *err) {
 __global__ void __launch_bounds__(kThreads)
 k_batch_conn_fill(const rq_batch_t B, const int64_t *__restrict__ rowptr, int32_t *__restrict__ col,
                   int32_t *__restrict__ grp, int *err) {
-    __shared__ uint32_t htab[kHashTableWords];
-    init_hash_tables(htab, 8);
+    __shared__ __align__(16) uint32_t htab[kHashTableWords];
+    copy_hash_tables(htab, 8);
     __syncthreads();
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < B.D;
          base += (int64_t)gridDim.x * blockDim.x) {
@@ -354,13 +354,14 @@ k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
         const int p0 = problem_of(__ldg(B.keys + r0)), p1 = problem_of(__ldg(B.keys + r0 + nr - 1));
         if (p0 == p1 && !gate_open(gate, gstride, gate2, p0)) continue;
         tile_product<V>(
-            B.rowptr, r0, nr,
+            B.rowptr, r0, nr, long_groups(B.terms),
             [&](int64_t e) {
                 const int m = __ldg(B.col + e), g = __ldg(B.grp + e);
                 const uint64_t key = __ldg(B.keys + m);
                 if (p0 != p1 && !gate_open(gate, gstride, gate2, problem_of(key))) return typename RT::P{};
                 return RT::product(B.terms, g, (key ^ __ldg(B.terms.xmask + g)) & kStateMask, x, m);
             },
+            [&](int64_t e) { return group_terms(B.terms, __ldg(B.grp + e)); },
             [&](int64_t i, typename RT::A &acc) { acc.add(RT::scaled((R)B.diag0[i], x, i)); },
             [&](int64_t i, const typename RT::A &acc) {
                 if (p0 == p1 || gate_open(gate, gstride, gate2, problem_of(__ldg(B.keys + i)))) RT::store(y, i, acc);

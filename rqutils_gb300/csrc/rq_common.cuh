@@ -136,16 +136,26 @@ __host__ __device__ constexpr uint32_t lin_word(int i) {
 constexpr int kHashTableWords = 8 * 256;  // shared-memory words for 64-bit keys
 constexpr int kBucketSlots = 4;
 
-// Fill T[b * 256 + v] for b < nbytes (all threads of the block; caller synchronises).
-__device__ inline void init_hash_tables(uint32_t *T, int nbytes) {
-    for (int idx = threadIdx.x; idx < nbytes * 256; idx += blockDim.x) {
-        const int b = idx >> 8, v = idx & 255;
-        uint32_t h = 0;
-#pragma unroll
+// The tables T[b][v] as compile-time values in global memory: a block copies the first nbytes of them
+// with vector loads (computing them took eight steps per entry).
+struct HashTables {
+    uint32_t t[kHashTableWords];
+};
+constexpr HashTables make_hash_tables() {
+    HashTables h{};
+    for (int i = 0; i < kHashTableWords; ++i) {
+        uint32_t v = 0;
         for (int bit = 0; bit < 8; ++bit)
-            if ((v >> bit) & 1) h ^= lin_word(8 * b + bit);
-        T[idx] = h;
+            if ((i >> bit) & 1) v ^= lin_word(8 * (i >> 8) + bit);
+        h.t[i] = v;
     }
+    return h;
+}
+static __device__ __align__(16) const HashTables g_hash_tables = make_hash_tables();
+
+__device__ __forceinline__ void copy_hash_tables(uint32_t *T, int nbytes) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(g_hash_tables.t);
+    for (int i = threadIdx.x; i < nbytes * 64; i += blockDim.x) reinterpret_cast<uint4 *>(T)[i] = __ldg(src + i);
 }
 
 __device__ __forceinline__ uint32_t lin_hash(const uint32_t *T, uint64_t k, int nbytes) {

@@ -10,6 +10,7 @@
 //
 // Modes: FREE (lookups every call, cache_level (0, *)), CONN (cached (row -> source, group)
 // lists, diagonals recomputed, cache_level (1, 0)), CSR (cached element values, (*, 2)).
+#include <algorithm>
 #include <cmath>
 
 #include "rq_common.cuh"
@@ -150,56 +151,97 @@ __device__ inline void load_lookup_smem(const rq_subspace_t &S, uint32_t *fb, ui
 }
 
 // ------------------------------------------------------------------------------------------
-// FREE mode with the hash table: the hot kernel
+// FREE mode with the hash table: the hot kernels
 // ------------------------------------------------------------------------------------------
-// One thread per row.  Per row: h(s) once; per X group: t = s ^ x_j, sector filter,
-// bucket = (h(s) ^ h(x_j)) >> shift, one bucket load.  The per-group data (x_j, h(x_j)) is read
-// with broadcast shared-memory loads (every thread walks the same group sequence); the terms of
-// a group are read from global memory only on a hit.  U bucket loads are issued together; the
-// loop only marks "hot" groups (a key match, a full bucket, or a target equal to the empty key)
-// in a 64-bit mask, resolved once per 64 groups so that the rare divergent work is not
-// interleaved with the probes.  Each bucket load is one 16- or 32-byte read at a random address,
-// one L1 wavefront per lane; at D = 2^20 (tables in L2) those wavefronts are the limit.
+// h(s) once per row; per X group t = s ^ x_j, bucket (h(s) ^ h(x_j)) >> shift.  A probe asks whether t
+// can be a state; the few groups that can ("hot") are resolved in the table afterwards, so that the
+// rare divergent work is not interleaved with the probes.
 //
-// With the line filter (rq_subspace_t.lmap) the probe is a bit test in a line chosen by the
-// target's prefix t >> lshift: the rows of a warp are consecutive sorted states that share their
+// k_matvec_line (a line filter is present): the probe is a two-bit test in a line chosen by the
+// target's prefix t >> lshift.  The rows of a warp are consecutive sorted states that share their
 // high bits, so for one X group their targets share them too and the warp's probes fall in a few
-// lines (one wavefront each) instead of one line per lane.  Set bits are resolved in the table.
+// lines.
+// k_matvec_hash (no line filter): the probe is the key bucket itself, behind the sector filter and
+// the presence bitmap.
 
-// Group keys live in shared memory for the whole launch: (x_j, h(x_j)) packed as uint2 for 32-bit
-// keys or as uint64 + uint32 arrays for 64-bit keys, then the line hash hl_j = h(x_j >> lshift)
-// (12 or 16 B per group).  The x = 0 group is left out of the list (its diagonal is applied before
-// the probes), so that the probe loop has no per-group skip test; resident index c is group
-// c + (c >= diag_group).  Large J runs one 1024-thread block per SM so that up to
-// max_resident_groups fit; above that the keys are streamed through in tiles.
-template <int KB>
-__host__ __device__ constexpr int max_resident_groups() {
-    return KB == 32 ? 16384 : 12288;  // 192 KB of shared memory either way
-}
-
-template <int KB>
-__host__ __device__ inline size_t group_key_bytes(int J) {
-    return align16((size_t)J * 8) + (KB == 32 ? 0 : align16((size_t)J * 4)) + (size_t)J * 4;
-}
-
-template <int KB>
-__host__ __device__ inline size_t group_line_offset(int kt) {
-    return align16((size_t)kt * 8) + (KB == 32 ? 0 : align16((size_t)kt * 4));
-}
-
-// Sector filter of the hash kernel: none, the general (popcount a, popcount b) bitset, or the
+// Sector filter of the hash kernels: none, the general (popcount a, popcount b) bitset, or the
 // common case of a subspace in one sector (a single bit set: two popcount compares, no table).
 enum { kFiltNone = 0, kFiltSet = 1, kFiltPoint = 2 };
 // line filters of at most 2^25 bytes (32 MB, a quarter of GB300's L2) skip the sector test:
 // measured faster without it at 16 MB (Hubbard D = 2^20: 0.089 against 0.107 ms) and slower at
-// 64 MB (chemistry, 2^22 rows: 80.2 against 65.6 ms)
+// 64 MB (chemistry, 2^22 rows: 80.2 against 65.6 ms); clustered subspaces keep it at any size, since
+// their probes are bound by the lines a warp touches (36 qubits, 150,001 rows: 2.03 against 2.29 ms)
 constexpr int kLineFilterL2Log2Bytes = 25;
 
-// shared memory of the hash kernel: the sector bitset, the hash byte tables (64-bit keys use
+// shared memory of the hash kernels: the sector bitset, the hash byte tables (64-bit keys use
 // all eight) and, in dynamic shared memory, the resident group keys
 __shared__ uint32_t hk_fb[RQ_FILTER_WORDS];
-__shared__ uint32_t hk_htab[kHashTableWords];
+__shared__ __align__(16) uint32_t hk_htab[kHashTableWords];
 extern __shared__ __align__(16) unsigned char hk_dyn[];
+
+// The sector test of a target for the filter form FM (pa0, pb0: the popcounts of the one sector).
+template <typename K, int FM>
+__device__ __forceinline__ bool sector_pass(K t, K fa, K fbm, int pa0, int pb0) {
+    if (FM == kFiltPoint) {
+        int pa, pb;
+        if (sizeof(K) == 8) {
+            pa = __popcll((unsigned long long)(t & fa));
+            pb = __popcll((unsigned long long)(t & fbm));
+        } else {
+            pa = __popc((unsigned)(t & fa));
+            pb = __popc((unsigned)(t & fbm));
+        }
+        return (pa == pa0) & (pb == pb0);
+    }
+    if (FM == kFiltSet) return sector_ok_k<K>(hk_fb, fa, fbm, t);
+    return true;
+}
+
+// ---- probes of the line filter ---------------------------------------------------------------
+// What bounds it: instruction issue and L2 latency when hits are rare (Hubbard 4x4, 2^20 rows: 0.24
+// hits a row of 64 groups), the resolution of hits when they are not (a molecule's low-energy
+// samples: 84 of 2760 groups).  So
+// * a row is probed by w = 1 to 32 lanes: small subspaces would leave most of the chip idle, and the
+//   rows of a sample with the most hits stand together and would keep one warp busy long after the
+//   others (for such samples the tiles of a block are spread over the array, too; otherwise they
+//   stand together, because neighbouring tiles share filter lines);
+// * the hits of all lanes are gathered, in row and group order, into a queue that the whole warp
+//   resolves in full rounds (bucket, row index, terms, x): no lane waits for another's longer list,
+//   and FP64 instructions, which cost a warp the same however few lanes are active, run full;
+//   groups of more than kShortTerms terms go to a second queue, so that short ones do not wait;
+// * the owner lane of a row adds its products from the queue in group order, as the cached products do.
+// QUEUE = false: each lane resolves its own hits in a loop.  That needs fewer registers (48 warps per
+// SM instead of 32) and is the better one in 32-bit arithmetic with few groups and one lane per row
+// (Hubbard 4x4, 2^20 rows, complex64: 78 us against 83).
+constexpr int kQueueSlots = 128;  // hits resolved together
+
+template <typename V>
+struct WarpWork {
+    uint32_t hit[kQueueSlots];                   // lane << 16 | resident group, or kMissed
+    int src[kQueueSlots];                        // source row
+    typename RowTerm<V>::P prod[kQueueSlots];
+    uint8_t late[kQueueSlots];                   // queue slots of long groups
+};
+constexpr uint32_t kMissed = 0xFFFFFFFFu;
+
+// Group keys in shared memory: (h(x), line word) and, for the sector test, x.  The x = 0 group is
+// left out (its diagonal is applied before the probes); resident index c is group
+// c + (c >= diag_group).  More groups than fit stream through in tiles.  Entries past the last group
+// are probed and masked out: they hold a valid word.
+template <int FM>
+__host__ __device__ constexpr size_t line_key_bytes() { return FM != kFiltNone ? 16 : 8; }
+// groups a lane probes between two resolutions (256 measured slower: 2.6 against 2.3 ms on the
+// molecule above), and the entries past the last group
+constexpr int kPart = 64;
+
+template <typename V, int BLOCK, bool QUEUE>
+__host__ __device__ constexpr size_t line_work_bytes() { return QUEUE ? (BLOCK / 32) * sizeof(WarpWork<V>) : 0; }
+
+constexpr size_t kLineSmem = 216 * 1024;  // shared memory of a block with many groups (one per SM)
+template <typename V, int FM, int BLOCK>
+__host__ __device__ constexpr int line_tile_groups() {  // groups of a tile, at most 2^16
+    return ((int)((kLineSmem - 16 * 1024 - (BLOCK / 32) * sizeof(WarpWork<V>)) / line_key_bytes<FM>()) & ~63) - kPart;
+}
 
 // Line-filter word of a key (a state or an X mask): the word index line << (lwbits - 5) | word
 // within the line, line = h(k >> lshift) >> (32 - lbits), word = (h(k) mod 2^lwbits) >> 5.  Every
@@ -209,16 +251,195 @@ __device__ __forceinline__ uint32_t line_word(uint32_t h, uint32_t hpre, const r
     return ((hpre >> (32 - S.lbits)) << (S.lwbits - 5)) | ((h & ((1u << S.lwbits) - 1u)) >> 5);
 }
 
-// Group keys of resident indices [c0, c0 + cn) into shared-memory slots [0, cn); the layout holds
-// kt slots (32-bit keys: (x, h(x)) pairs; 64-bit keys: x masks, then hashes; then, with the line
-// filter, the line-filter words of the X masks).  Resident index c is group c + (c >= diag_group).
-// All threads of the block call it.
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
+__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : QUEUE ? 4 : 6)
+k_matvec_line(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err, int lw, int kt,
+              int spread, const int *gate, const int *gate2) {
+    using R = typename VT<V>::R;
+    using RT = RowTerm<V>;
+    using K = typename KeyWidth<KB>::K;
+    constexpr int NB = KeyWidth<KB>::kNbytes;
+    // probes in flight per lane: what 64 (QUEUE) and 40 registers hold
+    constexpr int U = FM != kFiltNone ? 8 : QUEUE ? 16 : KB == 32 ? 32 : 8;
+    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
+    const rq_subspace_t &S = op.sub;
+    const rq_terms_t &T = op.terms;
+    const int64_t D = S.D;
+    const int skip = T.diag_group;
+    const int nres = T.J - (skip >= 0 ? 1 : 0);
+    copy_hash_tables(hk_htab, NB);
+    if (FM == kFiltSet)
+        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = S.fbits[w];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    WarpWork<V> &W = reinterpret_cast<WarpWork<V> *>(hk_dyn)[QUEUE ? warp : 0];
+    uint2 *gk = reinterpret_cast<uint2 *>(hk_dyn + line_work_bytes<V, BLOCK, QUEUE>());  // [kt + kPart]
+    uint64_t *gx = reinterpret_cast<uint64_t *>(gk + kt + kPart);                       // the same, FM only
+    auto load_keys = [&](int c0, int n) {
+        for (int c = threadIdx.x; c < n + kPart; c += blockDim.x) {
+            const int j = c0 + c + (skip >= 0 && c0 + c >= skip);
+            const uint64_t xv = c < n ? T.xmask[j] : 0ULL;
+            const uint32_t h = c >= n ? 0u : T.xhash ? T.xhash[j] : lin_hash(hk_htab, xv, NB);
+            gk[c] = make_uint2(h, line_word(h, lin_hash(hk_htab, S.lshift < 64 ? xv >> S.lshift : 0ULL, NB), S));
+            if (FM != kFiltNone) gx[c] = xv;
+        }
+    };
+    __syncthreads();
+    const bool tiled = nres > kt;
+    if (!tiled) {
+        load_keys(0, nres);
+        __syncthreads();
+    }
+    const int pa0 = S.fpoint / 65, pb0 = S.fpoint % 65;
+    const K fa = (K)S.fmask_a, fbm = (K)S.fmask_b;
+    const int shift = 32 - S.hbits;
+    const uint32_t *lmap = S.lmap;
+    const unsigned lt = (1u << lane) - 1u;
+    const int w = 1 << lw, sub = lane & (w - 1);
+    const int64_t rows = 32 >> lw, stride = (int64_t)gridDim.x * (BLOCK / 32) * rows;
+    const int64_t first = (spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * (BLOCK / 32) + warp) * rows;
+    for (int64_t base = 0; base < D; base += stride) {  // the same trips for every warp of a block
+        const int64_t i = base + first + (lane >> lw);
+        const bool active = i < D;
+        if (!tiled && base + first >= D) break;
+        const int64_t ir = active ? i : D - 1;
+        const uint64_t s64 = __ldg(S.states + ir);
+        const K s = (K)s64;
+        const uint32_t hs = lin_hash(hk_htab, s64, NB);
+        // the row's line-filter word: a target's word is wrow ^ word(x), its bits those of hs ^ h(x)
+        const uint32_t wrow = line_word(hs, lin_hash(hk_htab, S.lshift < 64 ? s64 >> S.lshift : 0ULL, NB), S);
+        typename RT::A acc;
+        if (sub == 0) {
+            if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[ir], x, ir));
+            else if (skip >= 0) acc.add(RT::product(T, skip, s64, x, ir));
+        }
+        for (int t0 = 0; t0 < nres; t0 += kt) {
+            const int tn = min(kt, nres - t0);
+            if (tiled) {
+                __syncthreads();  // the previous tile is no longer read
+                load_keys(t0, tn);
+                __syncthreads();
+            }
+            // lane `sub` of a row takes the sub-th part of the next up to kPart w groups
+            int part = 0;
+            for (int g0 = 0; g0 < tn; g0 += part << lw) {
+                part = min(kPart, (tn - g0 + w - 1) >> lw);
+                const int e0 = min(g0 + sub * part, tn), en = active ? min(part, tn - e0) : 0;
+                uint64_t hot = 0ULL;
+                for (int k0 = 0; k0 < part; k0 += U) {
+                    const uint2 *key = gk + e0 + k0;
+                    uint32_t v[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t *p = lmap + (wrow ^ key[u].y);
+                        v[u] = FM == kFiltNone ? __ldg(p)
+                                               : load_word(p, sector_pass<K, FM>(s ^ (K)gx[e0 + k0 + u], fa, fbm, pa0, pb0));
+                    }
+                    uint32_t hb = 0u;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {  // (the funnel shift takes its count mod 32)
+                        const uint32_t b = hs ^ key[u].x;
+                        hb += (__funnelshift_r(v[u], 0u, b) & (v[u] >> (b >> 27)) & 1u) << u;
+                    }
+                    hot |= (uint64_t)hb << k0;
+                }
+                hot &= en >= 64 ? ~0ULL : (1ULL << en) - 1ULL;
+                if (!QUEUE) {
+                    while (hot) {
+                        const int e = e0 + __ffsll((long long)hot) - 1, c = t0 + e, gg = c + (skip >= 0 && c >= skip);
+                        hot &= hot - 1ULL;
+                        const int m = lookup_hash_at<KB>(S, s64 ^ __ldg(T.xmask + gg), (hs ^ gk[e].x) >> shift, err);
+                        if (m >= 0) acc.add(RT::product(T, gg, s64, x, m));
+                    }
+                    __syncwarp();  // re-converge before the next probes
+                    continue;
+                }
+                // resolve the hits of the warp, kQueueSlots at a time
+                const int cnt = __popcll(hot);
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += u;
+                }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                if (total == 0) continue;
+                int off = incl - cnt;
+                // the row's range of the queue
+                const int ra = __shfl_sync(0xffffffffu, off, lane & ~(w - 1));
+                const int rb = __shfl_sync(0xffffffffu, incl, lane | (w - 1));
+                for (int q0 = 0; q0 < total; q0 += kQueueSlots) {
+                    const int n = min(kQueueSlots, total - q0);
+                    while (hot && off < q0 + n) {
+                        W.hit[off - q0] = (uint32_t)lane << 16 | (uint32_t)(e0 + __ffsll((long long)hot) - 1);
+                        hot &= hot - 1ULL;
+                        ++off;
+                    }
+                    __syncwarp();
+                    int late = 0;
+                    for (int q = lane; q - lane < n; q += 32) {
+                        const bool ok = q < n;
+                        const uint32_t hit = ok ? W.hit[q] : 0u;
+                        const uint64_t rs = __shfl_sync(0xffffffffu, s64, hit >> 16);
+                        const uint32_t rh = __shfl_sync(0xffffffffu, hs, hit >> 16);
+                        bool defer = false;
+                        if (ok) {
+                            const int e = (int)(hit & 0xFFFFu), c = t0 + e, gg = c + (skip >= 0 && c >= skip);
+                            const uint64_t xv = __ldg(T.xmask + gg);
+                            const int nt = group_terms(T, gg);
+                            const int m = lookup_hash_at<KB>(S, rs ^ xv, (rh ^ gk[e].x) >> shift, err);
+                            if (m < 0) W.hit[q] = kMissed;
+                            else if (nt > kShortTerms) defer = true;
+                            else W.prod[q] = RT::product(T, gg, rs, x, m);
+                            W.src[q] = m;
+                        }
+                        const unsigned dm = __ballot_sync(0xffffffffu, defer);
+                        if (defer) W.late[late + __popc(dm & lt)] = (uint8_t)q;
+                        late += __popc(dm);
+                    }
+                    __syncwarp();
+                    for (int k = lane; k - lane < late; k += 32) {
+                        const bool ok = k < late;
+                        const int q = ok ? W.late[k] : 0;
+                        const uint32_t hit = ok ? W.hit[q] : 0u;
+                        const uint64_t rs = __shfl_sync(0xffffffffu, s64, hit >> 16);
+                        if (ok) {
+                            const int c = t0 + (int)(hit & 0xFFFFu), gg = c + (skip >= 0 && c >= skip);
+                            W.prod[q] = RT::product(T, gg, rs, x, W.src[q]);
+                        }
+                    }
+                    __syncwarp();
+                    if (sub == 0)
+                        for (int k = max(ra, q0); k < min(rb, q0 + n); ++k)
+                            if (W.hit[k - q0] != kMissed) acc.add(W.prod[k - q0]);
+                    __syncwarp();
+                }
+            }
+        }
+        if (active && sub == 0) RT::store(y, i, acc);
+    }
+}
+
+// ---- probes of the key buckets ----------------------------------------------------------------
+// Group keys live in shared memory for the whole launch: (x_j, h(x_j)) packed as uint2 for 32-bit
+// keys or as uint64 + uint32 arrays for 64-bit keys (8 or 12 B per group), without the x = 0 group.
+// Large J runs one 1024-thread block per SM so that up to max_resident_groups fit; above that the
+// keys are streamed through in tiles.
 template <int KB>
-__device__ __forceinline__ void load_group_keys(const rq_terms_t &T, int c0, int cn, int kt,
-                                                const rq_subspace_t &S) {
+__host__ __device__ constexpr int max_resident_groups() {
+    return KB == 32 ? 24576 : 16384;  // 192 KB of shared memory either way
+}
+
+template <int KB>
+__host__ __device__ inline size_t group_key_bytes(int J) {
+    return align16((size_t)J * 8) + (KB == 32 ? 0 : align16((size_t)J * 4));
+}
+
+// Group keys of resident indices [c0, c0 + cn) into shared-memory slots [0, cn); the layout holds
+// kt slots.  All threads of the block call it.
+template <int KB>
+__device__ __forceinline__ void load_group_keys(const rq_terms_t &T, int c0, int cn, int kt) {
     constexpr int NB = KeyWidth<KB>::kNbytes;
     const int skip = T.diag_group;
-    uint32_t *hl = reinterpret_cast<uint32_t *>(hk_dyn + group_line_offset<KB>(kt));
     for (int c = threadIdx.x; c < cn; c += blockDim.x) {
         const int j = c0 + c + (skip >= 0 && c0 + c >= skip);
         const uint64_t xv = T.xmask[j];
@@ -229,72 +450,47 @@ __device__ __forceinline__ void load_group_keys(const rq_terms_t &T, int c0, int
             reinterpret_cast<uint64_t *>(hk_dyn)[c] = xv;
             reinterpret_cast<uint32_t *>(hk_dyn + align16((size_t)kt * 8))[c] = h;
         }
-        hl[c] = S.lmap ? line_word(h, lin_hash(hk_htab, S.lshift < 64 ? xv >> S.lshift : 0ULL, NB), S) : 0u;
     }
 }
 
-// Probes in flight per thread: four with key buckets (a 16- or 32-byte bucket per probe fills the
-// 40 registers of six resident 256-thread blocks).  With the line filter (one 4-byte word per
-// probe): 32 for 32-bit keys without a sector test, 16 in the 1024-thread kernel of 64-bit keys,
-// 8 otherwise, 4 with the bitset sector test: the most that compile without new spills (ptxas -v).
-// More probes in flight measured 5 % faster on the 64-qubit chemistry subspace (61.7 against
-// 65.4 ms at 2^22 rows, one-bit filter) and the same on Hubbard.  A divisor of the 64 groups of a
-// super-chunk.
-constexpr int kKeyProbes = 4;
-
-template <typename V, int KB, int FM, bool TL>
-__host__ __device__ constexpr int line_probes() {
-    return FM == kFiltSet ? 4 : (KB == 32 && FM == kFiltNone) ? 32 : (KB == 64 && TL) ? 16 : 8;
-}
-
-// LF: probe the line filter.  TL: the group keys may need streaming in tiles (1024-thread kernels
-// only; with 256-thread blocks they always fit and the tile loop is one pass known at compile
-// time).
-template <typename V, int KB, int FM, bool LF, bool TL>
-__device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__restrict__ x,
-                                          V *__restrict__ y, int *err, int pa0, int pb0) {
+// TL: the group keys may need streaming in tiles (1024-thread kernels only; with 256-thread blocks
+// they always fit and the tile loop is one pass known at compile time).  FM: the sector filter's
+// form, chosen on the host from rq_subspace_t.fpoint.
+template <typename V, int KB, int FM, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : (sizeof(V) <= 8 ? 6 : 4))
+k_matvec_hash(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err,
+              const int *gate, const int *gate2) {
     using R = typename VT<V>::R;
+    using RT = RowTerm<V>;
     using K = typename KeyWidth<KB>::K;
+    constexpr bool TL = BLOCK == 1024;
     constexpr int NB = KeyWidth<KB>::kNbytes;
     constexpr int kBucketBytes = KeyWidth<KB>::kBucketBytes;
-    constexpr int U = LF ? line_probes<V, KB, FM, TL>() : kKeyProbes;
+    constexpr int U = 4;  // buckets in flight: 16 or 32 bytes each fill the registers of six blocks
+    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     const rq_subspace_t &S = op.sub;
     const rq_terms_t &T = op.terms;
     const int64_t D = S.D;
     const int skip = T.diag_group;  // the x = 0 group is applied outside the probe loop
     const int nres = T.J - (skip >= 0 ? 1 : 0);  // groups of the probe loop
-    // shared-memory slots: every group's keys when they fit (loaded once by the kernel), else
-    // tiles of max_resident_groups streamed through for every row batch
+    copy_hash_tables(hk_htab, NB);
+    if (FM == kFiltSet)
+        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = S.fbits[w];
+    __syncthreads();
     constexpr int kMaxRes = max_resident_groups<KB>();
     const int kt = (!TL || nres <= kMaxRes) ? nres : kMaxRes;
     const bool tiled = TL && nres > kt;
+    if (!tiled) load_group_keys<KB>(T, 0, nres, nres);
+    __syncthreads();
     const uint2 *gk32 = reinterpret_cast<const uint2 *>(hk_dyn);
     const uint64_t *gx64 = reinterpret_cast<const uint64_t *>(hk_dyn);
     const uint32_t *gh64 = reinterpret_cast<const uint32_t *>(hk_dyn + align16((size_t)kt * 8));
-    const uint32_t *ghl = reinterpret_cast<const uint32_t *>(hk_dyn + group_line_offset<KB>(kt));
-    const bool d0 = (op.diag0 != nullptr) && (skip >= 0);
+    const int pa0 = S.fpoint / 65, pb0 = S.fpoint % 65;
     const K fa = (K)S.fmask_a, fbm = (K)S.fmask_b, empty = (K)S.empty_key;
     const int shift = 32 - S.hbits;
-    // the line filter replaces the presence bitmap
-    const uint32_t *pmap = (!LF && S.pbits > 0) ? S.pmap : nullptr;
+    const uint32_t *pmap = S.pbits > 0 ? S.pmap : nullptr;
     const int pshift = 32 - S.pbits;
     const unsigned char *keys = static_cast<const unsigned char *>(S.hkeys);
-    const uint32_t *lmap = S.lmap;
-    auto sector = [&](K t) -> bool {
-        if (FM == kFiltPoint) {
-            int pa, pb;
-            if (sizeof(K) == 8) {
-                pa = __popcll((unsigned long long)(t & fa));
-                pb = __popcll((unsigned long long)(t & fbm));
-            } else {
-                pa = __popc((unsigned)(t & fa));
-                pb = __popc((unsigned)(t & fbm));
-            }
-            return (pa == pa0) & (pb == pb0);
-        }
-        if (FM == kFiltSet) return sector_ok_k<K>(hk_fb, fa, fbm, t);
-        return true;
-    };
     // Every lane runs the same row batches and super-chunks, so that the warp can be
     // re-converged after each super-chunk's hot-group resolution; without the explicit
     // __syncwarp the lanes that took the rare path stay split from the rest for the remainder of
@@ -307,21 +503,14 @@ __device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__re
         const uint64_t s64 = __ldg(S.states + ir);
         const K s = (K)s64;
         const uint32_t hs = lin_hash(hk_htab, s64, NB);
-        // the row's line-filter word: a target's word is wrow ^ hl[j], its bit (hs ^ h(x)) mod 32
-        const uint32_t wrow = LF ? line_word(hs, lin_hash(hk_htab, S.lshift < 64 ? s64 >> S.lshift : 0ULL, NB), S) : 0u;
-        CAcc<R> acc;
-        const cx<R> xi = VT<V>::ld(x, ir);
-        if (d0) {
-            const R dv = (R)op.diag0[ir];
-            acc.add({dv * xi.re, dv * xi.im});
-        } else if (skip >= 0) {
-            acc.add(cmul(group_diag<R>(T, skip, s64), xi));
-        }
+        typename RT::A acc;
+        if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[ir], x, ir));
+        else if (skip >= 0) acc.add(RT::product(T, skip, s64, x, ir));
         for (int t0 = 0; TL ? t0 < nres : t0 < 1; t0 += TL ? kt : 1) {
             const int tn = TL ? min(kt, nres - t0) : nres;
             if (tiled) {
                 __syncthreads();  // the previous tile is no longer read
-                load_group_keys<KB>(T, t0, tn, kt, S);
+                load_group_keys<KB>(T, t0, tn, kt);
                 __syncthreads();
             }
             for (int gs0 = 0; gs0 < tn; gs0 += 64) {
@@ -330,7 +519,7 @@ __device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__re
                 int g = gs0;
                 for (; g + U <= gs1; g += U) {
                     K t[U];
-                    uint32_t b[U], ln[U];
+                    uint32_t b[U];
                     bool q[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
@@ -343,9 +532,8 @@ __device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__re
                             t[u] = s ^ (K)gx64[g + u];
                             hxg = gh64[g + u];
                         }
-                        q[u] = sector(t[u]);
+                        q[u] = sector_pass<K, FM>(t[u], fa, fbm, pa0, pb0);
                         b[u] = hs ^ hxg;
-                        if (LF) ln[u] = wrow ^ ghl[g + u];
                     }
                     if (pmap) {  // presence bitmap (L2-resident) in front of a table that is not
                         uint32_t pw[U];
@@ -358,36 +546,22 @@ __device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__re
                         for (int u = 0; u < U; ++u) q[u] = q[u] && ((pw[u] >> ((b[u] >> pshift) & 31)) & 1u);
                     }
                     uint32_t hb = 0u;  // hot bits of this batch, constant shifts
-                    if (LF) {
-                        // line filter: a hot lane's bit is set (a state, or another state's bit;
-                        // the resolution below compares the keys).  A lane whose target fails
-                        // the sector filter reads no word: the zero word it keeps is never hot,
-                        // so q need not stay live across the loads.
-                        uint32_t w[U];
+                    typename KeyWidth<KB>::Bucket w[U];
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            w[u] = load_word(lmap + ln[u], q[u]);
+                    for (int u = 0; u < U; ++u)
+                        w[u] = KeyWidth<KB>::load(keys + (size_t)(b[u] >> shift) * kBucketBytes,
+                                                  q[u], S.empty_key);
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            if ((w[u] >> (b[u] & 31u)) & (w[u] >> (b[u] >> 27)) & 1u) hb |= 1u << u;
-                    } else {
-                        typename KeyWidth<KB>::Bucket w[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            w[u] = KeyWidth<KB>::load(keys + (size_t)(b[u] >> shift) * kBucketBytes,
-                                                      q[u], S.empty_key);
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            bool any, open;
-                            test_bucket(w[u], t[u], empty, any, open);
-                            if (q[u] && (any || !open)) hb |= 1u << u;
-                        }
+                    for (int u = 0; u < U; ++u) {
+                        bool any, open;
+                        test_bucket(w[u], t[u], empty, any, open);
+                        if (q[u] && (any || !open)) hb |= 1u << u;
                     }
                     hot |= (uint64_t)hb << (g - gs0);
                 }
                 for (; g < gs1; ++g) {  // tail: mark and resolve below
                     const K t = s ^ (KB == 32 ? (K)gk32[g].x : (K)gx64[g]);
-                    if (sector(t)) hot |= 1ULL << (g - gs0);
+                    if (sector_pass<K, FM>(t, fa, fbm, pa0, pb0)) hot |= 1ULL << (g - gs0);
                 }
                 while (hot) {
                     const int gc = gs0 + __ffsll((long long)hot) - 1;  // slot in shared memory
@@ -397,44 +571,20 @@ __device__ __forceinline__ void hash_rows(const rq_operator_t &op, const V *__re
                     const uint64_t xv = __ldg(T.xmask + gg);
                     const uint32_t hxg = KB == 32 ? gk32[gc].y : gh64[gc];
                     const int m = lookup_hash_at<KB>(S, s64 ^ xv, (hs ^ hxg) >> shift, err);
-                    if (m >= 0) acc.add(cmul(group_diag<R>(T, gg, s64), VT<V>::ld(x, m)));
+                    if (m >= 0) acc.add(RT::product(T, gg, s64, x, m));
                 }
                 __syncwarp();
             }
         }
-        if (active) VT<V>::st(y, i, acc.get());
+        if (active) RT::store(y, i, acc);
     }
-}
-
-// FM: the sector filter's form, chosen on the host from rq_subspace_t.fpoint (one kernel per
-// form, so that the registers of the general bitset test do not weigh on the one-sector kernel)
-template <typename V, int KB, int FM, int BLOCK, bool LF>
-__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : (sizeof(V) <= 8 ? 6 : 4))
-k_matvec_hash(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err,
-              const int *gate, const int *gate2) {
-    constexpr int NB = KeyWidth<KB>::kNbytes;
-    if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
-    const rq_subspace_t &S = op.sub;
-    const rq_terms_t &T = op.terms;
-    init_hash_tables(hk_htab, NB);
-    if (FM == kFiltSet)
-        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = S.fbits[w];
-    __syncthreads();
-    const int nres = T.J - (T.diag_group >= 0 ? 1 : 0);
-    if (nres <= max_resident_groups<KB>())  // else in tiles
-        load_group_keys<KB>(T, 0, nres, nres, S);
-    __syncthreads();
-    if (FM == kFiltPoint)
-        hash_rows<V, KB, FM, LF, BLOCK == 1024>(op, x, y, err, S.fpoint / 65, S.fpoint % 65);
-    else
-        hash_rows<V, KB, FM, LF, BLOCK == 1024>(op, x, y, err, 0, 0);
 }
 
 // xhash[j] = h(xmask[j])
 template <int KB>
 __global__ void k_terms_hash(const uint64_t *__restrict__ xmask, int J, uint32_t *__restrict__ out) {
-    __shared__ uint32_t htab[KeyWidth<KB>::kNbytes * 256];
-    init_hash_tables(htab, KeyWidth<KB>::kNbytes);
+    __shared__ __align__(16) uint32_t htab[KeyWidth<KB>::kNbytes * 256];
+    copy_hash_tables(htab, KeyWidth<KB>::kNbytes);
     __syncthreads();
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < J; j += gridDim.x * blockDim.x)
         out[j] = lin_hash(htab, xmask[j], KeyWidth<KB>::kNbytes);
@@ -517,11 +667,11 @@ __global__ void __launch_bounds__(kThreads)
 k_conn_count(const rq_operator_t op, int64_t *__restrict__ rowcnt, int *err) {
     __shared__ uint32_t fb[RQ_FILTER_WORDS];
     __shared__ uint64_t samp[LK == RQ_LOOKUP_BSEARCH ? kSample : 1];
-    __shared__ uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 1];
+    __shared__ __align__(16) uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 4];
     const rq_subspace_t &S = op.sub;
     const int ns = (LK == RQ_LOOKUP_BSEARCH) ? (int)(S.D < kSample ? S.D : kSample) : 0;
     load_lookup_smem<LK>(S, fb, samp, ns);
-    if (LK == RQ_LOOKUP_HASH) init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    if (LK == RQ_LOOKUP_HASH) copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < S.D;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -542,11 +692,11 @@ k_conn_fill(const rq_operator_t op, const int64_t *__restrict__ rowptr, int32_t 
     using R = typename VT<V>::R;
     __shared__ uint32_t fb[RQ_FILTER_WORDS];
     __shared__ uint64_t samp[LK == RQ_LOOKUP_BSEARCH ? kSample : 1];
-    __shared__ uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 1];
+    __shared__ __align__(16) uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 4];
     const rq_subspace_t &S = op.sub;
     const int ns = (LK == RQ_LOOKUP_BSEARCH) ? (int)(S.D < kSample ? S.D : kSample) : 0;
     load_lookup_smem<LK>(S, fb, samp, ns);
-    if (LK == RQ_LOOKUP_HASH) init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    if (LK == RQ_LOOKUP_HASH) copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < S.D;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -668,11 +818,12 @@ k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y
     const int64_t D = op.sub.D;
     for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
         tile_product<V>(
-            op.rowptr, r0, (int)min((int64_t)rows, D - r0),
+            op.rowptr, r0, (int)min((int64_t)rows, D - r0), long_groups(T),
             [&](int64_t e) {
                 const int m = __ldg(op.col + e), g = __ldg(op.grp + e);
                 return RT::product(T, g, __ldg(op.sub.states + m) ^ __ldg(T.xmask + g), x, m);
             },
+            [&](int64_t e) { return group_terms(T, __ldg(op.grp + e)); },
             [&](int64_t i, typename RT::A &acc) {
                 if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
                 else if (T.diag_group >= 0) acc.add(RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
@@ -692,11 +843,12 @@ k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y,
     const int64_t D = op.sub.D;
     for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
         tile_product<V>(
-            op.rowptr, r0, (int)min((int64_t)rows, D - r0),
+            op.rowptr, r0, (int)min((int64_t)rows, D - r0), false,
             [&](int64_t e) {
                 const auto v = VT<VV>::ld(val, e);
                 return RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e));
             },
+            [](int64_t) { return 0; },
             [&](int64_t i, typename RT::A &acc) {
                 if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
             },
@@ -729,10 +881,10 @@ int launch_csr(const rq_operator_t &op, const void *x, void *y, cudaStream_t st,
 // ------------------------------------------------------------------------------------------
 // host dispatch
 // ------------------------------------------------------------------------------------------
-template <typename V, int KB, int FM, int BLOCK, bool LF>
+template <typename V, int KB, int FM, int BLOCK>
 int launch_hash_block(const rq_operator_t &op, const void *x, void *y, int *err, cudaStream_t st,
                       const int *gate, const int *gate2) {
-    auto kern = k_matvec_hash<V, KB, FM, BLOCK, LF>;
+    auto kern = k_matvec_hash<V, KB, FM, BLOCK>;
     const int nres = op.terms.J - (op.terms.diag_group >= 0 ? 1 : 0);
     constexpr int kMaxRes = max_resident_groups<KB>();
     const size_t smem = group_key_bytes<KB>(nres < kMaxRes ? nres : kMaxRes);
@@ -750,20 +902,78 @@ int launch_hash_block(const rq_operator_t &op, const void *x, void *y, int *err,
     return RQ_OK;
 }
 
+// Clustered subspaces (low-energy samples of a molecule) with many groups: their hits crowd on some
+// rows, which stand together, and their line prefix is short, so that a warp's probes fall in many
+// lines.  The prefix shift tells them: states spread over n bits get about n - log2 D + 3, less the
+// few bits that a sector takes (measured 1 to 3; molecules 4 to 11).
+constexpr int kClusterBits = 4;
+constexpr int kClusterGroups = 256;
+inline bool clustered(const rq_subspace_t &S, int J) {
+    const uint64_t used = S.fmask_a | S.fmask_b;
+    const int n = used ? 64 - __builtin_clzll(used) : 0, d = 63 - __builtin_clzll((uint64_t)S.D);
+    return J >= kClusterGroups && n - d + 3 - S.lshift >= kClusterBits;
+}
+
+// Lanes per row (log2): the most with which all rows are still resident at once, kLineThreads
+// threads per SM.  One lane is best for large subspaces (the rows of a warp share filter lines, and
+// every lane sums a row); at 16,384 rows one lane leaves 9 of 10 warp slots of the chip empty.
+// Clustered subspaces take as many lanes as make kLineWaves passes over the chip: 36 qubits, 150,001
+// rows, float64: 2.3 against 3.8 ms with one lane, 2.6 with eight passes; spread states want one lane
+// (40 qubits, 100,000 rows: 84 us against 121 with four).
+constexpr int kLineThreads = 1024;
+constexpr int kLineWaves = 4;
+constexpr int kOwnHitsGroups = 128;  // most groups of the kernel whose lanes resolve their own hits
+inline int line_lanes_log2(const rq_subspace_t &S, int J, int sms) {
+    const int waves = clustered(S, J) ? kLineWaves : 1;
+    int lw = 0;
+    while (lw < 5 && ((S.D << (lw + 1)) <= (int64_t)sms * kLineThreads ||
+                      (J >= 64 << (lw + 1) && (S.D << (lw + 1)) <= (int64_t)sms * kLineThreads * waves)))
+        ++lw;
+    return lw;
+}
+
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
+int launch_line_block(const rq_operator_t &op, int lw, const void *x, void *y, int *err, cudaStream_t st,
+                      const int *gate, const int *gate2) {
+    auto kern = k_matvec_line<V, KB, FM, BLOCK, QUEUE>;
+    const int nres = op.terms.J - (op.terms.diag_group >= 0 ? 1 : 0);
+    constexpr int kMaxTile = line_tile_groups<V, FM, BLOCK>();
+    static_assert(kMaxTile <= 65536, "a queue entry holds 16 bits of group");
+    const int kt = nres < kMaxTile ? std::max(nres, 1) : kMaxTile;
+    const size_t smem = line_work_bytes<V, BLOCK, QUEUE>() + (size_t)(kt + kPart) * line_key_bytes<FM>();
+    thread_local KernelLaunchCache table[kMaxCachedDevices];
+    KernelLaunchCache *c = nullptr;
+    int per_sm = 1;
+    RQ_TRY(cache_slot(table, &c));
+    RQ_TRY(configure_kernel(kern, *c, smem, BLOCK, &per_sm));
+    const int64_t rows = BLOCK >> lw;
+    int64_t g = (op.sub.D + rows - 1) / rows;
+    const int64_t cap = (int64_t)sm_count() * per_sm;
+    if (g > cap) g = cap;
+    kern<<<(int)g, BLOCK, smem, st>>>(op, static_cast<const V *>(x), static_cast<V *>(y), err, lw, kt,
+                                      clustered(op.sub, op.terms.J) ? 1 : 0, gate, gate2);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
 template <typename V, int KB, int FM>
 int launch_hash(const rq_operator_t &op, const void *x, void *y, int *err, cudaStream_t st,
                 const int *gate, const int *gate2) {
-    // small group sets: several 256-thread blocks per SM; large ones (streamed in tiles of
-    // max_resident_groups above that count): one 1024-thread block.
-    // With a line filter the probes test its bits (not with 64-bit keys and the bitset filter,
-    // whose line-filter kernel spills registers).
+    // small group sets: several 256-thread blocks per SM; large ones (streamed in tiles above what
+    // fits): one 1024-thread block
+    if (op.sub.lmap) {
+        const int lw = line_lanes_log2(op.sub, op.terms.J, sm_count());
+        if constexpr (sizeof(typename VT<V>::R) == 4)
+            if (lw == 0 && op.terms.J <= kOwnHitsGroups)
+                return launch_line_block<V, KB, FM, 256, false>(op, lw, x, y, err, st, gate, gate2);
+        return op.terms.J * line_key_bytes<FM>() <= 16 * 1024
+                   ? launch_line_block<V, KB, FM, 256, true>(op, lw, x, y, err, st, gate, gate2)
+                   : launch_line_block<V, KB, FM, 1024, true>(op, lw, x, y, err, st, gate, gate2);
+    }
     const bool small = op.terms.J <= max_resident_groups<KB>() &&
                        group_key_bytes<KB>(op.terms.J) <= 16 * 1024;
-    if (op.sub.lmap && !(KB == 64 && FM == kFiltSet))
-        return small ? launch_hash_block<V, KB, FM, 256, true>(op, x, y, err, st, gate, gate2)
-                     : launch_hash_block<V, KB, FM, 1024, true>(op, x, y, err, st, gate, gate2);
-    return small ? launch_hash_block<V, KB, FM, 256, false>(op, x, y, err, st, gate, gate2)
-                 : launch_hash_block<V, KB, FM, 1024, false>(op, x, y, err, st, gate, gate2);
+    return small ? launch_hash_block<V, KB, FM, 256>(op, x, y, err, st, gate, gate2)
+                 : launch_hash_block<V, KB, FM, 1024>(op, x, y, err, st, gate, gate2);
 }
 
 template <typename V, int LK>
@@ -804,7 +1014,7 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
                 // keeps it, since its words then compete for L2 or come from DRAM.
                 const bool line_in_l2 =
                     op.sub.lmap && op.sub.lbits + op.sub.lwbits - 3 <= kLineFilterL2Log2Bytes;
-                const int fm = ((op.sub.fmask_a | op.sub.fmask_b) == 0 || line_in_l2) ? kFiltNone
+                const int fm = ((op.sub.fmask_a | op.sub.fmask_b) == 0 || (line_in_l2 && !clustered(op.sub, op.terms.J))) ? kFiltNone
                                : op.sub.fpoint >= 0                                     ? kFiltPoint
                                                                                         : kFiltSet;
                 if (op.sub.key_bits == 32) {

@@ -7,37 +7,80 @@
 namespace rq {
 namespace {
 
-// sum_k c_k (-1)^popcount(s & z_k) over group g, stopping at the first zero coefficient
+// 64-bit coefficients enter as bit patterns: on GB300 a warp's FP64 instruction (a comparison too)
+// holds its SM quarter for 64 cycles, and integer ones do not.
+__device__ __forceinline__ bool is_zero(uint64_t bits) { return (bits << 1) == 0ULL; }
+__device__ __forceinline__ bool is_zero(float v) { return v == 0.f; }
+__device__ __forceinline__ uint64_t coef_bits(const double *p) {
+    return (uint64_t)__ldg(reinterpret_cast<const unsigned long long *>(p));
+}
+// the value of a coefficient in the arithmetic type, as (R)c
+template <typename R>
+struct CoefOf;
+template <>
+struct CoefOf<double> {
+    using B = uint64_t;
+    static __device__ __forceinline__ B load(const double *p) { return coef_bits(p); }
+    static __device__ __forceinline__ double signed_value(B b, bool neg) {
+        return __longlong_as_double((long long)(b ^ (neg ? 0x8000000000000000ULL : 0ULL)));
+    }
+};
+template <>
+struct CoefOf<float> {
+    using B = float;
+    static __device__ __forceinline__ B load(const double *p) { return (float)__ldg(p); }
+    static __device__ __forceinline__ float signed_value(B v, bool neg) { return neg ? -v : v; }
+};
+
+// sum_k c_k (-1)^popcount(s & z_k) over group g, stopping at the first zero coefficient.  A part that
+// is zero adds nothing (the sums start at +0, so they never become -0).
 template <typename R>
 __device__ __forceinline__ cx<R> group_diag(const rq_terms_t &T, int g, uint64_t s) {
+    using C = CoefOf<R>;
     CAcc<R> d;
     const int k1 = __ldg(T.toff + g + 1);
     for (int k = __ldg(T.toff + g); k < k1; ++k) {
-        const R re = (R)__ldg(T.coef + 2 * k), im = (R)__ldg(T.coef + 2 * k + 1);
-        if (re == (R)0 && im == (R)0) break;
-        if (__popcll(s & __ldg(T.zmask + k)) & 1) d.add({-re, -im});
-        else d.add({re, im});
+        const auto re = C::load(T.coef + 2 * k), im = C::load(T.coef + 2 * k + 1);
+        const bool zr = is_zero(re), zi = is_zero(im);
+        if (zr && zi) break;
+        const bool neg = __popcll(s & __ldg(T.zmask + k)) & 1;
+        if (!zr) d.re.add(C::signed_value(re, neg));
+        if (!zi) d.im.add(C::signed_value(im, neg));
     }
     return d.get();
 }
 
-// The real part alone, for real vectors (their operators have real coefficients): half of the
-// additions, and FP64 additions are what a cached product is made of on GB300 (FP64 runs at 1/64 of
-// the FP32 rate).  The same additions in the same order as group_diag's real part.
+// The real part alone, for real vectors (their operators have real coefficients): the same additions
+// in the same order as group_diag's real part.
 template <typename R>
 __device__ __forceinline__ R group_diag_re(const rq_terms_t &T, int g, uint64_t s) {
+    using C = CoefOf<R>;
     Acc<R> d;
     const int k1 = __ldg(T.toff + g + 1);
     for (int k = __ldg(T.toff + g); k < k1; ++k) {
-        const R re = (R)__ldg(T.coef + 2 * k);
-        if (re == (R)0 && (R)__ldg(T.coef + 2 * k + 1) == (R)0) break;
-        d.add((__popcll(s & __ldg(T.zmask + k)) & 1) ? -re : re);
+        const auto re = C::load(T.coef + 2 * k);
+        if (is_zero(re)) {
+            if (is_zero(C::load(T.coef + 2 * k + 1))) break;
+            continue;
+        }
+        d.add(C::signed_value(re, __popcll(s & __ldg(T.zmask + k)) & 1));
     }
     return d.get();
 }
 
+__device__ __forceinline__ int group_terms(const rq_terms_t &T, int g) { return __ldg(T.toff + g + 1) - __ldg(T.toff + g); }
+// sums with long groups: more than three terms a group on average
+__device__ __forceinline__ bool long_groups(const rq_terms_t &T) { return T.K > 3 * (int64_t)T.J; }
+
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+__device__ __forceinline__ bool zero_bits(float v) { return v == 0.f; }
+__device__ __forceinline__ bool zero_bits(double v) { return is_zero((uint64_t)__double_as_longlong(v)); }
+__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
+__device__ __forceinline__ bool finite_bits(double v) {
+    return ((uint32_t)(__double_as_longlong(v) >> 32) & 0x7FF00000u) != 0x7FF00000u;
+}
 
 // One element's contribution to its row and the row's accumulator: a complex value for complex
 // vectors, a real one for real vectors (the product rounded on its own, as cmul's is).  scaled is
@@ -52,7 +95,10 @@ struct RowTerm<V, true> {
     using P = cx<R>;
     using A = CAcc<R>;
     static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const V *x, int64_t m) {
-        return cmul(group_diag<R>(T, g, s), VT<V>::ld(x, m));
+        const cx<R> d = group_diag<R>(T, g, s), v = VT<V>::ld(x, m);
+        // a real diagonal times a finite value: the products with zero change nothing
+        if (zero_bits(d.im) && finite_bits(v.re) && finite_bits(v.im)) return {mul_rn(d.re, v.re), mul_rn(d.re, v.im)};
+        return cmul(d, v);
     }
     static __device__ __forceinline__ P scaled(R d, const V *x, int64_t i) {
         const cx<R> v = VT<V>::ld(x, i);
@@ -104,14 +150,21 @@ inline int tile_rows(int64_t D, int64_t nnz, int sms) {
 }
 
 // Rows [r0, r0 + nr), nr <= kTileRows: elem(e) is element e's product, first(i, acc) adds what
-// precedes the elements of row i, done(i, acc) stores.  All threads of the block call it.
-template <typename V, typename E, typename F, typename S>
-__device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, int nr, E &&elem, F &&first,
-                                             S &&done) {
+// precedes the elements of row i, done(i, acc) stores.  All threads of the block call it.  With
+// `split` elements of more than kShortTerms terms (terms(e) of them) wait for a second round, where
+// they stand together: a warp's additions cost what its longest group costs (molecules: 2 to 24
+// terms, most of them 2 or 4; 36 qubits, 150,001 rows, float64: 941 -> 738 us).
+constexpr int kShortTerms = 4;
+template <typename V, typename E, typename N, typename F, typename S>
+__device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, int nr, bool split, E &&elem,
+                                             N &&terms, F &&first, S &&done) {
     using RT = RowTerm<V>;
     constexpr int kT = tile_elems<V>();
     __shared__ int rp[kTileRows + 1];
     __shared__ __align__(16) unsigned char buf[kTileBytes];
+    __shared__ uint16_t late[kT];
+    __shared__ int nlate;
+    if (threadIdx.x == 0) nlate = 0;
     typename RT::P *prod = reinterpret_cast<typename RT::P *>(buf);
     const int64_t base = __ldg(rowptr + r0);
     for (int k = threadIdx.x; k <= nr; k += blockDim.x) rp[k] = (int)(__ldg(rowptr + r0 + k) - base);
@@ -123,8 +176,17 @@ __device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, 
     const int a = own ? rp[threadIdx.x] : 0, b = own ? rp[threadIdx.x + 1] : 0;
     for (int t0 = 0; t0 < n; t0 += kT) {
         const int m = min(kT, n - t0);
-        for (int k = threadIdx.x; k < m; k += blockDim.x) prod[k] = elem(base + t0 + k);
+        for (int k = threadIdx.x; k < m; k += blockDim.x) {
+            if (split && terms(base + t0 + k) > kShortTerms) late[atomicAdd(&nlate, 1)] = (uint16_t)k;
+            else prod[k] = elem(base + t0 + k);
+        }
         __syncthreads();
+        if (split) {
+            const int nl = nlate;
+            for (int q = threadIdx.x; q < nl; q += blockDim.x) prod[late[q]] = elem(base + t0 + late[q]);
+            __syncthreads();
+            if (threadIdx.x == 0) nlate = 0;  // (two barriers before the next pass adds to it)
+        }
         for (int k = max(a - t0, 0); k < min(b - t0, m); ++k) acc.add(prod[k]);
         __syncthreads();
     }

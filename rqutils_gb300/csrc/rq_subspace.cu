@@ -2,6 +2,7 @@
 //   rq_subspace_build  -- strict-increase check, empty-key choice, hash table, sector filter
 //   rq_xsource         -- get_xsource (rqutils/sqd.py:448-503) for any number of X masks
 //   rq_diagonal        -- get_diagonal (rqutils/sqd.py:554-575), stopping at the first zero
+#include <algorithm>
 #include <string>
 
 #include "rq_common.cuh"
@@ -44,8 +45,8 @@ __global__ void k_fill_u64(uint64_t *p, int64_t n, uint64_t v) {
 // presence bitmap: bit (hash(key) >> (32 - pbits)) for every key
 template <int KB>
 __global__ void k_pmap_build(const uint64_t *__restrict__ keys, int64_t D, uint32_t *pmap, int pbits) {
-    __shared__ uint32_t T[kHashTableWords];
-    init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    __shared__ __align__(16) uint32_t T[kHashTableWords];
+    copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -58,8 +59,8 @@ template <int KB>
 __global__ void __launch_bounds__(kThreads)
 k_hash_insert(const uint64_t *__restrict__ states, int64_t D, void *keys, int32_t *vals, int hbits,
               uint64_t empty, int *err) {
-    __shared__ uint32_t T[kHashTableWords];
-    init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    __shared__ __align__(16) uint32_t T[kHashTableWords];
+    copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     constexpr int kSlots = kBucketSlots;
     const uint32_t mask = (1u << hbits) - 1u;
@@ -92,19 +93,44 @@ k_hash_insert(const uint64_t *__restrict__ states, int64_t D, void *keys, int32_
     }
 }
 
-// Highest differing bit of neighbouring sorted states: hist[h] counts the i with
-// 63 - clz(s[i] ^ s[i - 1]) == h.  The number of distinct prefixes s >> b is then
-// 1 + sum_{h >= b} hist[h] for every b at once.
+// Prefix statistics of sorted states for every shift b at once: hist[h] counts the i with
+// 63 - clz(s[i] ^ s[i - 1]) == h, so that the number of distinct prefixes s >> b is
+// 1 + sum_{h >= b} hist[h]; for kRunSamples rows spread over the array, hist[64 + b] adds the number
+// of the 2 kRunReach neighbours that share the row's prefix s >> b, and the row itself.  One warp per
+// sample: its neighbours' highest differing bits at once, then a count per shift.
+constexpr int kRunSamples = 512;
+constexpr int kRunReach = 64;
 __global__ void k_prefix_hist(const uint64_t *__restrict__ s, int64_t D,
                               unsigned long long *__restrict__ hist) {
-    __shared__ unsigned int h[64];
-    if (threadIdx.x < 64) h[threadIdx.x] = 0u;
+    __shared__ unsigned int h[128];
+    for (int k = threadIdx.x; k < 128; k += blockDim.x) h[k] = 0u;
     __syncthreads();
     for (int64_t i = 1 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D;
          i += (int64_t)gridDim.x * blockDim.x)
         atomicAdd(&h[63 - __clzll((long long)(s[i] ^ s[i - 1]))], 1u);
+    const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
+    unsigned int run[2] = {0u, 0u};  // of shifts lane and lane + 32
+    for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < kRunSamples; k += warps) {
+        const int64_t i = D * k / kRunSamples;
+        const uint64_t v = s[i];
+        uint64_t diff[2 * kRunReach / 32];  // neighbours' differing bits; all ones past the ends
+#pragma unroll
+        for (int q = 0; q < 2 * kRunReach / 32; ++q) {
+            const int64_t j = i - kRunReach + 32 * q + lane + (32 * q >= kRunReach ? 1 : 0);
+            diff[q] = j >= 0 && j < D ? s[j] ^ v : ~0ULL;
+        }
+        for (int b = 0; b < 64; ++b) {
+            unsigned int n = 1u;
+#pragma unroll
+            for (int q = 0; q < 2 * kRunReach / 32; ++q) n += __popc(__ballot_sync(0xffffffffu, (diff[q] >> b) == 0ULL));
+            if ((b & 31) == lane) run[b >> 5] += n;
+        }
+    }
+    atomicAdd(&h[64 + lane], run[0]);
+    atomicAdd(&h[96 + lane], run[1]);
     __syncthreads();
-    if (threadIdx.x < 64 && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, (unsigned long long)h[threadIdx.x]);
+    for (int k = threadIdx.x; k < 128; k += blockDim.x)
+        if (h[k]) atomicAdd(hist + k, (unsigned long long)h[k]);
 }
 
 // Line filter: for every state s with h = hash(s), word (h mod 2^lwbits) >> 5 of line
@@ -116,8 +142,8 @@ template <int KB>
 __global__ void __launch_bounds__(kThreads)
 k_line_build(const uint64_t *__restrict__ s, int64_t D, uint32_t *__restrict__ lmap, int lbits,
              int lwbits, int lshift) {
-    __shared__ uint32_t T[kHashTableWords];
-    init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    __shared__ __align__(16) uint32_t T[kHashTableWords];
+    copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     const uint32_t bmask = (1u << lwbits) - 1u;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D;
@@ -159,12 +185,12 @@ k_xsource(const rq_subspace_t S, const uint64_t *__restrict__ xm, int J, int32_t
           int *err) {
     __shared__ uint32_t fb[RQ_FILTER_WORDS];
     __shared__ uint64_t samp[LK == RQ_LOOKUP_BSEARCH ? kSample : 1];
-    __shared__ uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 1];
+    __shared__ __align__(16) uint32_t T[LK == RQ_LOOKUP_HASH ? kHashTableWords : 4];
     for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) fb[w] = S.fbits[w];
     const int ns = (int)(S.D < kSample ? S.D : kSample);
     if (LK == RQ_LOOKUP_BSEARCH)
         for (int k = threadIdx.x; k < ns; k += blockDim.x) samp[k] = S.states[((int64_t)k * S.D) / ns];
-    if (LK == RQ_LOOKUP_HASH) init_hash_tables(T, KeyWidth<KB>::kNbytes);
+    if (LK == RQ_LOOKUP_HASH) copy_hash_tables(T, KeyWidth<KB>::kNbytes);
     __syncthreads();
     const int64_t total = (int64_t)J * S.D;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -371,15 +397,20 @@ RQ_API int rq_subspace_build(rq_subspace_t *sub, void *scratch, void *stream) {
                                    st, sub->pbits ? sub->pmap : nullptr, sub->pbits);
     if (rc != RQ_OK) return fail(rc, std::string("rq_subspace_build: ") + rq_last_error());
     if (sub->lookup == RQ_LOOKUP_HASH && sub->lmap) {
-        // prefix shift: the largest b with about 2^(lwbits - 5) states per distinct s >> b
-        // (the histogram sits in the reduction partials of the scratch, past the reduction
-        // counter, which must stay zero)
+        // prefix shift: the largest b with about 2^(lwbits - 5) states per distinct s >> b, and at
+        // most three times as many sharing the average state's prefix.  The second bound is for
+        // subspaces whose states cluster (low-energy samples of a molecule): lines of popular
+        // prefixes fill up, and targets are mostly in them (36 qubits, 150,001 rows: 473 of 2760
+        // groups pass the filter at shift 19, which the average alone would choose, 111 at shift
+        // 10; 84 are hits).  The histogram sits in the reduction partials of the scratch, past the
+        // reduction counter, which must stay zero.
         unsigned long long *hist = reinterpret_cast<unsigned long long *>(
             static_cast<char *>(scratch_reduce(scratch)) + 16);
-        RQ_CUDA(cudaMemsetAsync(hist, 0, 64 * sizeof(unsigned long long), st));
-        k_prefix_hist<<<grid_for(D), kThreads, 0, st>>>(sub->states, D, hist);
+        RQ_CUDA(cudaMemsetAsync(hist, 0, 128 * sizeof(unsigned long long), st));
+        // at least one warp per sample
+        k_prefix_hist<<<std::max(grid_for(D), kRunSamples * 32 / kThreads), kThreads, 0, st>>>(sub->states, D, hist);
         RQ_CUDA(cudaGetLastError());
-        unsigned long long h[64];
+        unsigned long long h[128];
         RQ_CUDA(cudaMemcpyAsync(h, hist, sizeof(h), cudaMemcpyDeviceToHost, st));
         RQ_CUDA(cudaStreamSynchronize(st));
         const double per = (double)(1 << (sub->lwbits - 5));
@@ -389,6 +420,7 @@ RQ_API int rq_subspace_build(rq_subspace_t *sub, void *scratch, void *stream) {
         for (int c = 1; c <= sub->key_bits; ++c) {
             above -= h[c - 1];
             if ((double)D > per * (double)(above + 1)) break;
+            if ((double)h[64 + c % 64] > 3. * per * kRunSamples && c > 1) break;
             b = c;
         }
         sub->lshift = b;

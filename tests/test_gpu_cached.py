@@ -57,3 +57,45 @@ def test_cached_products_keep_infinities_and_nan(mode):
     assert torch.equal(torch.isfinite(y), torch.isfinite(z))
     ok = torch.isfinite(y)
     assert torch.equal(y[ok], z[ok])
+
+
+def _clustered_states(rng, n, D):
+    """D states of two half-filled n / 2-bit blocks, few excitations above the lowest orbitals."""
+    half, have = n // 2, np.zeros(0, np.uint64)
+    while len(have) < D:
+        words = np.zeros(2 * D, np.uint64)
+        for block in range(2):
+            w = np.full(2 * D, (1 << (half // 2)) - 1, np.uint64)
+            for _ in range(3):  # up to three excitations, each with probability 1/2
+                a, b = rng.integers(0, half // 2, 2 * D), rng.integers(half // 2, half, 2 * D)
+                m = (np.uint64(1) << a.astype(np.uint64)) | (np.uint64(1) << b.astype(np.uint64))
+                ok = (rng.random(2 * D) < 0.5) & (((w >> a.astype(np.uint64)) & np.uint64(1)) == 1) & \
+                    (((w >> b.astype(np.uint64)) & np.uint64(1)) == 0)
+                w = np.where(ok, w ^ m, w)
+            words |= w << np.uint64(block * half)
+        have = np.unique(np.concatenate([have, words]))
+    return np.sort(rng.choice(have, size=D, replace=False))
+
+
+# one to 32 lanes per row, 32- and 64-bit keys, more hits between two resolutions than the queue
+# holds, and (36 qubits) the clustered launch: several passes, the sector test, spread tiles
+@pytest.mark.parametrize('n,keep,D', [(20, 3000, 100), (20, 3000, 2500), (28, 4000, 30001), (36, 6000, 60000)])
+@pytest.mark.parametrize('dtype', ['float32', 'float64', 'complex64', 'complex128'])
+def test_clustered_subspaces(n, keep, D, dtype):
+    import torch
+    from rqutils_gb300 import workloads
+    from rqutils_gb300.device import DeviceOperator, DeviceSubspace, DeviceTerms
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    rng = np.random.default_rng(n)
+    ham = PauliSumXZ.from_paulisum(workloads.chemistry_jw(n // 2, rng, keep=keep), force_real=True,
+                                   add_padding=True)
+    S = _clustered_states(rng, n, D)
+    terms = DeviceTerms(ham)
+    x = torch.randn(D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(D))
+    y = DeviceOperator(terms, DeviceSubspace(S, num_qubits=n, line_filter=False), mode='free').matvec(x)
+    for masks in (None, (0, 0), ((1 << n // 4) - 1, ((1 << n) - 1) ^ ((1 << n // 4) - 1))):
+        sub = DeviceSubspace(S, num_qubits=n, filter_masks=masks)
+        assert torch.equal(DeviceOperator(terms, sub, mode='free').matvec(x), y)
+    conn = DeviceOperator(terms, sub, mode='conn')
+    assert conn.nnz >= 2 * D  # 3 to 40 a row
+    assert torch.equal(conn.matvec(x), y)
