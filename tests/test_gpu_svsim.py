@@ -93,3 +93,25 @@ def test_svsim_matches_reference_fixtures(name):
     init = d['initial'] if d['initial'].ndim else int(d['initial'])
     got = svsim(d['circuit'], init)
     np.testing.assert_array_equal(got.cpu().numpy(), d['final'])
+
+
+@pytest.mark.parametrize('n', [1, 2, 3, 4, 5, 11, 12, 15])
+def test_tiles_and_wide_gates_bit_exact(n):
+    """Segments of gates on tiles, at the sizes where the tile's index bits run out: X masks on the
+    lowest and highest qubits, on more qubits than a tile has bits (one pass of their own), more
+    diagonal gates in a row than a segment holds, and cos or sin of 0 and 1."""
+    from oracle import svsim as osv
+    from rqutils_gb300.svsim import CircuitXZ, svsim
+    rng = np.random.default_rng(n)
+    N = 1 << n
+    x = [0] * 300 + [1, N - 1, N >> 1] + list(rng.integers(0, N, 40)) + [1 << int(q) for q in rng.integers(0, n, 60)]
+    x = np.array(x, dtype=np.int64)
+    z = rng.integers(0, N, len(x))
+    ang = rng.uniform(-np.pi, np.pi, len(x))
+    c, s = np.cos(ang), np.sin(ang)
+    c[::7], s[::7] = 0., -1.
+    c[3::11], s[3::11] = 1., 0.
+    s[5::13] = 1.
+    psi0 = rng.normal(size=N) + 1j * rng.normal(size=N)
+    got = svsim(CircuitXZ(x, z, c, s, n), initial_state=psi0).cpu().numpy()
+    assert np.array_equal(got, osv.svsim(x, z, c, s, n, initial_state=psi0))
