@@ -164,6 +164,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int q = 0; q < 32; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// 16 consecutive FP32 columns of this thread's TMEM lane
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
+}
+
 // ---------------------------------------------------------------------------------------------
 // activations
 // ---------------------------------------------------------------------------------------------
@@ -349,11 +363,17 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
         }
     } else if constexpr (EPI == EPI_HEAD || EPI == EPI_HEAD_TRAIN) {
         // pass 1: Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this half
-        float o0 = 0.f, o1 = 0.f;
+        // (in quarters of 64 columns, as the fused inference adds them)
+        float o0 = 0.f, o1 = 0.f, p0 = 0.f, p1 = 0.f;
 #pragma unroll 1
         for (int g0 = 0; g0 < kHalf; g0 += 32) {
             const int c0 = col0 + g0;
             float z[32], w[32];
+            if (g0 == kHalf / 2) {
+                p0 = o0;
+                p1 = o1;
+                o0 = o1 = 0.f;
+            }
             tmem_ld32(taddr + (uint32_t)c0, z);
             lds32(cst + c0, w);
 #pragma unroll
@@ -368,6 +388,8 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
 #pragma unroll
             for (int i = 0; i < 32; ++i) o1 += z[i] * w[i];
         }
+        o0 = p0 + o0;
+        o1 = p1 + o1;
         if (h == 1) {
             xch[par][row][0] = o0;
             xch[par][row][1] = o1;
@@ -753,6 +775,255 @@ int launch_gemm(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_t 
 }
 
 // ---------------------------------------------------------------------------------------------
+// fused inference
+// ---------------------------------------------------------------------------------------------
+// Both layers and the output layer of a 128-row tile in one persistent kernel: the hidden activations
+// H1 go from the epilogue warps to shared memory (the 128-byte swizzled layout that the MMA reads) and
+// never to HBM; as two GEMMs they were written and read back, 134 MB each way for 2^18 rows.  W1 and
+// W2 (160 KB) stay in shared memory, which leaves one tile of X (16 KB) and two of H1's four 64-column
+// quarters (32 KB).  TMEM holds both accumulators (2 x 256 columns).  Bound by the epilogue warps,
+// about 11 instructions per hidden unit of each layer: sixteen of them (eight left three of four issue
+// slots empty).  2^18 rows: 113 us as two GEMMs, 100 with eight epilogue warps, 74 with sixteen.
+constexpr uint32_t kInfW2 = 0, kInfW1 = 4 * 32768, kInfA = kInfW1 + 32768, kInfH = kInfA + kTileABytes,
+                   kInfEnd = kInfH + 2 * kTileABytes;  // 208 KB
+constexpr int kInfWarps = 16;                  // epilogue warps
+constexpr int kInfThreads = 64 + 32 * kInfWarps;
+
+struct InferArgs {
+    int64_t M, tiles;
+    const float *params;
+    float *out;  // [M][2]
+    int *err;
+};
+
+struct InferShared {
+    uint64_t wfull, afull, aempty, d1full, d1empty, d2full, d2empty, hfull[2], hempty[2], fin;
+    uint32_t tmem;
+    int abort, wwait;
+    int64_t issued, consumed;  // X tiles
+    __align__(16) float cst[4 * kHid];     // b1 | b2 | W3 row 0 | W3 row 1
+    float xch[2][3][kTileM][2];            // output sums of the column quarters 1..3
+};
+
+__global__ void __launch_bounds__(kInfThreads, 1)
+k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w1,
+        const __grid_constant__ CUtensorMap tma_w2, const InferArgs g) {
+    // all of it dynamic, so that the operand tiles start at the beginning of the block's memory,
+    // which is 1 KB aligned (checked: there is no room for slack)
+    extern __shared__ __align__(1024) unsigned char smem[];
+    InferShared &sh = *reinterpret_cast<InferShared *>(smem + kInfEnd);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t sbase = smem_u32(smem);
+    constexpr uint32_t kIdesc = make_idesc(kTileM, kHid);
+    if ((sbase & 1023u) != 0u) {
+        if (threadIdx.x == 0) atomicExch(g.err, RQ_E_CUDA);
+        return;
+    }
+    if (threadIdx.x == 0) {
+        mbar_init(&sh.wfull, 1);
+        mbar_init(&sh.afull, 1);
+        mbar_init(&sh.aempty, 1);
+        mbar_init(&sh.d1full, 1);
+        mbar_init(&sh.d1empty, kInfWarps);
+        mbar_init(&sh.d2full, 1);
+        mbar_init(&sh.d2empty, kInfWarps);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&sh.hfull[s], kInfWarps);
+            mbar_init(&sh.hempty[s], 1);
+        }
+        mbar_init(&sh.fin, 1);
+        fence_mbar_init();
+        sh.abort = sh.wwait = 0;
+        sh.issued = sh.consumed = 0;
+    }
+    if (warp == 1) tmem_alloc(&sh.tmem, 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem;
+    volatile int *abort_p = &sh.abort;
+
+    if (warp == 0) {  // ---- TMA producer
+        if (lane == 0) {
+            mbar_expect_tx(&sh.wfull, 5 * 32768);
+            tma_load_2d(sbase + kInfW1, &tma_w1, 0, 0, &sh.wfull);
+            for (int c = 0; c < 4; ++c) tma_load_2d(sbase + kInfW2 + 32768u * (uint32_t)c, &tma_w2, c * kChunkK, 0, &sh.wfull);
+        }
+        int64_t it = 0;
+        for (int64_t u = blockIdx.x; u < g.tiles; u += gridDim.x, ++it) {
+            if (it >= 1 && !wait_bar(&sh.aempty, (uint32_t)((it - 1) & 1), abort_p)) break;
+            if (lane == 0) {
+                mbar_expect_tx(&sh.afull, kTileABytes);
+                tma_load_2d(sbase + kInfA, &tma_x, 0, (int)(u * kTileM), &sh.afull);
+                sh.issued = it + 1;
+            }
+            __syncwarp();
+        }
+    } else if (warp == 1) {  // ---- MMA issuer
+        bool ok = wait_bar(&sh.wfull, 0u, abort_p);
+        if (ok && lane == 0) sh.wwait = 1;
+        int64_t it = 0, hq = 0;
+        for (int64_t u = blockIdx.x; u < g.tiles && ok; u += gridDim.x, ++it) {
+            ok = wait_bar(&sh.afull, (uint32_t)(it & 1), abort_p) &&
+                 (it < 1 || wait_bar(&sh.d1empty, (uint32_t)((it - 1) & 1), abort_p));
+            if (!ok) break;
+            tc_fence_after();
+            if (lane == 0) {
+#pragma unroll
+                for (int kk = 0; kk < kChunkK / 16; ++kk)
+                    mma_bf16(tmem, make_sdesc_sw128(sbase + kInfA + (uint32_t)kk * 32u),
+                             make_sdesc_sw128(sbase + kInfW1 + (uint32_t)kk * 32u), kIdesc, kk > 0 ? 1u : 0u);
+                mma_commit(&sh.aempty);
+                mma_commit(&sh.d1full);
+                sh.consumed = it + 1;
+            }
+            __syncwarp();
+            if (it >= 1 && !wait_bar(&sh.d2empty, (uint32_t)((it - 1) & 1), abort_p)) break;
+            for (int q = 0; q < 4; ++q, ++hq) {
+                const int s = (int)(hq & 1);
+                ok = wait_bar(&sh.hfull[s], (uint32_t)((hq >> 1) & 1), abort_p);
+                if (!ok) break;
+                tc_fence_after();
+                if (lane == 0) {
+                    const uint32_t a = sbase + kInfH + kTileABytes * (uint32_t)s, b = sbase + kInfW2 + 32768u * (uint32_t)q;
+#pragma unroll
+                    for (int kk = 0; kk < kChunkK / 16; ++kk)
+                        mma_bf16(tmem + kHid, make_sdesc_sw128(a + (uint32_t)kk * 32u), make_sdesc_sw128(b + (uint32_t)kk * 32u),
+                                 kIdesc, (q > 0 || kk > 0) ? 1u : 0u);
+                    mma_commit(&sh.hempty[s]);
+                    if (q == 3) mma_commit(&sh.d2full);
+                }
+                __syncwarp();
+            }
+        }
+    } else {  // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31; quarter (w - 2) / 4 of the columns
+        const int q4 = warp & 3, cq = (warp - 2) >> 2, row = 32 * q4 + lane, e = threadIdx.x - 64;
+        constexpr int kThreadsE = 32 * kInfWarps;
+        const uint32_t lanes = tmem + ((uint32_t)(32 * q4) << 16);
+        for (int i = e; i < kHid; i += kThreadsE) {
+            sh.cst[i] = g.params[kOffB1 + i];
+            sh.cst[kHid + i] = g.params[kOffB2 + i];
+            sh.cst[2 * kHid + i] = g.params[kOffW3 + i];
+            sh.cst[3 * kHid + i] = g.params[kOffW3 + kHid + i];
+        }
+        named_bar_sync(kEpiBar, kThreadsE);
+        int64_t it = 0, hq = 0;
+        for (int64_t u = blockIdx.x; u < g.tiles; u += gridDim.x, ++it) {
+            bool ok = wait_bar(&sh.d1full, (uint32_t)(it & 1), abort_p);
+            tc_fence_after();
+            for (int q = 0; q < 4; ++q, ++hq) {  // H1 quarter by quarter; this warp's 16 columns of it
+                const int s = (int)(hq & 1);
+                ok = ok && (hq < 2 || wait_bar(&sh.hempty[s], (uint32_t)(((hq >> 1) - 1) & 1), abort_p));
+                if (!ok) continue;
+                const int c0 = 64 * q + 16 * cq;
+                float z[16];
+                tmem_ld16(lanes + (uint32_t)c0, z);
+                if (q == 3) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.d1empty);
+                }
+                __align__(16) bf16 o[16];
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 b = *reinterpret_cast<const float4 *>(sh.cst + c0 + i);
+                    o[i] = __float2bfloat16_rn(gelu(z[i] + b.x));
+                    o[i + 1] = __float2bfloat16_rn(gelu(z[i + 1] + b.y));
+                    o[i + 2] = __float2bfloat16_rn(gelu(z[i + 2] + b.z));
+                    o[i + 3] = __float2bfloat16_rn(gelu(z[i + 3] + b.w));
+                }
+                // 16-byte chunk c of row r sits at chunk c ^ (r mod 8) of the row's 128 bytes
+                unsigned char *dst = smem + kInfH + kTileABytes * (uint32_t)s + row * 128;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    *reinterpret_cast<uint4 *>(dst + (((2 * cq + j) ^ (row & 7)) << 4)) = reinterpret_cast<const uint4 *>(o)[j];
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the MMA reads through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.hfull[s]);
+            }
+            ok = ok && wait_bar(&sh.d2full, (uint32_t)(it & 1), abort_p);
+            if (named_bar_or(kEpiBar, kThreadsE, !ok || *abort_p != 0)) break;  // the same answer in every epilogue thread
+            tc_fence_after();
+            // Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this quarter
+            float o0 = 0.f, o1 = 0.f;
+#pragma unroll 1
+            for (int g0 = 0; g0 < kHid / 4; g0 += 32) {
+                const int c0 = cq * (kHid / 4) + g0;
+                float z[32], w[32];
+                tmem_ld32(lanes + (uint32_t)(kHid + c0), z);
+                lds32(sh.cst + kHid + c0, w);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) z[i] += w[i];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) z[i] = gelu(z[i]);
+                lds32(sh.cst + 2 * kHid + c0, w);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) o0 += z[i] * w[i];
+                lds32(sh.cst + 3 * kHid + c0, w);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) o1 += z[i] * w[i];
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.d2empty);
+            float (*x)[kTileM][2] = sh.xch[it & 1];
+            if (cq > 0) {
+                x[cq - 1][row][0] = o0;
+                x[cq - 1][row][1] = o1;
+            }
+            named_bar_sync(kEpiBar, kThreadsE);
+            if (cq == 0) {
+                const int64_t m = u * kTileM + row;
+                o0 = (o0 + x[0][row][0]) + ((x[1][row][0] + x[2][row][0]) + __ldg(g.params + kOffB3));
+                o1 = (o1 + x[0][row][1]) + ((x[1][row][1] + x[2][row][1]) + __ldg(g.params + kOffB3 + 1));
+                if (m < g.M) {
+                    g.out[2 * m] = o0;
+                    g.out[2 * m + 1] = o1;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (sh.abort != 0) {
+        // let the copies and MMAs already issued land before the memory is released
+        if (threadIdx.x == 0) {
+            if (sh.consumed < sh.issued) wait_bar(&sh.afull, (uint32_t)((sh.issued - 1) & 1), nullptr);
+            if (!sh.wwait) wait_bar(&sh.wfull, 0u, nullptr);
+            atomicExch(g.err, RQ_E_CUDA);
+        }
+        if (warp == 1) {
+            if (lane == 0) mma_commit(&sh.fin);
+            __syncwarp();
+            wait_bar(&sh.fin, 0u, nullptr);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+int launch_infer(const rq_mlp_t *m, int64_t rows, const bf16 *x, float *out, int *err, cudaStream_t st) {
+    CUtensorMap tx, t1, t2;
+    RQ_TRY(make_tma(&tx, x, kIn, rows, kIn, kTileM));
+    RQ_TRY(make_tma(&t1, reinterpret_cast<const bf16 *>(m->w1b), kIn, kHid, kIn, kHid));
+    RQ_TRY(make_tma(&t2, reinterpret_cast<const bf16 *>(m->w2b), kHid, kHid, kHid, kHid));
+    constexpr size_t smem = kInfEnd + sizeof(InferShared);
+    static_assert(smem <= 227 * 1024, "one block's shared memory");
+    thread_local KernelLaunchCache table[kMaxCachedDevices];
+    KernelLaunchCache *c = nullptr;
+    int per_sm = 1;
+    RQ_TRY(cache_slot(table, &c));
+    RQ_TRY(configure_kernel(k_infer, *c, smem, kInfThreads, &per_sm));
+    const InferArgs g{rows, (rows + kTileM - 1) / kTileM, m->params, out, err};
+    k_infer<<<(unsigned)std::min<int64_t>(g.tiles, sm_count()), kInfThreads, smem, st>>>(tx, t1, t2, g);
+    RQ_CUDA(cudaGetLastError());
+    return RQ_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
 // elementwise kernels
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // SplitMix64 finaliser
@@ -780,10 +1051,27 @@ __device__ __forceinline__ void write_features(bf16 *row, uint64_t s, double u) 
     }
 }
 
-__global__ void k_features(const uint64_t *__restrict__ S, int64_t D, double U, bf16 *__restrict__ x) {
-    const double u = (U - 5.0) / 3.0;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D; k += (int64_t)gridDim.x * blockDim.x)
-        write_features(x + k * kIn, S[k], u);
+// A thread per 16-byte piece of a row, so that a warp writes 512 contiguous bytes; the features of U
+// are computed once, on the host (FP64 arithmetic per row took half of the kernel: 14.5 -> 8.4 us for
+// 2^18 rows).
+struct UFeatures {
+    float u[3];
+};
+__global__ void k_features(const uint64_t *__restrict__ S, int64_t D, const UFeatures f, bf16 *__restrict__ x) {
+    constexpr int kPieces = kIn / 8;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D * kPieces; k += (int64_t)gridDim.x * blockDim.x) {
+        const int p = (int)(k % kPieces);
+        __align__(16) bf16 b[8];
+        if (p < 4) {
+            const uint32_t s = (uint32_t)(__ldg(S + k / kPieces) >> (8 * p));
+#pragma unroll
+            for (int q = 0; q < 8; ++q) b[q] = __float2bfloat16_rn((s >> q) & 1u ? 1.f : -1.f);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) b[q] = __float2bfloat16_rn(p == 4 && q < 3 ? f.u[q < 3 ? q : 0] : 0.f);
+        }
+        *reinterpret_cast<uint4 *>(x + k * 8) = *reinterpret_cast<const uint4 *>(b);
+    }
 }
 
 __global__ void k_sample(const uint64_t *__restrict__ S, int64_t D, const double *__restrict__ U,
@@ -1095,7 +1383,9 @@ RQ_API int rq_mlp_sync(const rq_mlp_t *m, void *stream) {
 
 RQ_API int rq_mlp_features(const uint64_t *states, int64_t D, double U, uint16_t *x, void *stream) {
     if (!states || !x || D < 1) return fail(RQ_E_ARG, "rq_mlp_features: bad arguments");
-    k_features<<<grid_for(D), kThreads, 0, as_stream(stream)>>>(states, D, U, reinterpret_cast<bf16 *>(x));
+    const double u = (U - 5.0) / 3.0;
+    const UFeatures f{{(float)u, (float)(u * u), (float)(u * u * u)}};
+    k_features<<<grid_for(D * (kIn / 8)), kThreads, 0, as_stream(stream)>>>(states, D, f, reinterpret_cast<bf16 *>(x));
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -1207,24 +1497,7 @@ RQ_API int rq_mlp_infer(const rq_mlp_t *m, int64_t rows, const uint16_t *x, floa
     cudaStream_t st = as_stream(stream);
     int *err = reinterpret_cast<int *>(w + L.err);
     RQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-    GemmArgs g{};
-    g.M = rows;
-    g.nsplit = 1;
-    g.bias = m->params + kOffB1;
-    g.h_rm = reinterpret_cast<bf16 *>(w + L.h1);
-    g.err = err;
-    RQ_TRY((launch_gemm<kHid, EPI_HIDDEN>(reinterpret_cast<const bf16 *>(x), kIn,
-                                          reinterpret_cast<const bf16 *>(m->w1b), kIn, kIn, g, st)));
-    GemmArgs h{};
-    h.M = rows;
-    h.nsplit = 1;
-    h.bias = m->params + kOffB2;
-    h.out = out;
-    h.w3 = m->params + kOffW3;
-    h.b3 = m->params + kOffB3;
-    h.err = err;
-    return launch_gemm<kHid, EPI_HEAD>(reinterpret_cast<const bf16 *>(w + L.h1), kHid,
-                                       reinterpret_cast<const bf16 *>(m->w2b), kHid, kHid, h, st);
+    return launch_infer(m, rows, reinterpret_cast<const bf16 *>(x), out, err, st);
 }
 
 RQ_API int rq_mlp_loss(int64_t rows, const float *out, const float *tgt, float *dout, double *loss, void *ws,

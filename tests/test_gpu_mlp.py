@@ -262,3 +262,17 @@ def test_hubbard_family_and_learned_start_small():
         assert rl['iterations'] < rr['iterations'], (rl, rr)
     assert (sum(r['iterations'] for r in res['learned']) <=
             0.8 * sum(r['iterations'] for r in res['random'])), res
+
+
+@pytest.mark.parametrize('rows', [1, 127, 128, 129, 152 * 128, 152 * 128 + 1, 3 * 152 * 128 - 5])
+def test_fused_inference_equals_forward_bits(rows):
+    """infer() (one kernel, activations on chip) = forward() (two GEMMs) bit for bit: one tile and
+    ragged tiles, one and several tiles per SM."""
+    import torch
+    from rqutils_gb300.warmstart import WarmStartMLP
+    m = WarmStartMLP(seed=rows)
+    x = torch.randn((rows, 64), device='cuda', generator=torch.Generator('cuda').manual_seed(rows)).to(torch.bfloat16)
+    guard = torch.full((rows + 1, 2), 7., device='cuda')
+    m.infer(x, out=guard[:rows])
+    assert torch.equal(guard[:rows], m.forward(x)) and bool((guard[rows:] == 7.).all())
+    m.check_errors()
