@@ -209,7 +209,17 @@ def ptr(t):
     return None if t is None else int(t.data_ptr())
 
 
+_raw_stream = _get_device = None
+
+
 def stream_ptr(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    """The CUDA stream of a call as an int: ``stream``, or torch's current one."""
+    global _raw_stream, _get_device
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.current_stream()  # initialises CUDA
+        _get_device = torch._C._cuda_getDevice
+        _raw_stream = torch._C._cuda_getCurrentRawStream
+    return _raw_stream(_get_device())

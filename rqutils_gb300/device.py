@@ -240,8 +240,10 @@ class DeviceOperator:
         x = x.contiguous()
         if out is None:
             out = torch.empty_like(x)
-        L.check(L.lib().rq_matvec(ctypes.byref(self.c), vt, L.ptr(x), L.ptr(out),
-                                  L.ptr(self.scratch), L.stream_ptr(stream)), 'rq_matvec')
+        rc = L.lib().rq_matvec(self.c, vt, x.data_ptr(), out.data_ptr(), self.scratch.data_ptr(),
+                               L.stream_ptr(stream))
+        if rc:
+            L.check(rc, 'rq_matvec')
         return out
 
     __call__ = matvec

@@ -262,20 +262,20 @@ class PauliSumXZ:
         (PauliSumXZ.matmul, symplectic.py:142-147)."""
         J = len(self.xmask)
         coef = self.coef.astype(np.complex128)
-        keep = np.ones(len(coef), dtype=bool)
-        if truncate:
-            zero = coef == 0
-            for j in range(J):
-                a, b = int(self.toff[j]), int(self.toff[j + 1])
-                zs = np.nonzero(zero[a:b])[0]
-                if len(zs):
-                    keep[a + zs[0]:b] = False
-        counts = np.array([int(keep[self.toff[j]:self.toff[j + 1]].sum()) for j in range(J)],
-                          dtype=np.int64) if J else np.zeros(0, np.int64)
-        toff = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+        toff, zmask = self.toff, self.zmask
+        zero = np.flatnonzero(coef == 0) if truncate else ()
+        if len(zero):
+            group = np.repeat(np.arange(J), np.diff(toff))
+            end = np.array(toff[1:])  # one past the last kept term: the group's first zero
+            np.minimum.at(end, group[zero], zero)
+            keep = np.arange(len(coef)) < end[group]
+            zmask, coef_kept = zmask[keep], coef[keep]
+            toff = np.concatenate([[0], np.cumsum(end - toff[:-1])])
+        else:
+            zmask, coef_kept = zmask.copy(), coef
         diag = np.nonzero(self.xmask == 0)[0]
         diag_group = int(diag[0]) if len(diag) else -1
-        return (self.xmask.copy(), toff, self.zmask[keep].copy(), coef[keep].copy(), diag_group,
+        return (self.xmask.copy(), np.asarray(toff, dtype=np.int32), zmask, coef_kept, diag_group,
                 bool(np.all(coef.imag == 0)))
 
     # ------------------------------------------------------------------------------------------
