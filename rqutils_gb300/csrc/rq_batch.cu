@@ -80,9 +80,12 @@ __global__ void k_batch_diag(const uint64_t *__restrict__ keys, int64_t D, const
         if (g >= 0) {
             const int k1 = __ldg(T.toff + g + 1);
             for (int t = __ldg(T.toff + g); t < k1; ++t) {
-                const double c = __ldg(T.coef + 2 * t);
-                if (c == 0. && __ldg(T.coef + 2 * t + 1) == 0.) break;
-                d += (__popcll(s & __ldg(T.zmask + t)) & 1) ? -c : c;
+                const uint64_t c = coef_bits(T.coef + 2 * t);
+                if (is_zero(c)) {
+                    if (is_zero(coef_bits(T.coef + 2 * t + 1))) break;
+                    continue;
+                }
+                d += CoefOf<double>::signed_value(c, __popcll(s & __ldg(T.zmask + t)) & 1);
             }
         }
         out[i] = d;

@@ -16,8 +16,13 @@
 #include "rq_common.cuh"
 #include "rq_rows.cuh"
 #include "rq_host.h"
+#include "rq_line.cuh"
 
 namespace rq {
+
+// rq_conn.cu: row counts (col null: rows[i] = elements of row i) or the lists at rows[i]
+int conn_line(const rq_operator_t &op, int64_t *rows, int32_t *col, int32_t *grp, void *val, int32_t vtype, int *err,
+              cudaStream_t st);
 
 namespace {
 
@@ -157,266 +162,48 @@ __device__ inline void load_lookup_smem(const rq_subspace_t &S, uint32_t *fb, ui
 // can be a state; the few groups that can ("hot") are resolved in the table afterwards, so that the
 // rare divergent work is not interleaved with the probes.
 //
-// k_matvec_line (a line filter is present): the probe is a two-bit test in a line chosen by the
+// k_matvec_line (a line filter is present, rq_line.cuh): the probe is a two-bit test in a line chosen by the
 // target's prefix t >> lshift.  The rows of a warp are consecutive sorted states that share their
 // high bits, so for one X group their targets share them too and the warp's probes fall in a few
 // lines.
 // k_matvec_hash (no line filter): the probe is the key bucket itself, behind the sector filter and
 // the presence bitmap.
 
-// Sector filter of the hash kernels: none, the general (popcount a, popcount b) bitset, or the
-// common case of a subspace in one sector (a single bit set: two popcount compares, no table).
-enum { kFiltNone = 0, kFiltSet = 1, kFiltPoint = 2 };
-// line filters of at most 2^25 bytes (32 MB, a quarter of GB300's L2) skip the sector test:
-// measured faster without it at 16 MB (Hubbard D = 2^20: 0.089 against 0.107 ms) and slower at
-// 64 MB (chemistry, 2^22 rows: 80.2 against 65.6 ms); clustered subspaces keep it at any size, since
-// their probes are bound by the lines a warp touches (36 qubits, 150,001 rows: 2.03 against 2.29 ms)
-constexpr int kLineFilterL2Log2Bytes = 25;
-
-// shared memory of the hash kernels: the sector bitset, the hash byte tables (64-bit keys use
-// all eight) and, in dynamic shared memory, the resident group keys
-__shared__ uint32_t hk_fb[RQ_FILTER_WORDS];
-__shared__ __align__(16) uint32_t hk_htab[kHashTableWords];
-extern __shared__ __align__(16) unsigned char hk_dyn[];
-
-// The sector test of a target for the filter form FM (pa0, pb0: the popcounts of the one sector).
-template <typename K, int FM>
-__device__ __forceinline__ bool sector_pass(K t, K fa, K fbm, int pa0, int pb0) {
-    if (FM == kFiltPoint) {
-        int pa, pb;
-        if (sizeof(K) == 8) {
-            pa = __popcll((unsigned long long)(t & fa));
-            pb = __popcll((unsigned long long)(t & fbm));
-        } else {
-            pa = __popc((unsigned)(t & fa));
-            pb = __popc((unsigned)(t & fbm));
-        }
-        return (pa == pa0) & (pb == pb0);
-    }
-    if (FM == kFiltSet) return sector_ok_k<K>(hk_fb, fa, fbm, t);
-    return true;
-}
-
-// ---- probes of the line filter ---------------------------------------------------------------
-// What bounds it: instruction issue and L2 latency when hits are rare (Hubbard 4x4, 2^20 rows: 0.24
-// hits a row of 64 groups), the resolution of hits when they are not (a molecule's low-energy
-// samples: 84 of 2760 groups).  So
-// * a row is probed by w = 1 to 32 lanes: small subspaces would leave most of the chip idle, and the
-//   rows of a sample with the most hits stand together and would keep one warp busy long after the
-//   others (for such samples the tiles of a block are spread over the array, too; otherwise they
-//   stand together, because neighbouring tiles share filter lines);
-// * the hits of all lanes are gathered, in row and group order, into a queue that the whole warp
-//   resolves in full rounds (bucket, row index, terms, x): no lane waits for another's longer list,
-//   and FP64 instructions, which cost a warp the same however few lanes are active, run full;
-//   groups of more than kShortTerms terms go to a second queue, so that short ones do not wait;
-// * the owner lane of a row adds its products from the queue in group order, as the cached products do.
-// QUEUE = false: each lane resolves its own hits in a loop.  That needs fewer registers (48 warps per
-// SM instead of 32) and is the better one in 32-bit arithmetic with few groups and one lane per row
-// (Hubbard 4x4, 2^20 rows, complex64: 78 us against 83).
-constexpr int kQueueSlots = 128;  // hits resolved together
-
 template <typename V>
-struct WarpWork {
-    uint32_t hit[kQueueSlots];                   // lane << 16 | resident group, or kMissed
-    int src[kQueueSlots];                        // source row
-    typename RowTerm<V>::P prod[kQueueSlots];
-    uint8_t late[kQueueSlots];                   // queue slots of long groups
+struct UseProduct {  // y = H x
+    using RT = RowTerm<V>;
+    using R = typename VT<V>::R;
+    const rq_operator_t &op;
+    const V *x;
+    V *y;
+    typename RT::A acc;
+    __device__ __forceinline__ void start(int64_t i, uint64_t s, bool own) {
+        acc = typename RT::A();
+        if (!own) return;
+        const int skip = op.terms.diag_group;
+        if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+        else if (skip >= 0) acc.add(RT::product(op.terms, skip, s, x, i));
+    }
+    __device__ __forceinline__ void hit(int g, uint64_t s, int m) { acc.add(RT::product(op.terms, g, s, x, m)); }
+    __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int m) {
+        if (group_terms(op.terms, g) > kShortTerms) return true;
+        W.prod[q] = RT::product(op.terms, g, s, x, m);
+        return false;
+    }
+    __device__ __forceinline__ void late(WarpWork<V> &W, int q, int g, uint64_t s) {
+        W.prod[q] = RT::product(op.terms, g, s, x, W.src[q]);
+    }
+    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { acc.add(W.prod[q]); }
+    __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
 };
-constexpr uint32_t kMissed = 0xFFFFFFFFu;
-
-// Group keys in shared memory: (h(x), line word) and, for the sector test, x.  The x = 0 group is
-// left out (its diagonal is applied before the probes); resident index c is group
-// c + (c >= diag_group).  More groups than fit stream through in tiles.  Entries past the last group
-// are probed and masked out: they hold a valid word.
-template <int FM>
-__host__ __device__ constexpr size_t line_key_bytes() { return FM != kFiltNone ? 16 : 8; }
-// groups a lane probes between two resolutions (256 measured slower: 2.6 against 2.3 ms on the
-// molecule above), and the entries past the last group
-constexpr int kPart = 64;
-
-template <typename V, int BLOCK, bool QUEUE>
-__host__ __device__ constexpr size_t line_work_bytes() { return QUEUE ? (BLOCK / 32) * sizeof(WarpWork<V>) : 0; }
-
-constexpr size_t kLineSmem = 216 * 1024;  // shared memory of a block with many groups (one per SM)
-template <typename V, int FM, int BLOCK>
-__host__ __device__ constexpr int line_tile_groups() {  // groups of a tile, at most 2^16
-    return ((int)((kLineSmem - 16 * 1024 - (BLOCK / 32) * sizeof(WarpWork<V>)) / line_key_bytes<FM>()) & ~63) - kPart;
-}
-
-// Line-filter word of a key (a state or an X mask): the word index line << (lwbits - 5) | word
-// within the line, line = h(k >> lshift) >> (32 - lbits), word = (h(k) mod 2^lwbits) >> 5.  Every
-// step is linear over XOR, so the word of a target s ^ x is word(s) ^ word(x) (lbits + lwbits - 5
-// <= 32 bits, rq_line_filter_bits).
-__device__ __forceinline__ uint32_t line_word(uint32_t h, uint32_t hpre, const rq_subspace_t &S) {
-    return ((hpre >> (32 - S.lbits)) << (S.lwbits - 5)) | ((h & ((1u << S.lwbits) - 1u)) >> 5);
-}
 
 template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
 __global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : QUEUE ? 4 : 6)
 k_matvec_line(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err, int lw, int kt,
               int spread, const int *gate, const int *gate2) {
-    using R = typename VT<V>::R;
-    using RT = RowTerm<V>;
-    using K = typename KeyWidth<KB>::K;
-    constexpr int NB = KeyWidth<KB>::kNbytes;
-    // probes in flight per lane: what 64 (QUEUE) and 40 registers hold
-    constexpr int U = FM != kFiltNone ? 8 : QUEUE ? 16 : KB == 32 ? 32 : 8;
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
-    const rq_subspace_t &S = op.sub;
-    const rq_terms_t &T = op.terms;
-    const int64_t D = S.D;
-    const int skip = T.diag_group;
-    const int nres = T.J - (skip >= 0 ? 1 : 0);
-    copy_hash_tables(hk_htab, NB);
-    if (FM == kFiltSet)
-        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = S.fbits[w];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WarpWork<V> &W = reinterpret_cast<WarpWork<V> *>(hk_dyn)[QUEUE ? warp : 0];
-    uint2 *gk = reinterpret_cast<uint2 *>(hk_dyn + line_work_bytes<V, BLOCK, QUEUE>());  // [kt + kPart]
-    uint64_t *gx = reinterpret_cast<uint64_t *>(gk + kt + kPart);                       // the same, FM only
-    auto load_keys = [&](int c0, int n) {
-        for (int c = threadIdx.x; c < n + kPart; c += blockDim.x) {
-            const int j = c0 + c + (skip >= 0 && c0 + c >= skip);
-            const uint64_t xv = c < n ? T.xmask[j] : 0ULL;
-            const uint32_t h = c >= n ? 0u : T.xhash ? T.xhash[j] : lin_hash(hk_htab, xv, NB);
-            gk[c] = make_uint2(h, line_word(h, lin_hash(hk_htab, S.lshift < 64 ? xv >> S.lshift : 0ULL, NB), S));
-            if (FM != kFiltNone) gx[c] = xv;
-        }
-    };
-    __syncthreads();
-    const bool tiled = nres > kt;
-    if (!tiled) {
-        load_keys(0, nres);
-        __syncthreads();
-    }
-    const int pa0 = S.fpoint / 65, pb0 = S.fpoint % 65;
-    const K fa = (K)S.fmask_a, fbm = (K)S.fmask_b;
-    const int shift = 32 - S.hbits;
-    const uint32_t *lmap = S.lmap;
-    const unsigned lt = (1u << lane) - 1u;
-    const int w = 1 << lw, sub = lane & (w - 1);
-    const int64_t rows = 32 >> lw, stride = (int64_t)gridDim.x * (BLOCK / 32) * rows;
-    const int64_t first = (spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * (BLOCK / 32) + warp) * rows;
-    for (int64_t base = 0; base < D; base += stride) {  // the same trips for every warp of a block
-        const int64_t i = base + first + (lane >> lw);
-        const bool active = i < D;
-        if (!tiled && base + first >= D) break;
-        const int64_t ir = active ? i : D - 1;
-        const uint64_t s64 = __ldg(S.states + ir);
-        const K s = (K)s64;
-        const uint32_t hs = lin_hash(hk_htab, s64, NB);
-        // the row's line-filter word: a target's word is wrow ^ word(x), its bits those of hs ^ h(x)
-        const uint32_t wrow = line_word(hs, lin_hash(hk_htab, S.lshift < 64 ? s64 >> S.lshift : 0ULL, NB), S);
-        typename RT::A acc;
-        if (sub == 0) {
-            if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[ir], x, ir));
-            else if (skip >= 0) acc.add(RT::product(T, skip, s64, x, ir));
-        }
-        for (int t0 = 0; t0 < nres; t0 += kt) {
-            const int tn = min(kt, nres - t0);
-            if (tiled) {
-                __syncthreads();  // the previous tile is no longer read
-                load_keys(t0, tn);
-                __syncthreads();
-            }
-            // lane `sub` of a row takes the sub-th part of the next up to kPart w groups
-            int part = 0;
-            for (int g0 = 0; g0 < tn; g0 += part << lw) {
-                part = min(kPart, (tn - g0 + w - 1) >> lw);
-                const int e0 = min(g0 + sub * part, tn), en = active ? min(part, tn - e0) : 0;
-                uint64_t hot = 0ULL;
-                for (int k0 = 0; k0 < part; k0 += U) {
-                    const uint2 *key = gk + e0 + k0;
-                    uint32_t v[U];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const uint32_t *p = lmap + (wrow ^ key[u].y);
-                        v[u] = FM == kFiltNone ? __ldg(p)
-                                               : load_word(p, sector_pass<K, FM>(s ^ (K)gx[e0 + k0 + u], fa, fbm, pa0, pb0));
-                    }
-                    uint32_t hb = 0u;
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {  // (the funnel shift takes its count mod 32)
-                        const uint32_t b = hs ^ key[u].x;
-                        hb += (__funnelshift_r(v[u], 0u, b) & (v[u] >> (b >> 27)) & 1u) << u;
-                    }
-                    hot |= (uint64_t)hb << k0;
-                }
-                hot &= en >= 64 ? ~0ULL : (1ULL << en) - 1ULL;
-                if (!QUEUE) {
-                    while (hot) {
-                        const int e = e0 + __ffsll((long long)hot) - 1, c = t0 + e, gg = c + (skip >= 0 && c >= skip);
-                        hot &= hot - 1ULL;
-                        const int m = lookup_hash_at<KB>(S, s64 ^ __ldg(T.xmask + gg), (hs ^ gk[e].x) >> shift, err);
-                        if (m >= 0) acc.add(RT::product(T, gg, s64, x, m));
-                    }
-                    __syncwarp();  // re-converge before the next probes
-                    continue;
-                }
-                // resolve the hits of the warp, kQueueSlots at a time
-                const int cnt = __popcll(hot);
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += u;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                if (total == 0) continue;
-                int off = incl - cnt;
-                // the row's range of the queue
-                const int ra = __shfl_sync(0xffffffffu, off, lane & ~(w - 1));
-                const int rb = __shfl_sync(0xffffffffu, incl, lane | (w - 1));
-                for (int q0 = 0; q0 < total; q0 += kQueueSlots) {
-                    const int n = min(kQueueSlots, total - q0);
-                    while (hot && off < q0 + n) {
-                        W.hit[off - q0] = (uint32_t)lane << 16 | (uint32_t)(e0 + __ffsll((long long)hot) - 1);
-                        hot &= hot - 1ULL;
-                        ++off;
-                    }
-                    __syncwarp();
-                    int late = 0;
-                    for (int q = lane; q - lane < n; q += 32) {
-                        const bool ok = q < n;
-                        const uint32_t hit = ok ? W.hit[q] : 0u;
-                        const uint64_t rs = __shfl_sync(0xffffffffu, s64, hit >> 16);
-                        const uint32_t rh = __shfl_sync(0xffffffffu, hs, hit >> 16);
-                        bool defer = false;
-                        if (ok) {
-                            const int e = (int)(hit & 0xFFFFu), c = t0 + e, gg = c + (skip >= 0 && c >= skip);
-                            const uint64_t xv = __ldg(T.xmask + gg);
-                            const int nt = group_terms(T, gg);
-                            const int m = lookup_hash_at<KB>(S, rs ^ xv, (rh ^ gk[e].x) >> shift, err);
-                            if (m < 0) W.hit[q] = kMissed;
-                            else if (nt > kShortTerms) defer = true;
-                            else W.prod[q] = RT::product(T, gg, rs, x, m);
-                            W.src[q] = m;
-                        }
-                        const unsigned dm = __ballot_sync(0xffffffffu, defer);
-                        if (defer) W.late[late + __popc(dm & lt)] = (uint8_t)q;
-                        late += __popc(dm);
-                    }
-                    __syncwarp();
-                    for (int k = lane; k - lane < late; k += 32) {
-                        const bool ok = k < late;
-                        const int q = ok ? W.late[k] : 0;
-                        const uint32_t hit = ok ? W.hit[q] : 0u;
-                        const uint64_t rs = __shfl_sync(0xffffffffu, s64, hit >> 16);
-                        if (ok) {
-                            const int c = t0 + (int)(hit & 0xFFFFu), gg = c + (skip >= 0 && c >= skip);
-                            W.prod[q] = RT::product(T, gg, rs, x, W.src[q]);
-                        }
-                    }
-                    __syncwarp();
-                    if (sub == 0)
-                        for (int k = max(ra, q0); k < min(rb, q0 + n); ++k)
-                            if (W.hit[k - q0] != kMissed) acc.add(W.prod[k - q0]);
-                    __syncwarp();
-                }
-            }
-        }
-        if (active && sub == 0) RT::store(y, i, acc);
-    }
+    UseProduct<V> use{op, x, y, {}};
+    line_rows<V, KB, FM, BLOCK, QUEUE>(op, err, lw, kt, spread, use);
 }
 
 // ---- probes of the key buckets ----------------------------------------------------------------
@@ -902,35 +689,7 @@ int launch_hash_block(const rq_operator_t &op, const void *x, void *y, int *err,
     return RQ_OK;
 }
 
-// Clustered subspaces (low-energy samples of a molecule) with many groups: their hits crowd on some
-// rows, which stand together, and their line prefix is short, so that a warp's probes fall in many
-// lines.  The prefix shift tells them: states spread over n bits get about n - log2 D + 3, less the
-// few bits that a sector takes (measured 1 to 3; molecules 4 to 11).
-constexpr int kClusterBits = 4;
-constexpr int kClusterGroups = 256;
-inline bool clustered(const rq_subspace_t &S, int J) {
-    const uint64_t used = S.fmask_a | S.fmask_b;
-    const int n = used ? 64 - __builtin_clzll(used) : 0, d = 63 - __builtin_clzll((uint64_t)S.D);
-    return J >= kClusterGroups && n - d + 3 - S.lshift >= kClusterBits;
-}
-
-// Lanes per row (log2): the most with which all rows are still resident at once, kLineThreads
-// threads per SM.  One lane is best for large subspaces (the rows of a warp share filter lines, and
-// every lane sums a row); at 16,384 rows one lane leaves 9 of 10 warp slots of the chip empty.
-// Clustered subspaces take as many lanes as make kLineWaves passes over the chip: 36 qubits, 150,001
-// rows, float64: 2.3 against 3.8 ms with one lane, 2.6 with eight passes; spread states want one lane
-// (40 qubits, 100,000 rows: 84 us against 121 with four).
-constexpr int kLineThreads = 1024;
-constexpr int kLineWaves = 4;
 constexpr int kOwnHitsGroups = 128;  // most groups of the kernel whose lanes resolve their own hits
-inline int line_lanes_log2(const rq_subspace_t &S, int J, int sms) {
-    const int waves = clustered(S, J) ? kLineWaves : 1;
-    int lw = 0;
-    while (lw < 5 && ((S.D << (lw + 1)) <= (int64_t)sms * kLineThreads ||
-                      (J >= 64 << (lw + 1) && (S.D << (lw + 1)) <= (int64_t)sms * kLineThreads * waves)))
-        ++lw;
-    return lw;
-}
 
 template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
 int launch_line_block(const rq_operator_t &op, int lw, const void *x, void *y, int *err, cudaStream_t st,
@@ -966,7 +725,7 @@ int launch_hash(const rq_operator_t &op, const void *x, void *y, int *err, cudaS
         if constexpr (sizeof(typename VT<V>::R) == 4)
             if (lw == 0 && op.terms.J <= kOwnHitsGroups)
                 return launch_line_block<V, KB, FM, 256, false>(op, lw, x, y, err, st, gate, gate2);
-        return op.terms.J * line_key_bytes<FM>() <= 16 * 1024
+        return line_small<FM>(op.terms.J)
                    ? launch_line_block<V, KB, FM, 256, true>(op, lw, x, y, err, st, gate, gate2)
                    : launch_line_block<V, KB, FM, 1024, true>(op, lw, x, y, err, st, gate, gate2);
     }
@@ -1012,9 +771,7 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
                 // filter the sector test costs more than it saves: a target it would reject
                 // costs one L2-resident word of the line filter instead; a larger line filter
                 // keeps it, since its words then compete for L2 or come from DRAM.
-                const bool line_in_l2 =
-                    op.sub.lmap && op.sub.lbits + op.sub.lwbits - 3 <= kLineFilterL2Log2Bytes;
-                const int fm = ((op.sub.fmask_a | op.sub.fmask_b) == 0 || (line_in_l2 && !clustered(op.sub, op.terms.J))) ? kFiltNone
+                const int fm = ((op.sub.fmask_a | op.sub.fmask_b) == 0 || (line_in_l2(op.sub) && !clustered(op.sub, op.terms.J))) ? kFiltNone
                                : op.sub.fpoint >= 0                                     ? kFiltPoint
                                                                                         : kFiltSet;
                 if (op.sub.key_bits == 32) {
@@ -1188,7 +945,9 @@ RQ_API int rq_conn_build(const rq_operator_t *op, int64_t *rowptr, int32_t *col,
     if (!col) {
         RQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
         RQ_CUDA(cudaMemsetAsync(rowptr, 0, sizeof(int64_t), st));
-        if (S.lookup == RQ_LOOKUP_HASH && S.key_bits == 32)
+        if (line_in_l2(S))
+            RQ_TRY(conn_line(*op, rowptr + 1, nullptr, nullptr, nullptr, RQ_C128, err, st));
+        else if (S.lookup == RQ_LOOKUP_HASH && S.key_bits == 32)
             k_conn_count<RQ_LOOKUP_HASH, 32><<<grid_rows(D), kThreads, 0, st>>>(*op, rowptr + 1, err);
         else if (S.lookup == RQ_LOOKUP_HASH)
             k_conn_count<RQ_LOOKUP_HASH, 64><<<grid_rows(D), kThreads, 0, st>>>(*op, rowptr + 1, err);
@@ -1203,6 +962,7 @@ RQ_API int rq_conn_build(const rq_operator_t *op, int64_t *rowptr, int32_t *col,
         if (h_err) return fail(h_err, "rq_conn_build: lookup failed");
         return RQ_OK;
     }
+    if (line_in_l2(S)) return conn_line(*op, rowptr, col, grp, val, val ? vtype : RQ_C128, err, st);
     const int g = grid_rows(D);
 #define RQ_FILL(V)                                                                                  \
     do {                                                                                            \

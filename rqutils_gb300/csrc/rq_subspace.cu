@@ -96,10 +96,9 @@ k_hash_insert(const uint64_t *__restrict__ states, int64_t D, void *keys, int32_
 // Prefix statistics of sorted states for every shift b at once: hist[h] counts the i with
 // 63 - clz(s[i] ^ s[i - 1]) == h, so that the number of distinct prefixes s >> b is
 // 1 + sum_{h >= b} hist[h]; for kRunSamples rows spread over the array, hist[64 + b] adds the number
-// of the 2 kRunReach neighbours that share the row's prefix s >> b, and the row itself.  One warp per
-// sample: its neighbours' highest differing bits at once, then a count per shift.
+// of states that share the row's prefix s >> b.  One warp per sample, a lane per two shifts; each
+// side of the run by doubling steps, an estimate within a factor of 1.5 (up to 8192 states).
 constexpr int kRunSamples = 512;
-constexpr int kRunReach = 64;
 __global__ void k_prefix_hist(const uint64_t *__restrict__ s, int64_t D,
                               unsigned long long *__restrict__ hist) {
     __shared__ unsigned int h[128];
@@ -109,25 +108,16 @@ __global__ void k_prefix_hist(const uint64_t *__restrict__ s, int64_t D,
          i += (int64_t)gridDim.x * blockDim.x)
         atomicAdd(&h[63 - __clzll((long long)(s[i] ^ s[i - 1]))], 1u);
     const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
-    unsigned int run[2] = {0u, 0u};  // of shifts lane and lane + 32
     for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < kRunSamples; k += warps) {
         const int64_t i = D * k / kRunSamples;
         const uint64_t v = s[i];
-        uint64_t diff[2 * kRunReach / 32];  // neighbours' differing bits; all ones past the ends
-#pragma unroll
-        for (int q = 0; q < 2 * kRunReach / 32; ++q) {
-            const int64_t j = i - kRunReach + 32 * q + lane + (32 * q >= kRunReach ? 1 : 0);
-            diff[q] = j >= 0 && j < D ? s[j] ^ v : ~0ULL;
-        }
-        for (int b = 0; b < 64; ++b) {
-            unsigned int n = 1u;
-#pragma unroll
-            for (int q = 0; q < 2 * kRunReach / 32; ++q) n += __popc(__ballot_sync(0xffffffffu, (diff[q] >> b) == 0ULL));
-            if ((b & 31) == lane) run[b >> 5] += n;
+        for (int b = lane; b < 64; b += 32) {
+            int64_t l = 0, r = 0;  // farthest equal neighbours found
+            for (int64_t d = 1; d <= 4096 && i - d >= 0 && s[i - d] >> b == v >> b; d <<= 1) l = d;
+            for (int64_t d = 1; d <= 4096 && i + d < D && s[i + d] >> b == v >> b; d <<= 1) r = d;
+            atomicAdd(&h[64 + b], (unsigned int)(1 + (3 * (l + r)) / 2));
         }
     }
-    atomicAdd(&h[64 + lane], run[0]);
-    atomicAdd(&h[96 + lane], run[1]);
     __syncthreads();
     for (int k = threadIdx.x; k < 128; k += blockDim.x)
         if (h[k]) atomicAdd(hist + k, (unsigned long long)h[k]);
@@ -240,10 +230,12 @@ k_diagonal(const uint64_t *__restrict__ s, int64_t D, const uint64_t *__restrict
                 ci[k] = c[2 * (k0 + k) + 1];
             }
             __syncthreads();
+            // signs and the zero test on the bit patterns: one FP64 instruction per term
             for (int k = 0; k < n; ++k) {
-                const double sg = (__popcll(v & zs[k]) & 1) ? -1. : 1.;
-                re += sg * cr[k];
-                if (ci[k] != 0.) im += sg * ci[k];
+                const unsigned long long sg = (unsigned long long)(__popcll(v & zs[k]) & 1) << 63;
+                re += __longlong_as_double((long long)((unsigned long long)__double_as_longlong(cr[k]) ^ sg));
+                const unsigned long long c = (unsigned long long)__double_as_longlong(ci[k]);
+                if ((c << 1) != 0ULL) im += __longlong_as_double((long long)(c ^ sg));
             }
         }
         if (i < D) out[i] = make_double2(re, im);
