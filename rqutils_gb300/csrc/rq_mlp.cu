@@ -97,6 +97,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(nthreads) : "memory");
 }
+// arrives without waiting (the waiting threads use named_bar_sync with the same count)
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(nthreads) : "memory");
+}
 // barrier over nthreads threads returning the OR of their predicates (the same in every thread)
 __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool p) {
     uint32_t r;
@@ -363,17 +367,11 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
         }
     } else if constexpr (EPI == EPI_HEAD || EPI == EPI_HEAD_TRAIN) {
         // pass 1: Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this half
-        // (in quarters of 64 columns, as the fused inference adds them)
-        float o0 = 0.f, o1 = 0.f, p0 = 0.f, p1 = 0.f;
+        float o0 = 0.f, o1 = 0.f;
 #pragma unroll 1
         for (int g0 = 0; g0 < kHalf; g0 += 32) {
             const int c0 = col0 + g0;
             float z[32], w[32];
-            if (g0 == kHalf / 2) {
-                p0 = o0;
-                p1 = o1;
-                o0 = o1 = 0.f;
-            }
             tmem_ld32(taddr + (uint32_t)c0, z);
             lds32(cst + c0, w);
 #pragma unroll
@@ -388,8 +386,6 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
 #pragma unroll
             for (int i = 0; i < 32; ++i) o1 += z[i] * w[i];
         }
-        o0 = p0 + o0;
-        o1 = p1 + o1;
         if (h == 1) {
             xch[par][row][0] = o0;
             xch[par][row][1] = o1;
@@ -783,7 +779,7 @@ int launch_gemm(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_t 
 // W2 (160 KB) stay in shared memory, which leaves one tile of X (16 KB) and two of H1's four 64-column
 // quarters (32 KB).  TMEM holds both accumulators (2 x 256 columns).  Bound by the epilogue warps,
 // about 11 instructions per hidden unit of each layer: sixteen of them (eight left three of four issue
-// slots empty).  2^18 rows: 113 us as two GEMMs, 100 with eight epilogue warps, 74 with sixteen.
+// slots empty).  2^18 rows: 113 us as two GEMMs, 100 with eight epilogue warps, 80 with sixteen.
 constexpr uint32_t kInfW2 = 0, kInfW1 = 4 * 32768, kInfA = kInfW1 + 32768, kInfH = kInfA + kTileABytes,
                    kInfEnd = kInfH + 2 * kTileABytes;  // 208 KB
 constexpr int kInfWarps = 16;                  // epilogue warps
@@ -802,7 +798,7 @@ struct InferShared {
     int abort, wwait;
     int64_t issued, consumed;  // X tiles
     __align__(16) float cst[4 * kHid];     // b1 | b2 | W3 row 0 | W3 row 1
-    float xch[2][3][kTileM][2];            // output sums of the column quarters 1..3
+    float xch[2][3][kTileM][2];            // output sums: quarters 0 and 2, then 2 and 3 together
 };
 
 __global__ void __launch_bounds__(kInfThreads, 1)
@@ -944,38 +940,62 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
             ok = ok && wait_bar(&sh.d2full, (uint32_t)(it & 1), abort_p);
             if (named_bar_or(kEpiBar, kThreadsE, !ok || *abort_p != 0)) break;  // the same answer in every epilogue thread
             tc_fence_after();
-            // Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this quarter
-            float o0 = 0.f, o1 = 0.f;
-#pragma unroll 1
-            for (int g0 = 0; g0 < kHid / 4; g0 += 32) {
-                const int c0 = cq * (kHid / 4) + g0;
-                float z[32], w[32];
-                tmem_ld32(lanes + (uint32_t)(kHid + c0), z);
-                lds32(sh.cst + kHid + c0, w);
+            // Z2 = acc + b2, H2 = GELU(Z2) of this quarter, and the output layer's dot products in the
+            // order of the forward pass: over each half's 128 columns, then the halves.  An odd
+            // quarter holds its activations and goes on from the sums of the even one before it,
+            // which has gone to the next tile by then.
+            float z[2][32];
+            const int c0 = cq * (kHid / 4);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) z[i] += w[i];
+            for (int k = 0; k < 2; ++k) {
+                tmem_ld32(lanes + (uint32_t)(kHid + c0 + 32 * k), z[k]);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) z[i] = gelu(z[i]);
-                lds32(sh.cst + 2 * kHid + c0, w);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o0 += z[i] * w[i];
-                lds32(sh.cst + 3 * kHid + c0, w);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o1 += z[i] * w[i];
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 b = *reinterpret_cast<const float4 *>(sh.cst + kHid + c0 + 32 * k + i);
+                    z[k][i] = gelu(z[k][i] + b.x);
+                    z[k][i + 1] = gelu(z[k][i + 1] + b.y);
+                    z[k][i + 2] = gelu(z[k][i + 2] + b.z);
+                    z[k][i + 3] = gelu(z[k][i + 3] + b.w);
+                }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.d2empty);
+            float o0 = 0.f, o1 = 0.f;
             float (*x)[kTileM][2] = sh.xch[it & 1];
-            if (cq > 0) {
-                x[cq - 1][row][0] = o0;
-                x[cq - 1][row][1] = o1;
+            if (cq & 1) {
+                named_bar_sync(kEpiBar + 1, kThreadsE);
+                o0 = x[cq >> 1][row][0];
+                o1 = x[cq >> 1][row][1];
             }
-            named_bar_sync(kEpiBar, kThreadsE);
-            if (cq == 0) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 a = *reinterpret_cast<const float4 *>(sh.cst + 2 * kHid + c0 + 32 * k + i);
+                    const float4 b = *reinterpret_cast<const float4 *>(sh.cst + 3 * kHid + c0 + 32 * k + i);
+                    o0 += z[k][i] * a.x;
+                    o1 += z[k][i] * b.x;
+                    o0 += z[k][i + 1] * a.y;
+                    o1 += z[k][i + 1] * b.y;
+                    o0 += z[k][i + 2] * a.z;
+                    o1 += z[k][i + 2] * b.z;
+                    o0 += z[k][i + 3] * a.w;
+                    o1 += z[k][i + 3] * b.w;
+                }
+            if (!(cq & 1)) {
+                x[cq >> 1][row][0] = o0;
+                x[cq >> 1][row][1] = o1;
+                named_bar_arrive(kEpiBar + 1, kThreadsE);
+            } else if (cq == 3) {
+                x[2][row][0] = o0;
+                x[2][row][1] = o1;
+                named_bar_arrive(kEpiBar + 2, kThreadsE / 2);
+            } else {
+                named_bar_sync(kEpiBar + 2, kThreadsE / 2);
                 const int64_t m = u * kTileM + row;
-                o0 = (o0 + x[0][row][0]) + ((x[1][row][0] + x[2][row][0]) + __ldg(g.params + kOffB3));
-                o1 = (o1 + x[0][row][1]) + ((x[1][row][1] + x[2][row][1]) + __ldg(g.params + kOffB3 + 1));
+                o0 += x[2][row][0] + __ldg(g.params + kOffB3);
+                o1 += x[2][row][1] + __ldg(g.params + kOffB3 + 1);
                 if (m < g.M) {
                     g.out[2 * m] = o0;
                     g.out[2 * m + 1] = o1;
