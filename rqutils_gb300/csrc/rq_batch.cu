@@ -10,6 +10,7 @@
 
 #include "rq_common.cuh"
 #include "rq_host.h"
+#include "rq_line.cuh"
 #include "rq_rows.cuh"
 
 namespace rq {
@@ -309,6 +310,77 @@ k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
     }
 }
 
+// The same with a line filter, through line_rows (rq_line.cuh): a block takes a tile of consecutive
+// rows, problem by problem, with that problem's group keys in shared memory, probes every group (the
+// sector stage above costs more than the probes it spares, also when the filter does not fit in L2) and
+// resolves hits through the warp's queue.  complex64: 48 problems, 780,729 rows: 486 -> 189 us; 256
+// problems, 10.2 M rows (filter of 268 MB): 7.25 -> 3.34 ms.
+template <typename V>
+struct UseBatchProduct {
+    using RT = RowTerm<V>;
+    using R = typename VT<V>::R;
+    const rq_batch_t &B;
+    rq_terms_t T;  // the problem's groups
+    const V *x;
+    V *y;
+    typename RT::A acc;
+    __device__ __forceinline__ void start(int64_t i, uint64_t, bool own) {
+        acc = typename RT::A();
+        if (own) acc.add(RT::scaled((R)B.diag0[i], x, i));
+    }
+    __device__ __forceinline__ void hit(int, uint64_t, int) {}  // (the queue is always used)
+    __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t key, int m) {
+        if (group_terms(T, g) > kShortTerms) return true;
+        W.prod[q] = RT::product(T, g, key & kStateMask, x, m);
+        return false;
+    }
+    __device__ __forceinline__ void late(WarpWork<V> &W, int q, int g, uint64_t key) {
+        W.prod[q] = RT::product(T, g, key & kStateMask, x, W.src[q]);
+    }
+    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { acc.add(W.prod[q]); }
+    __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
+};
+
+constexpr int kBatchLineGroups = 1024;  // groups of a problem in shared memory at a time
+
+template <typename V>
+__global__ void __launch_bounds__(kThreads, 4)
+k_batch_matvec_line(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y, int *err, int lw,
+                    const int *gate, int64_t gstride, const int *gate2) {
+    copy_hash_tables(hk_htab, 8);
+    rq_subspace_t S = {};
+    S.states = B.keys;
+    S.D = B.D;
+    S.hkeys = B.hkeys;
+    S.hvals = B.hvals;
+    S.hbits = B.hbits;
+    S.lookup = RQ_LOOKUP_HASH;
+    S.key_bits = 64;
+    S.empty_key = B.empty_key;
+    S.lmap = B.lmap;
+    S.lbits = B.lbits;
+    S.lwbits = B.lwbits;
+    const int64_t rows = kThreads >> lw;
+    for (int64_t t0 = (int64_t)blockIdx.x * rows; t0 < B.D; t0 += (int64_t)gridDim.x * rows) {
+        const int64_t t1 = min(t0 + rows, B.D);
+        for (int64_t a = t0, e; a < t1; a = e) {
+            const int p = problem_of(__ldg(B.keys + a));
+            e = min(t1, B.prow[p + 1]);
+            if (!gate_open(gate, gstride, gate2, p)) continue;
+            S.lshift = B.lshift[p];
+            const int g0 = B.gofs[p];
+            UseBatchProduct<V> use{B, B.terms, x, y, {}};
+            use.T.J = B.gofs[p + 1] - g0;
+            use.T.diag_group = B.dgrp[p] >= 0 ? B.dgrp[p] - g0 : -1;
+            use.T.xmask += g0;
+            use.T.xhash += g0;
+            use.T.toff += g0;
+            line_rows<V, 64, kFiltNone, kThreads, true>(S, use.T, err, lw, kBatchLineGroups,
+                                                        a + (threadIdx.x >> 5) * (32 >> lw), a, rows, e, use);
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads)
 k_batch_conn_count(const rq_batch_t B, int64_t *__restrict__ rowcnt, int *err) {
     __shared__ __align__(16) uint32_t htab[kHashTableWords];
@@ -372,6 +444,31 @@ k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
     }
 }
 
+// A thread per row, for 32-bit values and more than kConnRowsD rows: 2.03 M rows of 40 problems,
+// complex64: 134 us against 181 with tiles, whose height fits the average problem and not the few with
+// long rows (780,729 rows of 48 problems: 20.8 against 21.1; complex128 wants tiles at any size: its
+// additions are what counts, 262 us against 351).
+constexpr int64_t kConnRowsD = int64_t(1) << 20;
+template <typename V>
+__global__ void __launch_bounds__(kThreads)
+k_batch_matvec_conn_rows(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y,
+                         const int *gate, int64_t gstride, const int *gate2) {
+    using RT = RowTerm<V>;
+    using R = typename VT<V>::R;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < B.D;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t key = __ldg(B.keys + i);
+        if (!gate_open(gate, gstride, gate2, problem_of(key))) continue;
+        const uint64_t s = key & kStateMask;
+        typename RT::A acc;
+        acc.add(RT::scaled((R)B.diag0[i], x, i));
+        const int64_t e1 = B.rowptr[i + 1];
+        for (int64_t e = B.rowptr[i]; e < e1; ++e)
+            acc.add(RT::product(B.terms, __ldg(B.grp + e), s, x, __ldg(B.col + e)));
+        RT::store(y, i, acc);
+    }
+}
+
 // scans of the CONN build live in rq_matvec.cu
 }  // namespace
 
@@ -380,12 +477,30 @@ int scan_row_counts(int64_t *rowptr_plus1, int64_t D, int64_t *bsum, cudaStream_
 template <typename V>
 int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cudaStream_t st,
                        const int *gate, int64_t gstride, const int *gate2) {
-    if (B.mode == RQ_MODE_FREE) {
+    if (B.mode == RQ_MODE_FREE && B.lmap) {
+        auto kern = k_batch_matvec_line<V>;
+        const size_t smem = line_work_bytes<V, kThreads, true>() + (kBatchLineGroups + kPart) * line_key_bytes<kFiltNone>();
+        thread_local KernelLaunchCache table[kMaxCachedDevices];
+        KernelLaunchCache *c = nullptr;
+        int per_sm = 1, lw = 0;
+        RQ_TRY(cache_slot(table, &c));
+        RQ_TRY(configure_kernel(kern, *c, smem, kThreads, &per_sm));
+        while (lw < 5 && B.D << (lw + 1) <= (int64_t)sm_count() * kLineThreads) ++lw;
+        const int64_t tiles = (B.D + (kThreads >> lw) - 1) / (kThreads >> lw);
+        kern<<<(int)std::min<int64_t>(tiles, (int64_t)sm_count() * per_sm), kThreads, smem, st>>>(
+            B, static_cast<const V *>(x), static_cast<V *>(y), err, lw, gate, gstride, gate2);
+    } else if (B.mode == RQ_MODE_FREE) {
         k_batch_matvec_free<V><<<grid_rows(B.D, 6), kThreads, 0, st>>>(
             B, static_cast<const V *>(x), static_cast<V *>(y), err, gate, gstride, gate2);
     } else if (B.mode == RQ_MODE_CONN) {
         if (!B.rowptr || (B.nnz > 0 && (!B.col || !B.grp)))
             return fail(RQ_E_ARG, "rq_batch_matvec: RQ_MODE_CONN needs rowptr, col and grp");
+        if (sizeof(typename VT<V>::R) == 4 && B.D > kConnRowsD) {
+            k_batch_matvec_conn_rows<V><<<grid_rows(B.D), kThreads, 0, st>>>(
+                B, static_cast<const V *>(x), static_cast<V *>(y), gate, gstride, gate2);
+            RQ_CUDA(cudaGetLastError());
+            return RQ_OK;
+        }
         const int rows = tile_rows<V>(B.D, B.nnz, sm_count());
         const int64_t tiles = (B.D + rows - 1) / rows, cap = (int64_t)sm_count() * 8;
         k_batch_matvec_conn<V><<<(int)std::min(tiles, cap), kThreads, 0, st>>>(

@@ -54,7 +54,7 @@ template <int KB, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 k_conn_count_line(const rq_operator_t op, int64_t *__restrict__ rows, int *err, int lw, int kt, int spread) {
     UseCount use{rows, 0};
-    line_rows<float, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
+    line_subspace<float, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
 }
 
 template <typename V, int KB, int BLOCK>
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 k_conn_fill_line(const rq_operator_t op, const int64_t *__restrict__ rowptr, int32_t *__restrict__ col,
                  int32_t *__restrict__ grp, V *__restrict__ val, int *err, int lw, int kt, int spread) {
     UseFill<V> use{op.terms, rowptr, col, grp, val, 0};
-    line_rows<V, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
+    line_subspace<V, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
 }
 
 // grid and shared memory of a kernel over the rows; launches through go(grid, smem, lw, kt, spread)

@@ -102,21 +102,18 @@ __device__ __forceinline__ uint32_t line_word(uint32_t h, uint32_t hpre, const r
 // sees for each row: start(i, s, own) -- own: the lane that sums the row -- then for each hit
 // resolve(W, q, g, s, m) on some lane of the warp (queue slot q, group g, row state s, source m;
 // true: call late() for it in the second round), take(W, q, g) on the owner in list order, and
-// finish(i).  Without a queue: hit(g, s, m) on the owner.
+// finish(i).  Without a queue: hit(g, s, m) on the owner.  A warp takes the 32 >> lw rows from
+// `first` + a multiple of `stride` while some row of the block's turn lies below `end`; the caller
+// has filled hk_htab (and hk_fb), and every thread of the block calls.
 template <typename V, int KB, int FM, int BLOCK, bool QUEUE, typename C>
-__device__ __forceinline__ void line_rows(const rq_operator_t &op, int *err, int lw, int kt, int spread, C &use) {
+__device__ __forceinline__ void line_rows(const rq_subspace_t &S, const rq_terms_t &T, int *err, int lw, int kt,
+                                          int64_t first, int64_t turn, int64_t stride, int64_t end, C &use) {
     using K = typename KeyWidth<KB>::K;
     constexpr int NB = KeyWidth<KB>::kNbytes;
     // probes in flight per lane: what 64 (QUEUE) and 40 registers hold
     constexpr int U = FM != kFiltNone ? 8 : QUEUE ? 16 : KB == 32 ? 32 : 8;
-    const rq_subspace_t &S = op.sub;
-    const rq_terms_t &T = op.terms;
-    const int64_t D = S.D;
     const int skip = T.diag_group;
     const int nres = T.J - (skip >= 0 ? 1 : 0);
-    copy_hash_tables(hk_htab, NB);
-    if (FM == kFiltSet)
-        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = S.fbits[w];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpWork<V> &W = reinterpret_cast<WarpWork<V> *>(hk_dyn)[QUEUE ? warp : 0];
     uint2 *gk = reinterpret_cast<uint2 *>(hk_dyn + line_work_bytes<V, BLOCK, QUEUE>());  // [kt + kPart]
@@ -142,13 +139,11 @@ __device__ __forceinline__ void line_rows(const rq_operator_t &op, int *err, int
     const uint32_t *lmap = S.lmap;
     const unsigned lt = (1u << lane) - 1u;
     const int w = 1 << lw, sub = lane & (w - 1);
-    const int64_t rows = 32 >> lw, stride = (int64_t)gridDim.x * (BLOCK / 32) * rows;
-    const int64_t first = (spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * (BLOCK / 32) + warp) * rows;
-    for (int64_t base = 0; base < D; base += stride) {  // the same trips for every warp of a block
-        const int64_t i = base + first + (lane >> lw);
-        const bool active = i < D;
-        if (!tiled && base + first >= D) break;
-        const int64_t ir = active ? i : D - 1;
+    for (int64_t base = 0; turn + base < end; base += stride) {  // the same trips for every warp of a block
+        const int64_t i = first + base + (lane >> lw);
+        const bool active = i < end;
+        if (!tiled && first + base >= end) break;
+        const int64_t ir = active ? i : end - 1;
         const uint64_t s64 = __ldg(S.states + ir);
         const K s = (K)s64;
         const uint32_t hs = lin_hash(hk_htab, s64, NB);
@@ -261,6 +256,20 @@ __device__ __forceinline__ void line_rows(const rq_operator_t &op, int *err, int
         }
         if (active && sub == 0) use.finish(i);
     }
+}
+
+// The tables and the calling warp's place for a kernel that walks the whole subspace: neighbouring
+// tiles of 32 >> lw rows to the same block, or (spread) to different SMs.
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE, typename C>
+__device__ __forceinline__ void line_subspace(const rq_operator_t &op, int *err, int lw, int kt, int spread, C &use) {
+    copy_hash_tables(hk_htab, KeyWidth<KB>::kNbytes);
+    if (FM == kFiltSet)
+        for (int w = threadIdx.x; w < RQ_FILTER_WORDS; w += blockDim.x) hk_fb[w] = op.sub.fbits[w];
+    const int warp = threadIdx.x >> 5;
+    const int64_t rows = 32 >> lw, stride = (int64_t)gridDim.x * (BLOCK / 32) * rows;
+    const int64_t first =
+        (spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * (BLOCK / 32) + warp) * rows;
+    line_rows<V, KB, FM, BLOCK, QUEUE>(op.sub, op.terms, err, lw, kt, first, 0, stride, op.sub.D, use);
 }
 
 // ---- launch rules -----------------------------------------------------------------------------

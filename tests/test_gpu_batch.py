@@ -254,3 +254,22 @@ def test_batch_persistent_launches_match_graph_chunks(variant, precision):
         r = b.rows(p)
         # both vectors meet the residual test, so they agree to about (residual / gap)^2
         assert abs(np.vdot(x1[r], x2[r])) > 1 - (1e-10 if precision == 'fp64' else 1e-8), p
+
+
+@pytest.mark.parametrize('dtype', ['complex64', 'complex128'])
+@pytest.mark.parametrize('seed,P,d_range', [(41, 3, (1, 40)), (42, 60, (200, 3000)), (43, 30, (30000, 260000))])
+def test_batch_products_agree_bit_for_bit(seed, P, d_range, dtype):
+    """The batched product through the line filter (tiles that cross problems, few and many rows), the
+    one without it and both cached-connectivity forms: the same additions, the same bits."""
+    import torch
+    from rqutils_gb300.batch import BatchedSQD
+    hams, states, ns = _random_problems(seed, P, d_range=d_range)
+    line = BatchedSQD(hams, states, cache_level=(0, 0))
+    x = torch.randn(line.D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(P))
+    y = line.matvec(x)
+    for b in (BatchedSQD(hams, states, cache_level=(0, 0), line_filter=False, presence=False),
+              BatchedSQD(hams, states, cache_level=(1, 0))):
+        assert torch.equal(b.matvec(x), y)
+        b.check_errors()
+    line.check_errors()
+    assert (line.D > 2 ** 20) == (P == 30)
