@@ -328,7 +328,6 @@ struct UseBatchProduct {
         acc = typename RT::A();
         if (own) acc.add(RT::scaled((R)B.diag0[i], x, i));
     }
-    __device__ __forceinline__ void hit(int, uint64_t, int) {}  // (the queue is always used)
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t key, int m) {
         if (group_terms(T, g) > kShortTerms) return true;
         W.prod[q] = RT::product(T, g, key & kStateMask, x, m);
@@ -375,7 +374,7 @@ k_batch_matvec_line(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
             use.T.xmask += g0;
             use.T.xhash += g0;
             use.T.toff += g0;
-            line_rows<V, 64, kFiltNone, kThreads, true>(S, use.T, err, lw, kBatchLineGroups,
+            line_rows<V, 64, kFiltNone, kThreads>(S, use.T, err, lw, kBatchLineGroups,
                                                         a + (threadIdx.x >> 5) * (32 >> lw), a, rows, e, use);
         }
     }
@@ -479,7 +478,7 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
                        const int *gate, int64_t gstride, const int *gate2) {
     if (B.mode == RQ_MODE_FREE && B.lmap) {
         auto kern = k_batch_matvec_line<V>;
-        const size_t smem = line_work_bytes<V, kThreads, true>() + (kBatchLineGroups + kPart) * line_key_bytes<kFiltNone>();
+        const size_t smem = line_work_bytes<V, kThreads>() + (kBatchLineGroups + kPart) * line_key_bytes<kFiltNone>();
         thread_local KernelLaunchCache table[kMaxCachedDevices];
         KernelLaunchCache *c = nullptr;
         int per_sm = 1, lw = 0;

@@ -11,7 +11,6 @@ struct UseCount {  // elements per row
     int64_t *out;
     int64_t n;
     __device__ __forceinline__ void start(int64_t, uint64_t, bool) { n = 0; }
-    __device__ __forceinline__ void hit(int, uint64_t, int) { ++n; }
     __device__ __forceinline__ bool resolve(WarpWork<float> &, int, int, uint64_t, int) { return false; }
     __device__ __forceinline__ void late(WarpWork<float> &, int, int, uint64_t) {}
     __device__ __forceinline__ void take(const WarpWork<float> &, int, int) { ++n; }
@@ -30,7 +29,6 @@ struct UseFill {  // (source, group) lists and, CSR, the elements
         else W.prod[q] = group_diag_re<typename VT<V>::R>(T, g, s);
     }
     __device__ __forceinline__ void start(int64_t i, uint64_t, bool own) { p = own ? rowptr[i] : 0; }
-    __device__ __forceinline__ void hit(int, uint64_t, int) {}  // (the queue is always used)
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int) {
         if (!val) return false;
         if (group_terms(T, g) > kShortTerms) return true;
@@ -54,7 +52,7 @@ template <int KB, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 k_conn_count_line(const rq_operator_t op, int64_t *__restrict__ rows, int *err, int lw, int kt, int spread) {
     UseCount use{rows, 0};
-    line_subspace<float, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
+    line_subspace<float, KB, kFiltNone, BLOCK>(op, err, lw, kt, spread, use);
 }
 
 template <typename V, int KB, int BLOCK>
@@ -62,7 +60,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 k_conn_fill_line(const rq_operator_t op, const int64_t *__restrict__ rowptr, int32_t *__restrict__ col,
                  int32_t *__restrict__ grp, V *__restrict__ val, int *err, int lw, int kt, int spread) {
     UseFill<V> use{op.terms, rowptr, col, grp, val, 0};
-    line_subspace<V, KB, kFiltNone, BLOCK, true>(op, err, lw, kt, spread, use);
+    line_subspace<V, KB, kFiltNone, BLOCK>(op, err, lw, kt, spread, use);
 }
 
 // grid and shared memory of a kernel over the rows; launches through go(grid, smem, lw, kt, spread)
@@ -72,7 +70,7 @@ int launch(K kern, KernelLaunchCache (&table)[kMaxCachedDevices], const rq_opera
     constexpr int kMaxTile = line_tile_groups<V, kFiltNone, BLOCK>();
     static_assert(kMaxTile <= 65536, "a queue entry holds 16 bits of group");
     const int kt = nres < kMaxTile ? std::max(nres, 1) : kMaxTile;
-    const size_t smem = line_work_bytes<V, BLOCK, true>() + (size_t)(kt + kPart) * line_key_bytes<kFiltNone>();
+    const size_t smem = line_work_bytes<V, BLOCK>() + (size_t)(kt + kPart) * line_key_bytes<kFiltNone>();
     KernelLaunchCache *c = nullptr;
     int per_sm = 1;
     RQ_TRY(cache_slot(table, &c));

@@ -184,7 +184,6 @@ struct UseProduct {  // y = H x
         if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[i], x, i));
         else if (skip >= 0) acc.add(RT::product(op.terms, skip, s, x, i));
     }
-    __device__ __forceinline__ void hit(int g, uint64_t s, int m) { acc.add(RT::product(op.terms, g, s, x, m)); }
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int m) {
         if (group_terms(op.terms, g) > kShortTerms) return true;
         W.prod[q] = RT::product(op.terms, g, s, x, m);
@@ -197,13 +196,13 @@ struct UseProduct {  // y = H x
     __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
 };
 
-template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
-__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : QUEUE ? 4 : 6)
+template <typename V, int KB, int FM, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : 4)
 k_matvec_line(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err, int lw, int kt,
               int spread, const int *gate, const int *gate2) {
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     UseProduct<V> use{op, x, y, {}};
-    line_subspace<V, KB, FM, BLOCK, QUEUE>(op, err, lw, kt, spread, use);
+    line_subspace<V, KB, FM, BLOCK>(op, err, lw, kt, spread, use);
 }
 
 // ---- probes of the key buckets ----------------------------------------------------------------
@@ -724,17 +723,15 @@ int launch_hash_block(const rq_operator_t &op, const void *x, void *y, int *err,
     return RQ_OK;
 }
 
-constexpr int kOwnHitsGroups = 128;  // most groups of the kernel whose lanes resolve their own hits
-
-template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
+template <typename V, int KB, int FM, int BLOCK>
 int launch_line_block(const rq_operator_t &op, int lw, const void *x, void *y, int *err, cudaStream_t st,
                       const int *gate, const int *gate2) {
-    auto kern = k_matvec_line<V, KB, FM, BLOCK, QUEUE>;
+    auto kern = k_matvec_line<V, KB, FM, BLOCK>;
     const int nres = op.terms.J - (op.terms.diag_group >= 0 ? 1 : 0);
     constexpr int kMaxTile = line_tile_groups<V, FM, BLOCK>();
     static_assert(kMaxTile <= 65536, "a queue entry holds 16 bits of group");
     const int kt = nres < kMaxTile ? std::max(nres, 1) : kMaxTile;
-    const size_t smem = line_work_bytes<V, BLOCK, QUEUE>() + (size_t)(kt + kPart) * line_key_bytes<FM>();
+    const size_t smem = line_work_bytes<V, BLOCK>() + (size_t)(kt + kPart) * line_key_bytes<FM>();
     thread_local KernelLaunchCache table[kMaxCachedDevices];
     KernelLaunchCache *c = nullptr;
     int per_sm = 1;
@@ -757,12 +754,9 @@ int launch_hash(const rq_operator_t &op, const void *x, void *y, int *err, cudaS
     // fits): one 1024-thread block
     if (op.sub.lmap) {
         const int lw = line_lanes_log2(op.sub, op.terms.J, sm_count());
-        if constexpr (sizeof(typename VT<V>::R) == 4)
-            if (lw == 0 && op.terms.J <= kOwnHitsGroups)
-                return launch_line_block<V, KB, FM, 256, false>(op, lw, x, y, err, st, gate, gate2);
         return line_small<FM>(op.terms.J)
-                   ? launch_line_block<V, KB, FM, 256, true>(op, lw, x, y, err, st, gate, gate2)
-                   : launch_line_block<V, KB, FM, 1024, true>(op, lw, x, y, err, st, gate, gate2);
+                   ? launch_line_block<V, KB, FM, 256>(op, lw, x, y, err, st, gate, gate2)
+                   : launch_line_block<V, KB, FM, 1024>(op, lw, x, y, err, st, gate, gate2);
     }
     const bool small = op.terms.J <= max_resident_groups<KB>() &&
                        group_key_bytes<KB>(op.terms.J) <= 16 * 1024;
