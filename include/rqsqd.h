@@ -421,9 +421,9 @@ int rq_mlp_bwd(const rq_mlp_t *m, int64_t rows, const uint16_t *xt, const float 
 /* One training step without the Adam update: forward, loss and backward of a minibatch (rows a
  * multiple of 128; x[rows][64] and xt[64][rows] BF16, tgt[rows][3] as rq_mlp_sample writes them).
  * m->grads = d loss / d params; out[rows][2] = f(x) when out is not NULL; loss[0] (device double)
- * = the loss of rq_mlp_loss when loss is not NULL.  Layer 2's epilogue computes the loss gradient
- * and dZ2 in place (the same gradients as rq_mlp_fwd + rq_mlp_loss + rq_mlp_bwd, with Z2 kept in
- * FP32 rather than rounded to BF16). */
+ * = the loss of rq_mlp_loss when loss is not NULL.  One kernel takes each tile of 128
+ * rows from x to dZ1 (the same gradients as rq_mlp_fwd + rq_mlp_loss + rq_mlp_bwd, with Z2 kept in
+ * FP32 rather than rounded to BF16); ws then holds no activations for rq_mlp_bwd. */
 int rq_mlp_train(const rq_mlp_t *m, int64_t rows, const uint16_t *x, const uint16_t *xt,
                  const float *tgt, float *out, double *loss, void *ws, void *stream);
 /* One Adam step (step number t >= 1) on params from grads; refreshes the BF16 copies. */

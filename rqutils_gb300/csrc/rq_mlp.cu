@@ -1,16 +1,13 @@
 // Learned warm start: a BF16 MLP (64 -> 256 -> 256 -> 2, GELU) mapping (state, U) to the ground
 // state's log-amplitude and sign, trained and evaluated with tcgen05 tensor-core GEMMs.
 //
-// GEMM: C[M][N] = A[M][K] B[N][K]^T, both operands K-major BF16, FP32 accumulators in TMEM.  A CTA
-// of 128 threads owns a 128-row tile and all N <= 256 columns; K runs in chunks of 64 through a
-// two-stage shared-memory ring filled with cp.async (16 B per thread and copy) in the no-swizzle
-// core-matrix layout: an 8-row x 16-byte core matrix is 128 contiguous bytes, core matrices
-// adjacent in K are 128 B apart (leading byte offset) and 8-row groups 1024 B apart (stride byte
-// offset).  One thread issues four tcgen05.mma (K = 16 each) per chunk and commits them to the
-// stage's mbarrier; the stage is refilled once that barrier completes, so the copies of chunk c
-// overlap the MMAs of chunk c - 1.  The epilogue reads the accumulator rows back with
-// tcgen05.ld (warp w owns TMEM lanes 32w..32w+31, one row per thread) and fuses bias, GELU,
-// the 256 -> 2 output layer, GELU' and the bias-gradient column sums.
+// GEMM (k_gemm: the layers of the separate forward and backward passes): C[M][N] = A[M][K] B[N][K]^T,
+// both operands K-major BF16, FP32 accumulators in TMEM.  A persistent CTA takes 128-row tiles with all
+// N <= 256 columns; warp 0 fills shared memory by TMA in the 128-byte swizzled layout, one thread of
+// warp 1 issues the tcgen05.mma, and eight warps read the accumulator rows back (tcgen05.ld, one row
+// per thread, two accumulators in turn) and fuse bias, GELU, the 256 -> 2 output layer, GELU' and the
+// bias-gradient column sums.
+// Inference (k_infer) and a training step (k_train, k_wgrad: rq_mlp_train.cuh) have fused kernels.
 //
 // Every mbarrier wait is bounded (about one second of clock cycles); on expiry the kernel records
 // RQ_E_CUDA in the error flag, skips the remaining work, frees its TMEM and returns.
@@ -37,7 +34,7 @@ static_assert(kNParams == RQ_MLP_NPARAMS, "parameter layout");
 constexpr int kHeadPart = kHid + kOut * kHid + kOut;  // db2 | dW3 | db3 partial sums per tile
 constexpr long long kWaitCycles = 2000000000LL;
 
-enum Epi { EPI_F32 = 0, EPI_HIDDEN = 1, EPI_HEAD = 2, EPI_DGELU = 3, EPI_HEAD_TRAIN = 4 };
+enum Epi { EPI_F32 = 0, EPI_HIDDEN = 1, EPI_HEAD = 2, EPI_DGELU = 3 };
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers
@@ -128,7 +125,9 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 }
 
-// instruction descriptor of kind::f16: BF16 x BF16 -> FP32, both K-major, M x N
+// instruction descriptor of kind::f16: BF16 x BF16 -> FP32, M x N, both K-major (kIdescTransA,
+// kIdescTransB: the operand is MN-major)
+constexpr uint32_t kIdescTransA = 1u << 15, kIdescTransB = 1u << 16;
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N) {
     return (1u << 4)                          // D: FP32
            | (1u << 7)                        // A: BF16
@@ -197,13 +196,13 @@ __device__ __forceinline__ float tanh_approx(float x) {
 constexpr float kGeluK0 = 0.7978845608028654f;           // sqrt(2 / pi)
 constexpr float kGeluK01 = 0.7978845608028654f * 0.044715f;
 __device__ __forceinline__ float gelu(float z) {
-    return 0.5f * z * (1.f + tanh_approx(z * fmaf(kGeluK01, z * z, kGeluK0)));
+    return z * fmaf(0.5f, tanh_approx(z * fmaf(kGeluK01, z * z, kGeluK0)), 0.5f);
 }
 // activation a and derivative d of one pre-activation
 __device__ __forceinline__ void gelu_both(float z, float &a, float &d) {
     const float z2 = z * z;
     const float t = tanh_approx(z * fmaf(kGeluK01, z2, kGeluK0));
-    const float h = 0.5f * (1.f + t);
+    const float h = fmaf(0.5f, t, 0.5f);
     a = z * h;
     d = fmaf(0.5f * z * (1.f - t * t), fmaf(3.f * kGeluK01, z2, kGeluK0), h);
 }
@@ -213,6 +212,63 @@ __device__ __forceinline__ float dgelu(float z) {
     return d;
 }
 
+// Two columns at a time: the packed FP32 instructions of sm_100 and later round each half as the scalar
+// ones do (the same bits) and take one issue slot for both, which bounds the fused kernels.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 x, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(x));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 tanh2(f32x2 x) {
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(tanh_approx(a), tanh_approx(b));
+}
+__device__ __forceinline__ f32x2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ f32x2 gelu2(f32x2 z) {
+    const f32x2 t = tanh2(mul2(z, fma2(both(kGeluK01), mul2(z, z), both(kGeluK0))));
+    return mul2(z, fma2(both(0.5f), t, both(0.5f)));
+}
+__device__ __forceinline__ void gelu_both2(f32x2 z, f32x2 &a, f32x2 &d) {
+    const f32x2 z2 = mul2(z, z);
+    const f32x2 t = tanh2(mul2(z, fma2(both(kGeluK01), z2, both(kGeluK0))));
+    const f32x2 h = fma2(both(0.5f), t, both(0.5f));
+    a = mul2(z, h);
+    // (-z / 2) (t^2 - 1): the packed forms take no negated operand
+    d = fma2(mul2(mul2(both(-0.5f), z), fma2(t, t, both(-1.f))), fma2(both(3.f * kGeluK01), z2, both(kGeluK0)), h);
+}
+__device__ __forceinline__ uint32_t bf16x2(f32x2 x) {  // both halves rounded to nearest
+    float lo, hi;
+    unpack2(x, lo, hi);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
 // ---------------------------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------------------------
@@ -220,28 +276,20 @@ constexpr int kGemmThreads = 320;  // warp 0: TMA producer, warp 1: MMA issuer, 
 constexpr int kEpiThreads = 256;
 constexpr int kEpiBar = 1;         // named barrier of the epilogue warps (0 is __syncthreads)
 constexpr uint32_t kTileABytes = kTileM * kChunkK * 2;
-constexpr int kSplitK = 76;        // K splits of the row-reduction GEMMs (2 row tiles x 76 = 152 units)
 
 struct GemmArgs {
     int64_t M;        // rows of A; rows >= M are read as zeros (TMA fill) and not stored
     int64_t mtiles;   // ceil(M / 128)
-    int64_t nsplit;   // K splits; EPI_F32 writes one partial product per split
     int64_t nchunks;  // K / 64
     const float *bias;
     bf16 *z_rm;       // pre-activations, row-major [M][N] (HIDDEN, HEAD; optional)
     bf16 *h_rm;       // activations, row-major [M][N] (HIDDEN)
-    bf16 *h_fm;       // feature-major [N][ld_fm]: HIDDEN activations (optional), DGELU and HEAD_TRAIN gradients
-    int64_t ld_fm;
     const bf16 *zin_rm;  // pre-activations read by DGELU, row-major [M][N]
-    float *out;          // F32: [M][N], or [nsplit][N][M] with split_cm; HEAD, HEAD_TRAIN: [M][2] (optional)
-    int split_cm;        // F32: column-major partial products (lane = row: coalesced stores)
-    const float *w3;     // HEAD, HEAD_TRAIN: [2][N]
-    const float *b3;     // HEAD, HEAD_TRAIN: [2]
-    const float *tgt;    // HEAD_TRAIN: [M][3] = log-amplitude target, sign, weight
-    float inv_rows;      // HEAD_TRAIN: 1 / rows (the loss is a mean over the rows)
-    bf16 *dz_rm;         // HEAD_TRAIN: dZ2, row-major [M][N]
-    float *colpart;      // DGELU: [gridDim.x][N]; HEAD_TRAIN: [gridDim.x][kHeadPart] (one row per CTA)
-    double *losspart;    // HEAD_TRAIN: [gridDim.x]
+    float *out;          // F32: [M][N]; HEAD: [M][2] (optional)
+    const float *w3;     // HEAD: [2][N]
+    const float *b3;     // HEAD: [2]
+    bf16 *dz_rm;         // DGELU: dZ1, row-major [M][N]
+    float *colpart;      // DGELU: [gridDim.x][N] (one row per CTA)
     int *err;
 };
 
@@ -255,14 +303,8 @@ struct GemmCfg {
 // epilogue constants in shared memory: bias | W3 row 0 | W3 row 1
 template <int N, int EPI>
 __host__ __device__ constexpr int const_floats() {
-    return EPI == EPI_HIDDEN ? N : ((EPI == EPI_HEAD || EPI == EPI_HEAD_TRAIN) ? 3 * N : 4);
+    return EPI == EPI_HIDDEN ? N : (EPI == EPI_HEAD ? 3 * N : 4);
 }
-// column sums accumulated per CTA: DGELU db1; HEAD_TRAIN db2, dW3 row 0, dW3 row 1
-template <int EPI>
-__host__ __device__ constexpr int colsum_quantities() {
-    return EPI == EPI_HEAD_TRAIN ? 3 : (EPI == EPI_DGELU ? 1 : 0);
-}
-
 // lane l returns sum over the 32 lanes of v[l] (v is consumed): each of the five exchange rounds
 // halves the columns a lane keeps, 31 shuffles for 32 column sums, in a fixed order
 __device__ __forceinline__ float col_sum32(float (&v)[32], int lane) {
@@ -310,21 +352,12 @@ __device__ __forceinline__ void lds32(const float *p, float (&v)[32]) {
     }
 }
 
-// running sums of the epilogue over the CTA's tiles: col points at this thread's row quarter of the
-// shared array csum[quantity][quarter][N] (quantity j at col[4 N j + c]; each (quarter, column) slot
-// belongs to one thread); d0, d1 and loss per thread
-template <int N, int EPI>
-struct EpiAcc {
-    float *col;
-    float d0 = 0.f, d1 = 0.f;
-    double loss = 0.;
-};
-
-// one epilogue thread: row `row` of the tile (its TMEM lane), columns [h N/2, (h + 1) N/2)
+// one epilogue thread: row `row` of the tile (its TMEM lane), columns [h N/2, (h + 1) N/2); DGELU: col =
+// the running column sums of this thread's row quarter over the CTA's tiles (each slot has one thread)
 template <int N, int EPI>
 __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int h, int lane, int row, int64_t m,
-                                         bool valid, int64_t sp, int par, float (*xch)[kTileM][2],
-                                         const float *cst, EpiAcc<N, EPI> &acc) {
+                                         bool valid, int par, float (*xch)[kTileM][2],
+                                         const float *cst, float *col) {
     constexpr int kHalf = N / 2;
     const int col0 = h * kHalf;
     if constexpr (EPI == EPI_F32) {
@@ -333,15 +366,9 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
             float v[32];
             tmem_ld32(taddr + (uint32_t)(col0 + g0), v);
             if (valid) {
-                if (g.split_cm) {
-                    float *dst = g.out + (sp * N + col0 + g0) * g.M + m;
+                float4 *dst = reinterpret_cast<float4 *>(g.out + m * N + col0 + g0);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) dst[(int64_t)i * g.M] = v[i];
-                } else {
-                    float4 *dst = reinterpret_cast<float4 *>(g.out + m * N + col0 + g0);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                }
+                for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
             }
         }
     } else if constexpr (EPI == EPI_HIDDEN) {
@@ -359,14 +386,10 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
             if (valid) {
                 if (g.z_rm) store_bf16x32(g.z_rm + m * N + c0, z);
                 store_bf16x32(g.h_rm + m * N + c0, b);
-                if (g.h_fm) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) g.h_fm[(int64_t)(c0 + i) * g.ld_fm + m] = __float2bfloat16_rn(b[i]);
-                }
             }
         }
-    } else if constexpr (EPI == EPI_HEAD || EPI == EPI_HEAD_TRAIN) {
-        // pass 1: Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this half
+    } else if constexpr (EPI == EPI_HEAD) {
+        // Z2 = acc + b2, H2 = GELU(Z2), the output layer's dot products over this half
         float o0 = 0.f, o1 = 0.f;
 #pragma unroll 1
         for (int g0 = 0; g0 < kHalf; g0 += 32) {
@@ -376,7 +399,7 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
             lds32(cst + c0, w);
 #pragma unroll
             for (int i = 0; i < 32; ++i) z[i] += w[i];
-            if (EPI == EPI_HEAD && valid && g.z_rm) store_bf16x32(g.z_rm + m * N + c0, z);
+            if (valid && g.z_rm) store_bf16x32(g.z_rm + m * N + c0, z);
 #pragma unroll
             for (int i = 0; i < 32; ++i) z[i] = gelu(z[i]);
             lds32(cst + N + c0, w);
@@ -399,64 +422,7 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
                 g.out[m * 2 + 1] = o1;
             }
         }
-        if constexpr (EPI == EPI_HEAD_TRAIN) {
-            // the loss of the row and its gradient (half 0), handed to half 1 through xch[par + 2]
-            float d0 = 0.f, d1 = 0.f;
-            if (h == 0) {
-                if (valid) {
-                    const float at = g.tgt[m * 3], sg = g.tgt[m * 3 + 1], w = g.tgt[m * 3 + 2];
-                    const float e = o0 - at;
-                    const float tt = -sg * o1;
-                    const float sp = tt > 20.f ? tt : log1pf(expf(tt));  // softplus(-s o1)
-                    const float sig = 1.f / (1.f + expf(-tt));           // sigmoid(-s o1)
-                    acc.loss += (double)(w * (e * e + sp));
-                    d0 = w * g.inv_rows * 2.f * e;
-                    d1 = -w * g.inv_rows * sg * sig;
-                }
-                acc.d0 += d0;
-                acc.d1 += d1;
-                xch[par + 2][row][0] = d0;
-                xch[par + 2][row][1] = d1;
-            }
-            named_bar_sync(kEpiBar, kEpiThreads);
-            if (h == 1) {
-                d0 = xch[par + 2][row][0];
-                d1 = xch[par + 2][row][1];
-            }
-            // pass 2: dZ2 = (dout W3) * GELU'(Z2) and the column sums of db2 and dW3
-#pragma unroll 1
-            for (int g0 = 0; g0 < kHalf; g0 += 32) {
-                const int c0 = col0 + g0;
-                float z[32], a[32], t[32];
-                tmem_ld32(taddr + (uint32_t)c0, z);
-                lds32(cst + c0, t);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) gelu_both(z[i] + t[i], a[i], z[i]);
-                lds32(cst + N + c0, t);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) t[i] *= d0;
-                {
-                    float w1[32];
-                    lds32(cst + 2 * N + c0, w1);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) z[i] *= fmaf(d1, w1[i], t[i]);
-                }
-                if (valid) {
-                    store_bf16x32(g.dz_rm + m * N + c0, z);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) g.h_fm[(int64_t)(c0 + i) * g.ld_fm + m] = __float2bfloat16_rn(z[i]);
-                }
-                float *cs = acc.col + c0 + lane;  // this thread's running sums, one column each
-                cs[0] += col_sum32(z, lane);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) t[i] = d0 * a[i];
-                cs[4 * N] += col_sum32(t, lane);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) t[i] = d1 * a[i];
-                cs[8 * N] += col_sum32(t, lane);
-            }
-        }
-    } else {  // EPI_DGELU: dZ1 = acc * GELU'(Z1), feature-major, with the column sums of db1
+    } else {  // EPI_DGELU: dZ1 = acc * GELU'(Z1) with the column sums of db1
 #pragma unroll 1
         for (int g0 = 0; g0 < kHalf; g0 += 32) {
             const int c0 = col0 + g0;
@@ -470,11 +436,8 @@ __device__ __forceinline__ void epilogue(const GemmArgs &g, uint32_t taddr, int 
             }
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = valid ? v[i] * dgelu(__bfloat162float(zin[i])) : 0.f;
-            if (valid) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) g.h_fm[(int64_t)(c0 + i) * g.ld_fm + m] = __float2bfloat16_rn(v[i]);
-            }
-            acc.col[c0 + lane] += col_sum32(v, lane);
+            if (valid) store_bf16x32(g.dz_rm + m * N + c0, v);
+            col[c0 + lane] += col_sum32(v, lane);
         }
     }
 }
@@ -495,7 +458,14 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t addr) {
     return d;
 }
 
-// C = A B^T over the units (row tile, K split) of the grid-stride loop.  BRES: B (N x K, K <= 256)
+// the same of an MN-major operand: rows of 128 B = 64 consecutive M (or N) at one K, eight K to an atom
+// of 1 KB; stride byte offset 1024 to the next eight K, leading byte offset `lead` to the next 64 of
+// M (N); one MMA's 16 K are 2048 B
+__device__ __forceinline__ uint64_t make_sdesc_mn(uint32_t addr, uint32_t lead) {
+    return (make_sdesc_sw128(addr) & ~((uint64_t)0x3FFFu << 16)) | (uint64_t)(lead >> 4) << 16;
+}
+
+// C = A B^T over the row tiles of the grid-stride loop.  BRES: B (N x K, K <= 256)
 // is loaded once and stays in shared memory; otherwise each stage of the ring holds a 64-wide K
 // chunk of A and of B.  Every operand tile is one TMA box of 64 columns (128 B) x its rows.
 template <int N, int EPI, bool BRES>
@@ -504,7 +474,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
     static_assert(N == 64 || N == 256, "N is 64 or 256");
     using C = GemmCfg<N, BRES>;
     constexpr int S = C::kStages;
-    constexpr int kNQ = colsum_quantities<EPI>();
+    constexpr bool kCols = EPI == EPI_DGELU;
     constexpr uint32_t kIdesc = make_idesc(kTileM, N);
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[S], empty[S], tfull[2], tempty[2], bfull, fin;
@@ -512,13 +482,11 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
     __shared__ int abort_s, bwait_s;
     __shared__ long long issued_s, consumed_s;
     __shared__ __align__(16) float cst[const_floats<N, EPI>()];
-    __shared__ float xch[(EPI == EPI_HEAD || EPI == EPI_HEAD_TRAIN) ? 4 : 1][kTileM][2];
-    __shared__ float csum[kNQ > 0 ? kNQ : 1][4][kNQ > 0 ? N : 1];
-    __shared__ float dsum[4][2];
-    __shared__ double lsum[4];
+    __shared__ float xch[EPI == EPI_HEAD ? 2 : 1][kTileM][2];
+    __shared__ float csum[4][kCols ? N : 1];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t units = g.mtiles * g.nsplit;
+    const int64_t units = g.mtiles;
     const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;  // the launch adds 1 KB for this
     const uint32_t ring = BRES ? (uint32_t)g.nchunks * C::kBChunk : 0u;
     if (threadIdx.x == 0) {
@@ -554,9 +522,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
         long long it = 0;
         bool bad = false;
         for (int64_t u = blockIdx.x; u < units && !bad; u += gridDim.x) {
-            const int64_t mt = u % g.mtiles, sp = u / g.mtiles;
-            const int64_t c0 = sp * g.nchunks / g.nsplit, c1 = (sp + 1) * g.nchunks / g.nsplit;
-            for (int64_t c = c0; c < c1; ++c, ++it) {
+            for (int64_t c = 0; c < g.nchunks; ++c, ++it) {
                 const int s = (int)(it % S);
                 if (it >= S && !wait_bar(&empty[s], (uint32_t)((it / S - 1) & 1), abort_p)) {
                     bad = true;
@@ -565,7 +531,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
                 if (lane == 0) {
                     const uint32_t st = sbase + ring + (uint32_t)s * C::kStageBytes;
                     mbar_expect_tx(&full[s], C::kStageBytes);
-                    tma_load_2d(st, &tma_a, (int)(c * kChunkK), (int)(mt * kTileM), &full[s]);
+                    tma_load_2d(st, &tma_a, (int)(c * kChunkK), (int)(u * kTileM), &full[s]);
                     if (!BRES) tma_load_2d(st + kTileABytes, &tma_b, (int)(c * kChunkK), 0, &full[s]);
                     issued_s = it + 1;
                 }
@@ -580,10 +546,8 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
             const int b = (int)(t & 1);
             if (t >= 2 && !wait_bar(&tempty[b], (uint32_t)((t / 2 - 1) & 1), abort_p)) break;
             tc_fence_after();
-            const int64_t sp = u / g.mtiles;
-            const int64_t c0 = sp * g.nchunks / g.nsplit, c1 = (sp + 1) * g.nchunks / g.nsplit;
             const uint32_t acc = tmem + (uint32_t)(b * N);
-            for (int64_t c = c0; c < c1; ++c, ++it) {
+            for (int64_t c = 0; c < g.nchunks; ++c, ++it) {
                 const int s = (int)(it % S);
                 if (!wait_bar(&full[s], (uint32_t)((it / S) & 1), abort_p)) {
                     bad = true;
@@ -596,7 +560,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
 #pragma unroll
                     for (int kk = 0; kk < kChunkK / 16; ++kk)
                         mma_bf16(acc, make_sdesc_sw128(sa + (uint32_t)kk * 32u), make_sdesc_sw128(sb + (uint32_t)kk * 32u),
-                                 kIdesc, (c > c0 || kk > 0) ? 1u : 0u);
+                                 kIdesc, (c > 0 || kk > 0) ? 1u : 0u);
                     mma_commit(&empty[s]);
                     consumed_s = it + 1;
                 }
@@ -618,12 +582,8 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
             }
             named_bar_sync(kEpiBar, kEpiThreads);
         }
-        EpiAcc<N, EPI> acc;
-        acc.col = &csum[0][q][0];
-        if constexpr (kNQ > 0) {
-            for (int j = 0; j < kNQ; ++j)
-                for (int k = 0; k < N / 64; ++k) csum[j][q][h * (N / 2) + 32 * k + lane] = 0.f;
-        }
+        if constexpr (kCols)
+            for (int k = 0; k < N / 64; ++k) csum[q][h * (N / 2) + 32 * k + lane] = 0.f;
         bool broke = false;
         long long t = 0;
         for (int64_t u = blockIdx.x; u < units; u += gridDim.x, ++t) {
@@ -634,36 +594,18 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
                 break;
             }
             tc_fence_after();
-            const int64_t mt = u % g.mtiles, sp = u / g.mtiles;
-            const int64_t m = mt * kTileM + row;
-            epilogue<N, EPI>(g, tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * N), h, lane, row, m, m < g.M, sp,
-                             b, xch, cst, acc);
+            const int64_t m = u * kTileM + row;
+            epilogue<N, EPI>(g, tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * N), h, lane, row, m, m < g.M,
+                             b, xch, cst, csum[q]);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
         }
-        if (kNQ > 0 && !broke) {
+        if (kCols && !broke) {
             // this CTA's column sums: the four row quarters added in order, one row of partials
-            if (EPI == EPI_HEAD_TRAIN && h == 0) {
-                const float s0 = warp_sum(acc.d0), s1 = warp_sum(acc.d1);
-                const double sl = warp_sum(acc.loss);
-                if (lane == 0) {
-                    dsum[q][0] = s0;
-                    dsum[q][1] = s1;
-                    lsum[q] = sl;
-                }
-            }
             named_bar_sync(kEpiBar, kEpiThreads);
-            float *part = g.colpart + (int64_t)blockIdx.x * (EPI == EPI_HEAD_TRAIN ? kHeadPart : N);
-            for (int c = e; c < N; c += kEpiThreads)
-#pragma unroll
-                for (int j = 0; j < (kNQ > 0 ? kNQ : 1); ++j)
-                    part[j * N + c] = ((csum[j][0][c] + csum[j][1][c]) + csum[j][2][c]) + csum[j][3][c];
-            if (EPI == EPI_HEAD_TRAIN && e == 0) {
-                part[3 * N] = ((dsum[0][0] + dsum[1][0]) + dsum[2][0]) + dsum[3][0];
-                part[3 * N + 1] = ((dsum[0][1] + dsum[1][1]) + dsum[2][1]) + dsum[3][1];
-                g.losspart[blockIdx.x] = ((lsum[0] + lsum[1]) + lsum[2]) + lsum[3];
-            }
+            for (int c = e; c < (kCols ? N : 0); c += kEpiThreads)
+                g.colpart[(int64_t)blockIdx.x * N + c] = ((csum[0][c] + csum[1][c]) + csum[2][c]) + csum[3][c];
         }
     }
     __syncthreads();
@@ -728,13 +670,13 @@ int make_tma(CUtensorMap *map, const bf16 *base, int64_t cols, int64_t rows, int
     return RQ_OK;
 }
 
-// A [M][K] (lda), B [N][K] (ldb), K a multiple of 64; g.M, g.nsplit and the epilogue fields set by
+// A [M][K] (lda), B [N][K] (ldb), K a multiple of 64; g.M and the epilogue fields set by
 // the caller; *grid_out (optional) = the CTAs launched (rows of the per-CTA partial sums)
 template <int N, int EPI, bool BRES>
 int launch_gemm_t(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_t K, GemmArgs g, cudaStream_t st,
                   int64_t *grid_out) {
     using C = GemmCfg<N, BRES>;
-    if (g.M < 1 || K < kChunkK || K % kChunkK != 0 || g.nsplit < 1 || g.nsplit > K / kChunkK || (BRES && K > 256))
+    if (g.M < 1 || K < kChunkK || K % kChunkK != 0 || (BRES && K > 256))
         return fail(RQ_E_ARG, "bf16 GEMM: bad shape");
     g.mtiles = (g.M + kTileM - 1) / kTileM;
     g.nchunks = K / kChunkK;
@@ -749,7 +691,7 @@ int launch_gemm_t(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_
     int per_sm = 1;
     RQ_TRY(cache_slot(table, &c));
     RQ_TRY(configure_kernel(k_gemm<N, EPI, BRES>, *c, smem, kGemmThreads, &per_sm));
-    const int64_t units = g.mtiles * g.nsplit;
+    const int64_t units = g.mtiles;
     const int64_t cap = (int64_t)sm_count() * per_sm;
     const int64_t grid = units < cap ? units : cap;
     if (grid > 0x7FFFFFFF) return fail(RQ_E_RANGE, "bf16 GEMM: grid out of range");
@@ -763,7 +705,7 @@ template <int N, int EPI>
 int launch_gemm(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_t K, const GemmArgs &g,
                 cudaStream_t st, int64_t *grid_out = nullptr) {
     if constexpr (EPI == EPI_F32) {  // K <= 256: B stays in shared memory; else B streams with A
-        if (K <= 256 && g.nsplit == 1) return launch_gemm_t<N, EPI, true>(A, lda, B, ldb, K, g, st, grid_out);
+        if (K <= 256) return launch_gemm_t<N, EPI, true>(A, lda, B, ldb, K, g, st, grid_out);
         return launch_gemm_t<N, EPI, false>(A, lda, B, ldb, K, g, st, grid_out);
     } else {  // the layer GEMMs: K = 64 or 256
         return launch_gemm_t<N, EPI, true>(A, lda, B, ldb, K, g, st, grid_out);
@@ -778,8 +720,9 @@ int launch_gemm(const bf16 *A, int64_t lda, const bf16 *B, int64_t ldb, int64_t 
 // never to HBM; as two GEMMs they were written and read back, 134 MB each way for 2^18 rows.  W1 and
 // W2 (160 KB) stay in shared memory, which leaves one tile of X (16 KB) and two of H1's four 64-column
 // quarters (32 KB).  TMEM holds both accumulators (2 x 256 columns).  Bound by the epilogue warps,
-// about 11 instructions per hidden unit of each layer: sixteen of them (eight left three of four issue
-// slots empty).  2^18 rows: 113 us as two GEMMs, 100 with eight epilogue warps, 80 with sixteen.
+// about 8 instructions per hidden unit of each layer: sixteen of them (eight left three of four issue
+// slots empty).  2^18 rows: 113 us as two GEMMs, 100 with eight epilogue warps, 80 with sixteen, 75 with
+// the packed instructions.
 constexpr uint32_t kInfW2 = 0, kInfW1 = 4 * 32768, kInfA = kInfW1 + 32768, kInfH = kInfA + kTileABytes,
                    kInfEnd = kInfH + 2 * kTileABytes;  // 208 KB
 constexpr int kInfWarps = 16;                  // epilogue warps
@@ -919,14 +862,12 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh.d1empty);
                 }
-                __align__(16) bf16 o[16];
+                __align__(16) uint32_t o[8];
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) {
-                    const float4 b = *reinterpret_cast<const float4 *>(sh.cst + c0 + i);
-                    o[i] = __float2bfloat16_rn(gelu(z[i] + b.x));
-                    o[i + 1] = __float2bfloat16_rn(gelu(z[i + 1] + b.y));
-                    o[i + 2] = __float2bfloat16_rn(gelu(z[i + 2] + b.z));
-                    o[i + 3] = __float2bfloat16_rn(gelu(z[i + 3] + b.w));
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(sh.cst + c0 + i);
+                    o[i / 2] = bf16x2(gelu2(add2(pack2(z[i], z[i + 1]), b.x)));
+                    o[i / 2 + 1] = bf16x2(gelu2(add2(pack2(z[i + 2], z[i + 3]), b.y)));
                 }
                 // 16-byte chunk c of row r sits at chunk c ^ (r mod 8) of the row's 128 bytes
                 unsigned char *dst = smem + kInfH + kTileABytes * (uint32_t)s + row * 128;
@@ -951,11 +892,9 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
                 tmem_ld32(lanes + (uint32_t)(kHid + c0 + 32 * k), z[k]);
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
-                    const float4 b = *reinterpret_cast<const float4 *>(sh.cst + kHid + c0 + 32 * k + i);
-                    z[k][i] = gelu(z[k][i] + b.x);
-                    z[k][i + 1] = gelu(z[k][i + 1] + b.y);
-                    z[k][i + 2] = gelu(z[k][i + 2] + b.z);
-                    z[k][i + 3] = gelu(z[k][i + 3] + b.w);
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(sh.cst + kHid + c0 + 32 * k + i);
+                    unpack2(gelu2(add2(pack2(z[k][i], z[k][i + 1]), b.x)), z[k][i], z[k][i + 1]);
+                    unpack2(gelu2(add2(pack2(z[k][i + 2], z[k][i + 3]), b.y)), z[k][i + 2], z[k][i + 3]);
                 }
             }
             tc_fence_before();
@@ -1042,6 +981,8 @@ int launch_infer(const rq_mlp_t *m, int64_t rows, const bf16 *x, float *out, int
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
+
+#include "rq_mlp_train.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // elementwise kernels
@@ -1144,25 +1085,30 @@ __global__ void k_loss(int64_t rows, const float *__restrict__ out, const float 
 
 // loss = sum of the n partial sums / rows: thread t adds part[t], part[t + 256], ... in order, then
 // a fixed tree over the threads (the same sum on every run)
-__global__ void __launch_bounds__(kThreads) k_loss_sum(const double *__restrict__ part, int n, int64_t rows,
-                                                       double *loss) {
+struct LossSum {
+    const double *part;
+    int n;
+    int64_t rows;
+    double *loss;  // null: no sum
+};
+__device__ __forceinline__ void loss_sum(const LossSum &L) {
     __shared__ double red[kThreads];
     double s = 0.;
-    for (int i = threadIdx.x; i < n; i += kThreads) s += part[i];
+    for (int i = threadIdx.x; i < L.n; i += kThreads) s += L.part[i];
     red[threadIdx.x] = s;
     __syncthreads();
     for (int w = kThreads / 2; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *loss = red[0] / (double)rows;
+    if (threadIdx.x == 0) *L.loss = red[0] / (double)L.rows;
 }
+__global__ void __launch_bounds__(kThreads) k_loss_sum(const LossSum L) { loss_sum(L); }
 
 // backward through the output layer: thread j = hidden unit j, 128 rows per block
 __global__ void __launch_bounds__(kHid) k_head_bwd(const bf16 *__restrict__ z2, const float *__restrict__ dout,
-                                                   const float *__restrict__ params, int64_t rows,
-                                                   bf16 *__restrict__ dz2_rm, bf16 *__restrict__ dz2_fm,
-                                                   float *__restrict__ part) {
+                                                   const float *__restrict__ params,
+                                                   bf16 *__restrict__ dz2_rm, float *__restrict__ part) {
     __shared__ float d_s[kTileM][2];
     const int64_t m0 = (int64_t)blockIdx.x * kTileM;
     for (int i = threadIdx.x; i < kTileM * 2; i += blockDim.x) d_s[i >> 1][i & 1] = dout[m0 * 2 + i];
@@ -1171,7 +1117,6 @@ __global__ void __launch_bounds__(kHid) k_head_bwd(const bf16 *__restrict__ z2, 
     const float w30 = params[kOffW3 + j], w31 = params[kOffW3 + kHid + j];
     float aw0 = 0.f, aw1 = 0.f, ab = 0.f;
     for (int r0 = 0; r0 < kTileM; r0 += 8) {
-        __align__(16) bf16 buf[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int64_t m = m0 + r0 + q;
@@ -1179,14 +1124,11 @@ __global__ void __launch_bounds__(kHid) k_head_bwd(const bf16 *__restrict__ z2, 
             const float h = gelu(z);
             const float d0 = d_s[r0 + q][0], d1 = d_s[r0 + q][1];
             const float dz = (d0 * w30 + d1 * w31) * dgelu(z);
-            const bf16 b = __float2bfloat16_rn(dz);
-            dz2_rm[m * kHid + j] = b;
-            buf[q] = b;
+            dz2_rm[m * kHid + j] = __float2bfloat16_rn(dz);
             aw0 += d0 * h;
             aw1 += d1 * h;
             ab += dz;
         }
-        *reinterpret_cast<uint4 *>(dz2_fm + (int64_t)j * rows + m0 + r0) = *reinterpret_cast<const uint4 *>(buf);
     }
     float *p = part + (int64_t)blockIdx.x * kHeadPart;
     p[j] = ab;
@@ -1199,6 +1141,8 @@ __global__ void __launch_bounds__(kHid) k_head_bwd(const bf16 *__restrict__ z2, 
     }
 }
 
+// Bound by the latency of its reads (31 MB of partials for 65,536 rows): kColsumRows rows are in flight
+// per lane (two: 11.2 us; eight, with the loss sum that was a launch of 4.6 us: 9.9 us).
 // dst[c] = sum_t part[t * ncols + c] for up to four sets of partial sums in one launch: a block
 // of kColsumWarps warps per 32 VW columns of one set (lane = VW consecutive columns, so every row
 // of partials is read in 32 VW-wide coalesced pieces); warp w adds the rows t in its contiguous
@@ -1206,6 +1150,7 @@ __global__ void __launch_bounds__(kHid) k_head_bwd(const bf16 *__restrict__ z2, 
 // order of every addition is fixed, so the sums are the same on every run.  VW = 4 needs ncols a
 // multiple of 4 and 16-byte aligned rows.
 constexpr int kColsumWarps = 8;
+constexpr int kColsumRows = 8;  // even
 struct ColsumSet {
     const float *part;
     int64_t nt, ncols;
@@ -1228,6 +1173,25 @@ __device__ __forceinline__ void colsum_block(const ColsumSet &g, int64_t blk, fl
     float a[2][VW] = {};
     if (c < ncols) {
         int64_t t = t0;
+        for (; t + kColsumRows <= t1; t += kColsumRows) {  // rows in flight together
+            float v[kColsumRows][VW];
+#pragma unroll
+            for (int k = 0; k < kColsumRows; ++k) {
+                if constexpr (VW == 4) {
+                    const float4 f = __ldg(reinterpret_cast<const float4 *>(part + (t + k) * ncols + c));
+                    v[k][0] = f.x;
+                    v[k][1] = f.y;
+                    v[k][2] = f.z;
+                    v[k][3] = f.w;
+                } else {
+                    v[k][0] = __ldg(part + (t + k) * ncols + c);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kColsumRows; ++k)
+#pragma unroll
+                for (int j = 0; j < VW; ++j) a[k & 1][j] += v[k][j];
+        }
         for (; t + 2 <= t1; t += 2) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -1267,19 +1231,22 @@ __device__ __forceinline__ void colsum_block(const ColsumSet &g, int64_t blk, fl
     }
 }
 
-__global__ void __launch_bounds__(kColsumWarps * 32) k_colsum(const ColsumSets S) {
+__global__ void __launch_bounds__(kColsumWarps * 32) k_colsum(const ColsumSets S, const LossSum L) {
+    static_assert(kColsumWarps * 32 == kThreads, "the blocks of loss_sum");
     __shared__ float ws[kColsumWarps][32 * 4 + 1];
     int64_t b = blockIdx.x;
     int k = 0;
-    while (k < S.n - 1 && b >= S.s[k].blocks) b -= S.s[k++].blocks;
-    if (S.s[k].vw == 4)
+    while (k < S.n && b >= S.s[k].blocks) b -= S.s[k++].blocks;
+    if (k == S.n)  // the block after the last set's
+        loss_sum(L);
+    else if (S.s[k].vw == 4)
         colsum_block<4>(S.s[k], b, ws);
     else
         colsum_block<1>(S.s[k], b, ws);
 }
 
-// the column sums of n (<= 4) sets of partials, one launch
-int launch_colsums(const ColsumSet *sets, int n, cudaStream_t st) {
+// the column sums of n (<= 4) sets of partials and, where wanted, the loss, one launch
+int launch_colsums(const ColsumSet *sets, int n, const LossSum &loss, cudaStream_t st) {
     ColsumSets S{};
     S.n = n;
     int64_t total = 0;
@@ -1289,8 +1256,8 @@ int launch_colsums(const ColsumSet *sets, int n, cudaStream_t st) {
         S.s[k].blocks = (int)((sets[k].ncols + 32 * S.s[k].vw - 1) / (32 * S.s[k].vw));
         total += S.s[k].blocks;
     }
-    if (n < 1 || n > 4 || total < 1 || total > 0x7FFFFFFF) return fail(RQ_E_RANGE, "column sums: bad sets");
-    k_colsum<<<(unsigned)total, kColsumWarps * 32, 0, st>>>(S);
+    if (n < 1 || n > 4 || total < 1 || total >= 0x7FFFFFFF) return fail(RQ_E_RANGE, "column sums: bad sets");
+    k_colsum<<<(unsigned)(total + (loss.loss ? 1 : 0)), kColsumWarps * 32, 0, st>>>(S, loss);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -1338,7 +1305,7 @@ __global__ void k_warm_start(int64_t D, const float *__restrict__ out, V *__rest
 // ---------------------------------------------------------------------------------------------
 struct MlpLayout {
     int64_t Mp, tiles, nsplit, nsplit1;
-    size_t err, z1, h1, h1t, z2, dz2, dz2t, dz1t, colpart1, part2, split2, split1, lossp, total;
+    size_t err, z1, h1, z2, dz2, dz1, colpart1, part2, split2, split1, lossp, total;
 };
 
 
@@ -1358,11 +1325,9 @@ MlpLayout mlp_layout(int64_t rows) {
     L.err = take(16);
     L.z1 = take(act);
     L.h1 = take(act);
-    L.h1t = take(act);
     L.z2 = take(act);
     L.dz2 = take(act);
-    L.dz2t = take(act);
-    L.dz1t = take(act);
+    L.dz1 = take(act);
     L.colpart1 = take((size_t)L.tiles * kHid * sizeof(float));  // one row per tile (k_head_bwd) or CTA
     L.part2 = take((size_t)L.tiles * kHeadPart * sizeof(float));
     L.split2 = take((size_t)L.nsplit * kHid * kHid * sizeof(float));
@@ -1425,63 +1390,33 @@ RQ_API int rq_mlp_sample(const uint64_t *states, int64_t D, const double *U, con
 namespace rq {
 namespace {
 
-// layer 1: Z1 = X W1^T + b1 and H1 = GELU(Z1), row-major, and H1 feature-major (the B operand of dW2)
+// layer 1: Z1 = X W1^T + b1 and H1 = GELU(Z1)
 int layer1(const rq_mlp_t *m, int64_t rows, const uint16_t *x, const MlpLayout &L, char *w, int *err,
            cudaStream_t st) {
     GemmArgs g{};
     g.M = rows;
-    g.nsplit = 1;
     g.bias = m->params + kOffB1;
     g.z_rm = reinterpret_cast<bf16 *>(w + L.z1);
     g.h_rm = reinterpret_cast<bf16 *>(w + L.h1);
-    g.h_fm = reinterpret_cast<bf16 *>(w + L.h1t);
-    g.ld_fm = L.Mp;
     g.err = err;
     return launch_gemm<kHid, EPI_HIDDEN>(reinterpret_cast<const bf16 *>(x), kIn,
                                          reinterpret_cast<const bf16 *>(m->w1b), kIn, kIn, g, st);
 }
 
-// dZ1 = (dZ2 W2) * GELU'(Z1) feature-major with the b1 partial sums, dW2 = dZ2^T H1 and
-// dW1 = dZ1^T X split over the rows (column-major partial products), and the sums of every set of
-// partials into m->grads
-int backward_tail(const rq_mlp_t *m, int64_t rows, const uint16_t *xt, const MlpLayout &L, char *w, int *err,
-                  const float *part2, int64_t part2_rows, cudaStream_t st) {
-    GemmArgs g{};
-    g.M = rows;
-    g.nsplit = 1;
-    g.zin_rm = reinterpret_cast<const bf16 *>(w + L.z1);
-    g.h_fm = reinterpret_cast<bf16 *>(w + L.dz1t);
-    g.ld_fm = L.Mp;
-    g.colpart = reinterpret_cast<float *>(w + L.colpart1);
-    g.err = err;
-    int64_t grid1 = 0;
-    RQ_TRY((launch_gemm<kHid, EPI_DGELU>(reinterpret_cast<const bf16 *>(w + L.dz2), kHid,
-                                         reinterpret_cast<const bf16 *>(m->w2tb), kHid, kHid, g, st, &grid1)));
-    // dW2^T = H1^T dZ2: A = H1 feature-major (rows n), B = dZ2 feature-major (columns j); the
-    // column-major partial product [j][n] is dW2 in its row-major layout
-    GemmArgs a{};
-    a.M = kHid;
-    a.nsplit = L.nsplit;
-    a.out = reinterpret_cast<float *>(w + L.split2);
-    a.split_cm = 1;
-    a.err = err;
-    RQ_TRY((launch_gemm<kHid, EPI_F32>(reinterpret_cast<const bf16 *>(w + L.h1t), L.Mp,
-                                       reinterpret_cast<const bf16 *>(w + L.dz2t), L.Mp, L.Mp, a, st)));
-    // dW1^T = X^T dZ1: a 64-row A tile (rows 64..127 read as zeros), one row tile, twice the splits
-    GemmArgs b{};
-    b.M = kIn;
-    b.nsplit = L.nsplit1;
-    b.out = reinterpret_cast<float *>(w + L.split1);
-    b.split_cm = 1;
-    b.err = err;
-    RQ_TRY((launch_gemm<kHid, EPI_F32>(reinterpret_cast<const bf16 *>(xt), L.Mp,
-                                       reinterpret_cast<const bf16 *>(w + L.dz1t), L.Mp, L.Mp, b, st)));
+// dW2 = dZ2^T H1 and dW1 = dZ1^T X split over the rows, and the sums of every set of partials (b1's of
+// np1, the head's of np2 rows) into m->grads; with loss, the sum of its np2 partials there
+int weight_grads(const rq_mlp_t *m, int64_t rows, const uint16_t *xt, const MlpLayout &L, char *w, int *err,
+                 int64_t np1, int64_t np2, double *loss, cudaStream_t st) {
+    RQ_TRY(launch_wgrad(reinterpret_cast<const bf16 *>(w + L.h1), reinterpret_cast<const bf16 *>(w + L.dz2),
+                        reinterpret_cast<const bf16 *>(xt), reinterpret_cast<const bf16 *>(w + L.dz1), L.Mp, L.nsplit,
+                        L.nsplit1, reinterpret_cast<float *>(w + L.split2), reinterpret_cast<float *>(w + L.split1), err,
+                        st));
     const ColsumSet sets[4] = {
         {reinterpret_cast<const float *>(w + L.split1), L.nsplit1, kHid * kIn, m->grads + kOffW1, 0, 0},
-        {reinterpret_cast<const float *>(w + L.colpart1), grid1, kHid, m->grads + kOffB1, 0, 0},
+        {reinterpret_cast<const float *>(w + L.colpart1), np1, kHid, m->grads + kOffB1, 0, 0},
         {reinterpret_cast<const float *>(w + L.split2), L.nsplit, kHid * kHid, m->grads + kOffW2, 0, 0},
-        {part2, part2_rows, kHeadPart, m->grads + kOffB2, 0, 0}};
-    return launch_colsums(sets, 4, st);
+        {reinterpret_cast<const float *>(w + L.part2), np2, kHeadPart, m->grads + kOffB2, 0, 0}};
+    return launch_colsums(sets, 4, LossSum{reinterpret_cast<const double *>(w + L.lossp), (int)np2, rows, loss}, st);
 }
 
 }  // namespace
@@ -1498,7 +1433,6 @@ RQ_API int rq_mlp_fwd(const rq_mlp_t *m, int64_t rows, const uint16_t *x, float 
     RQ_TRY(layer1(m, rows, x, L, w, err, st));
     GemmArgs h{};
     h.M = rows;
-    h.nsplit = 1;
     h.bias = m->params + kOffB2;
     h.z_rm = reinterpret_cast<bf16 *>(w + L.z2);
     h.out = out;
@@ -1528,7 +1462,7 @@ RQ_API int rq_mlp_loss(int64_t rows, const float *out, const float *tgt, float *
     const int grid = std::min(grid_for(rows), 4096);
     cudaStream_t st = as_stream(stream);
     k_loss<<<grid, kThreads, 0, st>>>(rows, out, tgt, dout, part);
-    if (loss) k_loss_sum<<<1, kThreads, 0, st>>>(part, grid, rows, loss);
+    if (loss) k_loss_sum<<<1, kThreads, 0, st>>>(LossSum{part, grid, rows, loss});
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }
@@ -1544,10 +1478,19 @@ RQ_API int rq_mlp_bwd(const rq_mlp_t *m, int64_t rows, const uint16_t *xt, const
     int *err = reinterpret_cast<int *>(w + L.err);
     float *part2 = reinterpret_cast<float *>(w + L.part2);
     k_head_bwd<<<(unsigned)L.tiles, kHid, 0, st>>>(reinterpret_cast<const bf16 *>(w + L.z2), dout, m->params,
-                                                   L.Mp, reinterpret_cast<bf16 *>(w + L.dz2),
-                                                   reinterpret_cast<bf16 *>(w + L.dz2t), part2);
+                                                   reinterpret_cast<bf16 *>(w + L.dz2), part2);
     RQ_CUDA(cudaGetLastError());
-    return backward_tail(m, rows, xt, L, w, err, part2, L.tiles, st);
+    // dZ1 = (dZ2 W2) * GELU'(Z1) with the b1 partial sums
+    GemmArgs g{};
+    g.M = rows;
+    g.zin_rm = reinterpret_cast<const bf16 *>(w + L.z1);
+    g.dz_rm = reinterpret_cast<bf16 *>(w + L.dz1);
+    g.colpart = reinterpret_cast<float *>(w + L.colpart1);
+    g.err = err;
+    int64_t grid1 = 0;
+    RQ_TRY((launch_gemm<kHid, EPI_DGELU>(reinterpret_cast<const bf16 *>(w + L.dz2), kHid,
+                                         reinterpret_cast<const bf16 *>(m->w2tb), kHid, kHid, g, st, &grid1)));
+    return weight_grads(m, rows, xt, L, w, err, grid1, L.tiles, nullptr, st);
 }
 
 RQ_API int rq_mlp_train(const rq_mlp_t *m, int64_t rows, const uint16_t *x, const uint16_t *xt, const float *tgt,
@@ -1560,31 +1503,12 @@ RQ_API int rq_mlp_train(const rq_mlp_t *m, int64_t rows, const uint16_t *x, cons
     cudaStream_t st = as_stream(stream);
     int *err = reinterpret_cast<int *>(w + L.err);
     RQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-    RQ_TRY(layer1(m, rows, x, L, w, err, st));
-    // layer 2 with the output layer, the loss and its gradient back to dZ2 in one epilogue
-    GemmArgs h{};
-    h.M = rows;
-    h.nsplit = 1;
-    h.bias = m->params + kOffB2;
-    h.out = out;
-    h.w3 = m->params + kOffW3;
-    h.b3 = m->params + kOffB3;
-    h.tgt = tgt;
-    h.inv_rows = 1.f / (float)rows;
-    h.dz_rm = reinterpret_cast<bf16 *>(w + L.dz2);
-    h.h_fm = reinterpret_cast<bf16 *>(w + L.dz2t);
-    h.ld_fm = L.Mp;
-    h.colpart = reinterpret_cast<float *>(w + L.part2);
-    h.losspart = reinterpret_cast<double *>(w + L.lossp);
-    h.err = err;
-    int64_t grid2 = 0;
-    RQ_TRY((launch_gemm<kHid, EPI_HEAD_TRAIN>(reinterpret_cast<const bf16 *>(w + L.h1), kHid,
-                                              reinterpret_cast<const bf16 *>(m->w2b), kHid, kHid, h, st, &grid2)));
-    if (loss) {
-        k_loss_sum<<<1, kThreads, 0, st>>>(reinterpret_cast<const double *>(w + L.lossp), (int)grid2, rows, loss);
-        RQ_CUDA(cudaGetLastError());
-    }
-    return backward_tail(m, rows, xt, L, w, err, reinterpret_cast<const float *>(w + L.part2), grid2, st);
+    int64_t grid = 0;
+    RQ_TRY(launch_train(m, rows, reinterpret_cast<const bf16 *>(x), tgt, out, reinterpret_cast<bf16 *>(w + L.h1),
+                        reinterpret_cast<bf16 *>(w + L.dz2), reinterpret_cast<bf16 *>(w + L.dz1),
+                        reinterpret_cast<float *>(w + L.colpart1), reinterpret_cast<float *>(w + L.part2),
+                        reinterpret_cast<double *>(w + L.lossp), err, st, &grid));
+    return weight_grads(m, rows, xt, L, w, err, grid, grid, loss, st);
 }
 
 RQ_API int rq_mlp_step(const rq_mlp_t *m, int32_t t, float lr, float beta1, float beta2, float eps,
@@ -1623,7 +1547,6 @@ RQ_API int rq_bf16_gemm(const uint16_t *A, int64_t lda, const uint16_t *B, int64
     RQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     GemmArgs g{};
     g.M = M;
-    g.nsplit = 1;
     g.out = C;
     g.err = err;
     const bf16 *a = reinterpret_cast<const bf16 *>(A), *b = reinterpret_cast<const bf16 *>(B);

@@ -276,3 +276,36 @@ def test_fused_inference_equals_forward_bits(rows):
     m.infer(x, out=guard[:rows])
     assert torch.equal(guard[:rows], m.forward(x)) and bool((guard[rows:] == 7.).all())
     m.check_errors()
+
+
+@pytest.mark.parametrize('tiles', [1, 2, 151, 152, 153, 305])
+def test_training_step_over_tile_counts(tiles):
+    """The fused training step with fewer tiles than CTAs, one per CTA, one more, and a third turn: the
+    outputs have the bits of the forward pass, the gradients are those of the separate calls up to the
+    BF16 rounding of Z2 that only these do, and outputs are optional."""
+    import torch
+    from rqutils_gb300.warmstart import WarmStartMLP, OFF_B1, OFF_B2, OFF_W2, NPARAMS
+    rows = 128 * tiles
+    m = WarmStartMLP(seed=31)
+    g = torch.Generator().manual_seed(32)
+    x = _features(1024, 33)[torch.randint(0, 1024, (rows,), generator=g).cuda()].contiguous()
+    tgt = torch.stack([torch.randn(rows, generator=g) - 2.,
+                       torch.where(torch.rand(rows, generator=g) < 0.5, -1., 1.),
+                       torch.rand(rows, generator=g) + 0.1], 1).cuda()
+    xt = x.T.contiguous()
+    ref = m.forward(x)
+    loss = [torch.zeros(1, dtype=torch.float64, device='cuda') for _ in range(2)]
+    dout = m.loss(ref, tgt, loss=loss[0])
+    m.backward(xt, dout)
+    ga = m.grads.clone()
+    out = torch.empty_like(ref)
+    m.train_step(x, xt, tgt, out=out, loss=loss[1])
+    gb = m.grads.clone()
+    m.train_step(x, xt, tgt)
+    torch.cuda.synchronize()
+    m.check_errors()
+    assert torch.equal(out, ref)
+    assert abs(loss[1].item() - loss[0].item()) <= 1e-6 * abs(loss[0].item())
+    assert torch.equal(m.grads, gb)
+    for a, b in [(0, OFF_B1), (OFF_B1, OFF_W2), (OFF_W2, OFF_B2), (OFF_B2, NPARAMS)]:
+        assert (gb[a:b] - ga[a:b]).norm().item() < 1e-2 * ga[a:b].norm().item(), (a, b)
