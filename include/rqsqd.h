@@ -97,7 +97,8 @@ typedef struct rq_subspace {
     int32_t   lbits;         /* log2(lines) of lmap, from rq_line_filter_bits               */
     int32_t   lwbits;        /* log2(bits per line): 8 (32-byte lines) .. 10 (128-byte)     */
     int32_t   lshift;        /* written by rq_subspace_build: the prefix shift, chosen so that
-                                about 2^(lwbits - 5) states share a prefix on average        */
+                                about 2^(lwbits - 5) states share a prefix on average, and at
+                                most three times as many the average state's prefix          */
     int32_t   fpoint;        /* written by rq_subspace_build: pa * 65 + pb when every state has
                                 the same pair pa = popcount(s & fmask_a), pb = popcount(s &
                                 fmask_b) (a subspace in one sector), else -1; -1 with the
@@ -407,8 +408,8 @@ int rq_mlp_sample(const uint64_t *states, int64_t D, const double *U, const floa
 /* out[rows][2] = f(x); keeps the activations in ws for rq_mlp_bwd. */
 int rq_mlp_fwd(const rq_mlp_t *m, int64_t rows, const uint16_t *x, float *out, void *ws,
                void *stream);
-/* out[rows][2] = f(x) without keeping the activations for rq_mlp_bwd (inference: only the
- * hidden activations that layer 2 reads are written to ws). */
+/* out[rows][2] = f(x) without keeping the activations for rq_mlp_bwd (inference: one kernel, which
+ * writes only its error flag to ws). */
 int rq_mlp_infer(const rq_mlp_t *m, int64_t rows, const uint16_t *x, float *out, void *ws,
                  void *stream);
 /* dout[rows][2] of the weighted loss mean_i w_i ((o0 - a_i)^2 + softplus(-s_i o1)); the loss

@@ -501,8 +501,8 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
             return RQ_OK;
         }
         const int rows = tile_rows<V>(B.D, B.nnz, sm_count());
-        const int64_t tiles = (B.D + rows - 1) / rows, cap = (int64_t)sm_count() * 8;
-        k_batch_matvec_conn<V><<<(int)std::min(tiles, cap), kThreads, 0, st>>>(
+        const int64_t tiles = (B.D + rows - 1) / rows;
+        k_batch_matvec_conn<V><<<(int)std::min<int64_t>(tiles, 0x7FFFFFFF), kThreads, 0, st>>>(
             B, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gstride, gate2);
     } else {
         return fail(RQ_E_ARG, "rq_batch_matvec: mode must be RQ_MODE_FREE or RQ_MODE_CONN");

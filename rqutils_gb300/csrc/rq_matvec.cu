@@ -582,18 +582,79 @@ int grid_rows(int64_t n) {
     return (int)(g > cap ? cap : (g < 1 ? 1 : g));
 }
 
-// blocks of the tiled cached products: 8 resident per SM (17 KB of shared memory, 32 registers)
-int grid_tiles(int64_t D, int rows) {
-    const int64_t g = (D + rows - 1) / rows, cap = (int64_t)sm_count() * 8;
-    return (int)(g > cap ? cap : g);
-}
+// Blocks of the tiled cached products: one per tile, so that a block that ends makes room for the next
+// (with as many as are resident, each walking several tiles, the chip waited for the longest walk:
+// 36 qubits, 150,001 rows, CONN 731 against 570 us in float64, 1616 against 1297 in complex128).
+int grid_tiles(int64_t D, int rows) { return (int)std::min<int64_t>((D + rows - 1) / rows, 0x7FFFFFFF); }
 
 // ------------------------------------------------------------------------------------------
 // CONN and CSR modes
 // ------------------------------------------------------------------------------------------
+template <typename R>
+__device__ __forceinline__ R shfl_product(R v, int src) {
+    return __shfl_sync(0xffffffffu, v, src);
+}
+template <typename R>
+__device__ __forceinline__ cx<R> shfl_product(cx<R> v, int src) {
+    return {__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+}
+
+// Rows shorter than one element on average: a warp takes 32 kShortRows rows, whose elements are
+// consecutive in the list, forms up to 32 products at once (the FP64 pipe takes 64 cycles for a
+// warp's instruction, however few lanes have an element) and hands them to the rows by shuffles, in
+// list order.  No barriers, and twice the loads in flight.  2^20 rows of 0.2 (Hubbard 4x4), CSR, against
+// a thread per row: float64 10.4 us against 14.4, complex64 8.3 against 10.4, complex128 18.5 against
+// 32.8 (one row a lane: 11.5, 8.9, 22.6; four: 10.8, 8.4, 19.7); CONN, against tiles: float64 14.5
+// against 16.7, complex64 13.7 against 16.7, but complex128 28.7 against 26.9: that one keeps them.
+// elem, first and done as of tile_product.
+constexpr int kShortRows = 2;
+template <typename V, typename E, typename F, typename S>
+__device__ __forceinline__ void short_rows(const int64_t *rowptr, int64_t D, E &&elem, F &&first, S &&done) {
+    using RT = RowTerm<V>;
+    constexpr int kR = kShortRows;
+    const int lane = threadIdx.x & 31;
+    const int64_t b = (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kR);
+    if (b >= D) return;
+    int64_t e[kR], e1[kR];
+    typename RT::A acc[kR];
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+        const int64_t i = b + 32 * k + lane;
+        e[k] = rowptr[i < D ? i : D];
+        e1[k] = rowptr[i < D ? i + 1 : D];
+        if (i < D) first(i, acc[k]);
+    }
+    const int64_t w0 = __shfl_sync(0xffffffffu, e[0], 0), w1 = __shfl_sync(0xffffffffu, e1[kR - 1], 31);
+    for (int64_t c = w0; c < w1; c += 32) {
+        typename RT::P p{};
+        if (c + lane < w1) p = elem(c + lane);
+#pragma unroll
+        for (int k = 0; k < kR; ++k) {
+            const int64_t stop = e1[k] < c + 32 ? e1[k] : c + 32;
+            while (__any_sync(0xffffffffu, e[k] < stop)) {
+                const typename RT::P q = shfl_product(p, (int)(e[k] - c) & 31);
+                if (e[k] < stop) {
+                    acc[k].add(q);
+                    ++e[k];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+        const int64_t i = b + 32 * k + lane;
+        if (i < D) done(i, acc[k]);
+    }
+}
+inline bool rows_short(int64_t D, int64_t nnz) { return nnz < D; }
+inline unsigned grid_short(int64_t D) {
+    constexpr int kRows = kThreads * kShortRows;
+    return (unsigned)((D + kRows - 1) / kRows);
+}
+
 // Element e of group g with source row m belongs to the row of state S[m] ^ x_g, so an element
-// needs no search for its row.
-template <typename V>
+// needs no search for its row.  SHORT: rows shorter than one element.
+template <typename V, bool SHORT>
 __global__ void __launch_bounds__(kThreads)
 k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int rows, const int *gate,
               const int *gate2) {
@@ -602,23 +663,26 @@ k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     const rq_terms_t &T = op.terms;
     const int64_t D = op.sub.D;
-    for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
-        tile_product<V>(
-            op.rowptr, r0, (int)min((int64_t)rows, D - r0), long_groups(T),
-            [&](int64_t e) {
-                const int m = __ldg(op.col + e), g = __ldg(op.grp + e);
-                return RT::product(T, g, __ldg(op.sub.states + m) ^ __ldg(T.xmask + g), x, m);
-            },
-            [&](int64_t e) { return group_terms(T, __ldg(op.grp + e)); },
-            [&](int64_t i, typename RT::A &acc) {
-                if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
-                else if (T.diag_group >= 0) acc.add(RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
-            },
-            [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); });
+    auto elem = [&](int64_t e) {
+        const int m = __ldg(op.col + e), g = __ldg(op.grp + e);
+        return RT::product(T, g, __ldg(op.sub.states + m) ^ __ldg(T.xmask + g), x, m);
+    };
+    auto first = [&](int64_t i, typename RT::A &acc) {
+        if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+        else if (T.diag_group >= 0) acc.add(RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
+    };
+    auto done = [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); };
+    if constexpr (SHORT)
+        short_rows<V>(op.rowptr, D, elem, first, done);
+    else
+        for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
+            tile_product<V>(
+                op.rowptr, r0, (int)min((int64_t)rows, D - r0), long_groups(T), elem,
+                [&](int64_t e) { return group_terms(T, __ldg(op.grp + e)); }, first, done);
 }
 
 // VV: storage type of the element values (converted to the vector's precision on load)
-template <typename V, typename VV>
+template <typename V, typename VV, bool SHORT>
 __global__ void __launch_bounds__(kThreads)
 k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int rows, const int *gate,
              const int *gate2) {
@@ -627,24 +691,24 @@ k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y,
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     const VV *val = reinterpret_cast<const VV *>(op.val);
     const int64_t D = op.sub.D;
-    for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
-        tile_product<V>(
-            op.rowptr, r0, (int)min((int64_t)rows, D - r0), false,
-            [&](int64_t e) {
-                const auto v = VT<VV>::ld(val, e);
-                return RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e));
-            },
-            [](int64_t) { return 0; },
-            [&](int64_t i, typename RT::A &acc) {
-                if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
-            },
-            [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); });
+    auto elem = [&](int64_t e) {
+        const auto v = VT<VV>::ld(val, e);
+        return RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e));
+    };
+    auto first = [&](int64_t i, typename RT::A &acc) {
+        if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+    };
+    auto done = [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); };
+    if constexpr (SHORT)
+        short_rows<V>(op.rowptr, D, elem, first, done);
+    else
+        for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
+            tile_product<V>(op.rowptr, r0, (int)min((int64_t)rows, D - r0), false, elem, [](int64_t) { return 0; }, first,
+                            done);
 }
 
-// A thread per row: no barriers, so better where rows are shorter than one element on average (2^20
-// rows of 0.2, float64: 10.3 us against 12.5 with tiles) and, for complex128, where they are long and
-// there are enough of them (150,001 rows of 83: 745 us against 891; its products fill a tile's buffer
-// with a dozen rows).
+// A thread per row, for complex128 rows that are long and many (150,001 rows of 83: 750 us against 805
+// with tiles, whose buffer a dozen rows fill).
 template <typename V, typename VV>
 __global__ void __launch_bounds__(kThreads)
 k_matvec_csr_rows(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, const int *gate,
@@ -670,11 +734,13 @@ template <typename V, typename VV>
 void run_csr(const rq_operator_t &op, const V *x, V *y, cudaStream_t st, const int *gate, const int *gate2) {
     const int64_t D = op.sub.D;
     const double avg = (double)op.nnz / (double)D;
-    if (avg < 1. || (sizeof(V) == 16 && avg > 48. && D > 65536)) {
+    if (rows_short(D, op.nnz)) {
+        k_matvec_csr<V, VV, true><<<grid_short(D), kThreads, 0, st>>>(op, x, y, 0, gate, gate2);
+    } else if (sizeof(V) == 16 && avg > 48. && D > 65536) {
         k_matvec_csr_rows<V, VV><<<grid_rows(D), kThreads, 0, st>>>(op, x, y, gate, gate2);
     } else {
         const int rows = tile_rows<V>(D, op.nnz, sm_count());
-        k_matvec_csr<V, VV><<<grid_tiles(D, rows), kThreads, 0, st>>>(op, x, y, rows, gate, gate2);
+        k_matvec_csr<V, VV, false><<<grid_tiles(D, rows), kThreads, 0, st>>>(op, x, y, rows, gate, gate2);
     }
 }
 
@@ -818,9 +884,12 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
         case RQ_MODE_CONN:
             if (!op.rowptr || (op.nnz > 0 && (!op.col || !op.grp)))
                 return fail(RQ_E_ARG, "rq_matvec: RQ_MODE_CONN needs rowptr, col and grp");
-            {
+            if (sizeof(V) < 16 && rows_short(op.sub.D, op.nnz)) {
+                k_matvec_conn<V, true><<<grid_short(op.sub.D), kThreads, 0, st>>>(
+                    op, static_cast<const V *>(x), static_cast<V *>(y), 0, gate, gate2);
+            } else {
                 const int rows = tile_rows<V>(op.sub.D, op.nnz, sm_count());
-                k_matvec_conn<V><<<grid_tiles(op.sub.D, rows), kThreads, 0, st>>>(
+                k_matvec_conn<V, false><<<grid_tiles(op.sub.D, rows), kThreads, 0, st>>>(
                     op, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gate2);
             }
             RQ_CUDA(cudaGetLastError());

@@ -253,8 +253,6 @@ __device__ __forceinline__ Lists<V> load_lists(const ListOp &L, int64_t r0, int6
 }
 
 // accumulator of a product row: FP64 plain, FP32 compensated
-template <typename V>
-struct MvAcc;
 template <typename R, bool CPLX>
 struct MvAccT {
     Acc<R> re, im;

@@ -99,3 +99,35 @@ def test_clustered_subspaces(n, keep, D, dtype):
     conn = DeviceOperator(terms, sub, mode='conn')
     assert conn.nnz >= 2 * D  # 3 to 40 a row
     assert torch.equal(conn.matvec(x), y)
+
+
+@pytest.mark.parametrize('first', [True, False])
+@pytest.mark.parametrize('D', [1100, 1983, 1984, 1985, 2047, 2048, 2049, 4097])
+@pytest.mark.parametrize('dtype', ['float64', 'complex64', 'complex128'])
+def test_short_rows_equal_matrix_free_bits(D, first, dtype):
+    """Fewer elements than rows, at the edges of a warp's 64 rows and a block's 512: 32 rows of up to 32
+    elements (several times 32 for one warp, at either end of the array) among empty ones."""
+    import torch
+    from rqutils_gb300 import workloads
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    from rqutils_gb300.sqd import SQDProblem
+    rng = np.random.default_rng(D)
+    labels, coeffs = workloads.random_pauli_masks(rng, 5, 150, locality=(1, 5))
+    if dtype == 'float64':
+        labels = [s if s.count('Y') % 2 == 0 else s.replace('Y', 'X') for s in labels]
+    labels = ['IZ' + 'I' * 17 + s for s in labels]
+    ham = PauliSumXZ.from_paulisum((labels, coeffs), force_real=True, add_padding=True)
+    group = np.arange(32) + (0 if first else 1 << 23)
+    # spread states differ from each other and from the group above the bits that the terms flip
+    spread = (rng.choice(np.arange(1, 1 << 18), size=D - 32, replace=False) << 5) + rng.integers(0, 32, D - 32)
+    S = np.sort(np.concatenate([group, spread])).astype(np.uint64)
+    free, conn, csr = [SQDProblem(ham, S, cache_level=c).op for c in ((0, 0), (1, 0), (1, 2))]
+    assert 32 * 16 < conn.c.nnz < D
+    x = torch.randn(D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(D))
+    y = free.matvec(x)
+    assert torch.equal(conn.matvec(x), y)
+    if dtype != 'complex64':
+        assert torch.equal(csr.matvec(x), y)
+    else:
+        ref = csr.matvec(x.to(torch.complex128))
+        assert torch.linalg.vector_norm(csr.matvec(x) - ref) <= 1e-6 * torch.linalg.vector_norm(ref)
