@@ -58,7 +58,7 @@ __device__ __forceinline__ bool sector_pass(K t, K fa, K fbm, int pa0, int pb0) 
 //   groups of more than kShortTerms terms go to a second queue, so that short ones do not wait;
 // * the owner lane of a row adds its products from the queue in group order, as the cached products do.
 // Hubbard 4x4, complex64, against a loop of each lane over its own hits (48 warps per SM instead of
-// 32): 2^20 rows 75 us against 78, 2^17 low-energy rows 47 against 59.
+// 32): 2^20 rows 75 us against 78, 2^18 low-energy rows 47 against 59.
 constexpr int kQueueSlots = 128;  // hits resolved together
 
 template <typename V>

@@ -807,7 +807,7 @@ int launch_line_block(const rq_operator_t &op, int lw, const void *x, void *y, i
     int64_t g = (op.sub.D + rows - 1) / rows;
     // As many blocks as are resident, each walking several tiles; four times as many where each still has
     // a tile: one that ends early makes room (Hubbard 4x4, 2^20 rows, complex64: 75.7 against 71.8 us;
-    // with fewer tiles the group keys of the extra blocks cost more: 2^17 low-energy rows, float64, 44.3
+    // with fewer tiles the group keys of the extra blocks cost more: 2^18 low-energy rows, float64, 44.3
     // against 47.2 us, 2760 groups and 150,001 rows 1.95 against 2.85 ms)
     const int64_t cap = (int64_t)sm_count() * per_sm;
     if (g > cap) g = g >= 4 * cap ? 4 * cap : cap;
