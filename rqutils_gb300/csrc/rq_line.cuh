@@ -295,8 +295,11 @@ inline int line_lanes_log2(const rq_subspace_t &S, int J, int sms) {
 template <int FM>
 inline bool line_small(int J) { return J * line_key_bytes<FM>() <= 16 * 1024; }
 
-// whether the line filter stays in L2 beside the other tables
-inline bool line_in_l2(const rq_subspace_t &S) { return S.lmap && S.lbits + S.lwbits - 3 <= kLineFilterL2Log2Bytes; }
+// whether there is a line filter (rq_subspace_build fills it for hash lookups only, whatever lmap holds
+// otherwise) and it stays in L2 beside the other tables
+inline bool line_in_l2(const rq_subspace_t &S) {
+    return S.lookup == RQ_LOOKUP_HASH && S.lmap && S.lbits + S.lwbits - 3 <= kLineFilterL2Log2Bytes;
+}
 
 }  // namespace
 }  // namespace rq

@@ -131,3 +131,28 @@ def test_short_rows_equal_matrix_free_bits(D, first, dtype):
     else:
         ref = csr.matvec(x.to(torch.complex128))
         assert torch.linalg.vector_norm(csr.matvec(x) - ref) <= 1e-6 * torch.linalg.vector_norm(ref)
+
+
+def test_binary_search_lists_do_not_read_a_line_filter():
+    """The C interface takes a binary-search subspace whose lmap is set: rq_subspace_build leaves it
+    unfilled and there are no hash arrays, so the lists come from the states alone."""
+    import torch
+    from rqutils_gb300 import _lib as L
+    from rqutils_gb300 import workloads
+    from rqutils_gb300.device import DeviceOperator, DeviceSubspace, DeviceTerms
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    rng = np.random.default_rng(3)
+    ham = PauliSumXZ.from_paulisum(workloads.random_pauli_masks(rng, 12, 80), force_real=True, add_padding=True)
+    S = np.sort(rng.choice(1 << 12, size=700, replace=False)).astype(np.uint64)
+    terms = DeviceTerms(ham)
+    sub = DeviceSubspace(S, num_qubits=12, lookup='bsearch')
+    lmap = torch.zeros(1 << 12, dtype=torch.int32, device='cuda')
+    sub.c.lmap, sub.c.lbits, sub.c.lwbits, sub.c.lshift = L.ptr(lmap), 9, 8, 2
+    for mode in ('conn', 'csr'):
+        got = DeviceOperator(terms, sub, mode=mode)
+        ref = DeviceOperator(terms, DeviceSubspace(S, num_qubits=12), mode=mode)
+        assert ref.nnz > 0
+        for a, b in zip(got.connectivity(), ref.connectivity()):
+            assert np.array_equal(a, b)
+        if mode == 'csr':
+            assert torch.equal(got.val, ref.val)
