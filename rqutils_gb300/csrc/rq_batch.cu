@@ -286,7 +286,7 @@ template <typename V>
 __global__ void __launch_bounds__(kThreads, 4)
 k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y, int *err,
                     const int *gate, int64_t gstride, const int *gate2) {
-    using R = typename VT<V>::R;
+    using RT = RowTerm<V>;
     __shared__ __align__(16) uint32_t htab[kHashTableWords];
     copy_hash_tables(htab, 8);
     __syncthreads();
@@ -296,17 +296,12 @@ k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
         bool act = i < B.D;
         const uint64_t key = act ? __ldg(B.keys + i) : 0ULL;
         act = act && gate_open(gate, gstride, gate2, problem_of(key));
-        CAcc<R> acc;
-        if (act) {
-            const cx<R> xi = VT<V>::ld(x, i);
-            const R dv = (R)B.diag0[i];
-            acc.add({dv * xi.re, dv * xi.im});
-        }
+        typename RT::A acc;
+        if (act) RT::add(acc, RT::scaled((typename VT<V>::R)B.diag0[i], x, i));
         const uint64_t s = key & kStateMask;
-        batch_row_hits(B, htab, act, key, err, [&](int g, int m) {
-            acc.add(cmul(group_diag<R>(B.terms, g, s), VT<V>::ld(x, m)));
-        });
-        if (act) VT<V>::st(y, i, acc.get());
+        batch_row_hits(B, htab, act, key, err,
+                       [&](int g, int m) { RT::add(acc, RT::product(B.terms, g, s, x, m)); });
+        if (act) RT::store(y, i, acc);
     }
 }
 
@@ -326,7 +321,7 @@ struct UseBatchProduct {
     typename RT::A acc;
     __device__ __forceinline__ void start(int64_t i, uint64_t, bool own) {
         acc = typename RT::A();
-        if (own) acc.add(RT::scaled((R)B.diag0[i], x, i));
+        if (own) RT::add(acc, RT::scaled((R)B.diag0[i], x, i));
     }
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t key, int m) {
         if (group_terms(T, g) > kShortTerms) return true;
@@ -336,7 +331,7 @@ struct UseBatchProduct {
     __device__ __forceinline__ void late(WarpWork<V> &W, int q, int g, uint64_t key) {
         W.prod[q] = RT::product(T, g, key & kStateMask, x, W.src[q]);
     }
-    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { acc.add(W.prod[q]); }
+    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { RT::add(acc, W.prod[q]); }
     __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
 };
 
@@ -427,7 +422,7 @@ k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
         // a tile within one problem that is closed is passed over (every thread sees the same)
         const int p0 = problem_of(__ldg(B.keys + r0)), p1 = problem_of(__ldg(B.keys + r0 + nr - 1));
         if (p0 == p1 && !gate_open(gate, gstride, gate2, p0)) continue;
-        tile_product<V>(
+        tile_product<V, RT>(
             B.rowptr, r0, nr, long_groups(B.terms),
             [&](int64_t e) {
                 const int m = __ldg(B.col + e), g = __ldg(B.grp + e);
@@ -436,7 +431,7 @@ k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
                 return RT::product(B.terms, g, (key ^ __ldg(B.terms.xmask + g)) & kStateMask, x, m);
             },
             [&](int64_t e) { return group_terms(B.terms, __ldg(B.grp + e)); },
-            [&](int64_t i, typename RT::A &acc) { acc.add(RT::scaled((R)B.diag0[i], x, i)); },
+            [&](int64_t i, typename RT::A &acc) { RT::add(acc, RT::scaled((R)B.diag0[i], x, i)); },
             [&](int64_t i, const typename RT::A &acc) {
                 if (p0 == p1 || gate_open(gate, gstride, gate2, problem_of(__ldg(B.keys + i)))) RT::store(y, i, acc);
             });
@@ -460,10 +455,10 @@ k_batch_matvec_conn_rows(const rq_batch_t B, const V *__restrict__ x, V *__restr
         if (!gate_open(gate, gstride, gate2, problem_of(key))) continue;
         const uint64_t s = key & kStateMask;
         typename RT::A acc;
-        acc.add(RT::scaled((R)B.diag0[i], x, i));
+        RT::add(acc, RT::scaled((R)B.diag0[i], x, i));
         const int64_t e1 = B.rowptr[i + 1];
         for (int64_t e = B.rowptr[i]; e < e1; ++e)
-            acc.add(RT::product(B.terms, __ldg(B.grp + e), s, x, __ldg(B.col + e)));
+            RT::add(acc, RT::product(B.terms, __ldg(B.grp + e), s, x, __ldg(B.col + e)));
         RT::store(y, i, acc);
     }
 }
@@ -502,7 +497,7 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
             RQ_CUDA(cudaGetLastError());
             return RQ_OK;
         }
-        const int rows = tile_rows<V>(B.D, B.nnz, sm_count());
+        const int rows = tile_rows<RowTerm<V>>(B.D, B.nnz, sm_count());
         const int64_t tiles = (B.D + rows - 1) / rows;
         k_batch_matvec_conn<V><<<(int)std::min<int64_t>(tiles, 0x7FFFFFFF), kThreads, 0, st>>>(
             B, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gstride, gate2);

@@ -26,7 +26,7 @@ struct UseFill {  // (source, group) lists and, CSR, the elements
     int64_t p;
     __device__ __forceinline__ void value(WarpWork<V> &W, int q, int g, uint64_t s) const {
         if constexpr (VT<V>::kComplex) W.prod[q] = group_diag<typename VT<V>::R>(T, g, s);
-        else W.prod[q] = group_diag_re<typename VT<V>::R>(T, g, s);
+        else reinterpret_cast<V &>(W.prod[q]) = group_diag_re<V>(T, g, s);
     }
     __device__ __forceinline__ void start(int64_t i, uint64_t, bool own) { p = own ? rowptr[i] : 0; }
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int) {
@@ -41,7 +41,7 @@ struct UseFill {  // (source, group) lists and, CSR, the elements
         if (grp) grp[p] = g;
         if (val) {
             if constexpr (VT<V>::kComplex) VT<V>::st(val, p, W.prod[q]);
-            else val[p] = W.prod[q];
+            else val[p] = reinterpret_cast<const V &>(W.prod[q]);
         }
         ++p;
     }

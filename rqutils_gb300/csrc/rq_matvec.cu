@@ -181,8 +181,8 @@ struct UseProduct {  // y = H x
         acc = typename RT::A();
         if (!own) return;
         const int skip = op.terms.diag_group;
-        if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[i], x, i));
-        else if (skip >= 0) acc.add(RT::product(op.terms, skip, s, x, i));
+        if (op.diag0 && skip >= 0) RT::add(acc, RT::scaled((R)op.diag0[i], x, i));
+        else if (skip >= 0) RT::add(acc, RT::product(op.terms, skip, s, x, i));
     }
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int m) {
         if (group_terms(op.terms, g) > kShortTerms) return true;
@@ -192,7 +192,7 @@ struct UseProduct {  // y = H x
     __device__ __forceinline__ void late(WarpWork<V> &W, int q, int g, uint64_t s) {
         W.prod[q] = RT::product(op.terms, g, s, x, W.src[q]);
     }
-    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { acc.add(W.prod[q]); }
+    __device__ __forceinline__ void take(const WarpWork<V> &W, int q, int) { RT::add(acc, W.prod[q]); }
     __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
 };
 
@@ -290,8 +290,8 @@ k_matvec_hash(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y
         const K s = (K)s64;
         const uint32_t hs = lin_hash(hk_htab, s64, NB);
         typename RT::A acc;
-        if (op.diag0 && skip >= 0) acc.add(RT::scaled((R)op.diag0[ir], x, ir));
-        else if (skip >= 0) acc.add(RT::product(T, skip, s64, x, ir));
+        if (op.diag0 && skip >= 0) RT::add(acc, RT::scaled((R)op.diag0[ir], x, ir));
+        else if (skip >= 0) RT::add(acc, RT::product(T, skip, s64, x, ir));
         for (int t0 = 0; TL ? t0 < nres : t0 < 1; t0 += TL ? kt : 1) {
             const int tn = TL ? min(kt, nres - t0) : nres;
             if (tiled) {
@@ -357,7 +357,7 @@ k_matvec_hash(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y
                     const uint64_t xv = __ldg(T.xmask + gg);
                     const uint32_t hxg = KB == 32 ? gk32[gc].y : gh64[gc];
                     const int m = lookup_hash_at<KB>(S, s64 ^ xv, (hs ^ hxg) >> shift, err);
-                    if (m >= 0) acc.add(RT::product(T, gg, s64, x, m));
+                    if (m >= 0) RT::add(acc, RT::product(T, gg, s64, x, m));
                 }
                 __syncwarp();
             }
@@ -590,9 +590,12 @@ int grid_tiles(int64_t D, int rows) { return (int)std::min<int64_t>((D + rows - 
 // ------------------------------------------------------------------------------------------
 // CONN and CSR modes
 // ------------------------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ R shfl_product(R v, int src) {
-    return __shfl_sync(0xffffffffu, v, src);
+__device__ __forceinline__ float shfl_product(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ CsrTerm<float>::P shfl_product(CsrTerm<float>::P v, int src) {
+    return {__shfl_sync(0xffffffffu, v.p, src), __shfl_sync(0xffffffffu, v.low, src)};
+}
+__device__ __forceinline__ RowTerm<double>::P shfl_product(RowTerm<double>::P v, int src) {
+    return {__shfl_sync(0xffffffffu, v.d, src), __shfl_sync(0xffffffffu, v.x, src)};
 }
 template <typename R>
 __device__ __forceinline__ cx<R> shfl_product(cx<R> v, int src) {
@@ -608,9 +611,8 @@ __device__ __forceinline__ cx<R> shfl_product(cx<R> v, int src) {
 // against 16.7, complex64 13.7 against 16.7, but complex128 28.7 against 26.9: that one keeps them.
 // elem, first and done as of tile_product.
 constexpr int kShortRows = 2;
-template <typename V, typename E, typename F, typename S>
+template <typename RT, typename E, typename F, typename S>
 __device__ __forceinline__ void short_rows(const int64_t *rowptr, int64_t D, E &&elem, F &&first, S &&done) {
-    using RT = RowTerm<V>;
     constexpr int kR = kShortRows;
     const int lane = threadIdx.x & 31;
     const int64_t b = (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kR);
@@ -634,7 +636,7 @@ __device__ __forceinline__ void short_rows(const int64_t *rowptr, int64_t D, E &
             while (__any_sync(0xffffffffu, e[k] < stop)) {
                 const typename RT::P q = shfl_product(p, (int)(e[k] - c) & 31);
                 if (e[k] < stop) {
-                    acc[k].add(q);
+                    RT::add(acc[k], q);
                     ++e[k];
                 }
             }
@@ -668,15 +670,15 @@ k_matvec_conn(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y
         return RT::product(T, g, __ldg(op.sub.states + m) ^ __ldg(T.xmask + g), x, m);
     };
     auto first = [&](int64_t i, typename RT::A &acc) {
-        if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
-        else if (T.diag_group >= 0) acc.add(RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
+        if (op.diag0) RT::add(acc, RT::scaled((R)op.diag0[i], x, i));
+        else if (T.diag_group >= 0) RT::add(acc, RT::product(T, T.diag_group, __ldg(op.sub.states + i), x, i));
     };
     auto done = [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); };
     if constexpr (SHORT)
-        short_rows<V>(op.rowptr, D, elem, first, done);
+        short_rows<RT>(op.rowptr, D, elem, first, done);
     else
         for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
-            tile_product<V>(
+            tile_product<V, RT>(
                 op.rowptr, r0, (int)min((int64_t)rows, D - r0), long_groups(T), elem,
                 [&](int64_t e) { return group_terms(T, __ldg(op.grp + e)); }, first, done);
 }
@@ -686,7 +688,7 @@ template <typename V, typename VV, bool SHORT>
 __global__ void __launch_bounds__(kThreads)
 k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int rows, const int *gate,
              const int *gate2) {
-    using RT = RowTerm<V>;
+    using RT = CsrTerm<V>;
     using R = typename VT<V>::R;
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     const VV *val = reinterpret_cast<const VV *>(op.val);
@@ -696,35 +698,39 @@ k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y,
         return RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e));
     };
     auto first = [&](int64_t i, typename RT::A &acc) {
-        if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+        if (op.diag0) RT::add(acc, RT::scaled((R)op.diag0[i], x, i));
     };
     auto done = [&](int64_t i, const typename RT::A &acc) { RT::store(y, i, acc); };
     if constexpr (SHORT)
-        short_rows<V>(op.rowptr, D, elem, first, done);
+        short_rows<RT>(op.rowptr, D, elem, first, done);
     else
         for (int64_t r0 = (int64_t)blockIdx.x * rows; r0 < D; r0 += (int64_t)gridDim.x * rows)
-            tile_product<V>(op.rowptr, r0, (int)min((int64_t)rows, D - r0), false, elem, [](int64_t) { return 0; }, first,
+            tile_product<V, RT>(op.rowptr, r0, (int)min((int64_t)rows, D - r0), false, elem, [](int64_t) { return 0; }, first,
                             done);
 }
 
-// A thread per row, for complex128 rows that are long and many (150,001 rows of 83: 750 us against 805
-// with tiles, whose buffer a dozen rows fill).
+// A thread per row, for 64-bit rows that are many: a row's owner adds them one by one either way, and with
+// full warps of owners the FP64 pipe does more a cycle than in tiles.  float64: 400,000 rows of 4 elements
+// 15.2 us against 18.2 with tiles (28.6 with each product rounded before its addition), 700,000 rows of 7
+// 40 against 42; 20,000 rows of 34 44 against 26.  complex128, long rows only (150,001 of 83: 750 us
+// against 805 with tiles, whose buffer a dozen rows fill).
+constexpr int64_t kCsrRowsD = int64_t(1) << 15;
 template <typename V, typename VV>
 __global__ void __launch_bounds__(kThreads)
 k_matvec_csr_rows(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, const int *gate,
                   const int *gate2) {
-    using RT = RowTerm<V>;
+    using RT = CsrTerm<V>;
     using R = typename VT<V>::R;
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     const VV *val = reinterpret_cast<const VV *>(op.val);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < op.sub.D;
          i += (int64_t)gridDim.x * blockDim.x) {
         typename RT::A acc;
-        if (op.diag0) acc.add(RT::scaled((R)op.diag0[i], x, i));
+        if (op.diag0) RT::add(acc, RT::scaled((R)op.diag0[i], x, i));
         const int64_t e1 = op.rowptr[i + 1];
         for (int64_t e = op.rowptr[i]; e < e1; ++e) {
             const auto v = VT<VV>::ld(val, e);
-            acc.add(RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e)));
+            RT::add(acc, RT::times(cx<R>{(R)v.re, (R)v.im}, x, __ldg(op.col + e)));
         }
         RT::store(y, i, acc);
     }
@@ -734,12 +740,13 @@ template <typename V, typename VV>
 void run_csr(const rq_operator_t &op, const V *x, V *y, cudaStream_t st, const int *gate, const int *gate2) {
     const int64_t D = op.sub.D;
     const double avg = (double)op.nnz / (double)D;
-    if (rows_short(D, op.nnz)) {
+    const bool many = std::is_same<V, double>::value && D >= kCsrRowsD;
+    if (rows_short(D, op.nnz) && !many) {
         k_matvec_csr<V, VV, true><<<grid_short(D), kThreads, 0, st>>>(op, x, y, 0, gate, gate2);
-    } else if (sizeof(V) == 16 && avg > 48. && D > 65536) {
+    } else if (many || (sizeof(V) == 16 && avg > 48. && D > 65536)) {
         k_matvec_csr_rows<V, VV><<<grid_rows(D), kThreads, 0, st>>>(op, x, y, gate, gate2);
     } else {
-        const int rows = tile_rows<V>(D, op.nnz, sm_count());
+        const int rows = tile_rows<CsrTerm<V>>(D, op.nnz, sm_count());
         k_matvec_csr<V, VV, false><<<grid_tiles(D, rows), kThreads, 0, st>>>(op, x, y, rows, gate, gate2);
     }
 }
@@ -892,7 +899,7 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
                 k_matvec_conn<V, true><<<grid_short(op.sub.D), kThreads, 0, st>>>(
                     op, static_cast<const V *>(x), static_cast<V *>(y), 0, gate, gate2);
             } else {
-                const int rows = tile_rows<V>(op.sub.D, op.nnz, sm_count());
+                const int rows = tile_rows<RowTerm<V>>(op.sub.D, op.nnz, sm_count());
                 k_matvec_conn<V, false><<<grid_tiles(op.sub.D, rows), kThreads, 0, st>>>(
                     op, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gate2);
             }

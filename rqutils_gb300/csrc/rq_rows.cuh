@@ -2,6 +2,8 @@
 // LOBPCG kernel: the diagonal of one X group on a row, and the tiled cached products.
 #pragma once
 
+#include <type_traits>
+
 #include "rq_common.cuh"
 
 namespace rq {
@@ -82,18 +84,19 @@ __device__ __forceinline__ bool finite_bits(double v) {
     return ((uint32_t)(__double_as_longlong(v) >> 32) & 0x7FF00000u) != 0x7FF00000u;
 }
 
-// One element's contribution to its row and the row's accumulator: a complex value for complex
-// vectors, a real one for real vectors (the product rounded on its own, as cmul's is).  scaled is
-// the diagonal's part; inlined into the first addition, the compiler's fused multiply-add keeps
-// its rounding error in the 32-bit accumulator's compensation, here as in the matrix-free kernel.
+// One element's contribution to its row (P) and the row's accumulator (A).  scaled is the diagonal's
+// part; inlined into the first addition, the compiler's fused multiply-add keeps its rounding error in
+// the 32-bit accumulator's compensation.
 template <typename V, bool CPLX = VT<V>::kComplex>
 struct RowTerm;
 
 template <typename V>
-struct RowTerm<V, true> {
+struct RowTerm<V, true> {  // the complex product
     using R = typename VT<V>::R;
     using P = cx<R>;
     using A = CAcc<R>;
+    static constexpr int kTileBytes = 16 * 1024;  // products of one pass over a tile (below)
+    static constexpr bool kPair = false;          // a product takes two values
     static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const V *x, int64_t m) {
         const cx<R> d = group_diag<R>(T, g, s), v = VT<V>::ld(x, m);
         // a real diagonal times a finite value: the products with zero change nothing
@@ -105,20 +108,68 @@ struct RowTerm<V, true> {
         return {d * v.re, d * v.im};
     }
     static __device__ __forceinline__ P times(cx<R> v, const V *x, int64_t m) { return cmul(v, VT<V>::ld(x, m)); }
+    static __device__ __forceinline__ void add(A &a, P p) { a.add(p); }
     static __device__ __forceinline__ void store(V *y, int64_t i, const A &a) { VT<V>::st(y, i, a.get()); }
 };
 
-template <typename V>
-struct RowTerm<V, false> {
-    using R = typename VT<V>::R;
-    using P = R;
-    using A = Acc<R>;
-    static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const V *x, int64_t m) {
-        return mul_rn(group_diag_re<R>(T, g, s), x[m]);
+template <>
+struct RowTerm<float, false> {  // the product, rounded on its own
+    using P = float;
+    using A = Acc<float>;
+    static constexpr int kTileBytes = 16 * 1024;
+    static constexpr bool kPair = false;
+    static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const float *x, int64_t m) {
+        return mul_rn(group_diag_re<float>(T, g, s), x[m]);
     }
-    static __device__ __forceinline__ P scaled(R d, const V *x, int64_t i) { return d * x[i]; }
-    static __device__ __forceinline__ P times(cx<R> v, const V *x, int64_t m) { return mul_rn(v.re, x[m]); }
-    static __device__ __forceinline__ void store(V *y, int64_t i, const A &a) { y[i] = a.get(); }
+    static __device__ __forceinline__ P scaled(float d, const float *x, int64_t i) { return d * x[i]; }
+    static __device__ __forceinline__ void add(A &a, P p) { a.add(p); }
+    static __device__ __forceinline__ void store(float *y, int64_t i, const A &a) { y[i] = a.get(); }
+};
+
+template <>
+struct RowTerm<double, false> {  // both factors: the row's owner adds their exact product (one FP64 instruction, not two)
+    struct P {
+        double d, x;
+    };
+    using A = Acc<double>;
+    static constexpr int kTileBytes = 16 * 1024;
+    static constexpr bool kPair = true;
+    static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const double *x, int64_t m) {
+        return {group_diag_re<double>(T, g, s), x[m]};
+    }
+    static __device__ __forceinline__ P scaled(double d, const double *x, int64_t i) { return {d, x[i]}; }
+    static __device__ __forceinline__ P times(cx<double> v, const double *x, int64_t m) { return {v.re, x[m]}; }
+    static __device__ __forceinline__ void add(A &a, P p) { a.s = fma(p.d, p.x, a.s); }
+    static __device__ __forceinline__ void store(double *y, int64_t i, const A &a) { y[i] = a.get(); }
+};
+
+// The same for cached elements.  In 32 bits a real product comes with its rounding error, which goes into
+// the accumulator's compensation.
+template <typename V>
+struct CsrTerm : RowTerm<V> {};
+template <>
+struct CsrTerm<double> : RowTerm<double> {
+    static constexpr int kTileBytes = 32 * 1024;  // tiles serve at most 2^15 rows here, which leave room
+};
+template <>
+struct CsrTerm<float> {
+    struct P {
+        float p, low;
+    };
+    using A = Acc<float>;
+    static constexpr int kTileBytes = 16 * 1024;
+    static constexpr bool kPair = true;
+    static __device__ __forceinline__ P of(float d, float x) {
+        const float p = mul_rn(d, x);
+        return {p, fmaf(d, x, -p)};
+    }
+    static __device__ __forceinline__ P scaled(float d, const float *x, int64_t i) { return of(d, x[i]); }
+    static __device__ __forceinline__ P times(cx<float> v, const float *x, int64_t m) { return of(v.re, x[m]); }
+    static __device__ __forceinline__ void add(A &a, P p) {
+        a.add(p.p);
+        a.c += p.low;
+    }
+    static __device__ __forceinline__ void store(float *y, int64_t i, const A &a) { y[i] = a.get(); }
 };
 
 // ------------------------------------------------------------------------------------------
@@ -131,21 +182,27 @@ struct RowTerm<V, false> {
 // threads form the products of the tile's elements (list reads coalesced, every gather in flight
 // at once) into shared memory, then one thread per row adds its row's products from there in list
 // order -- the same additions in the same order, so the results keep their bits.
-constexpr int kTileBytes = 16 * 1024;  // products of one pass over a tile
-constexpr int kTileRows = 256;         // most rows of a tile (one per thread)
-
-template <typename V>
+constexpr int kTileRows = 256;  // most rows of a tile (one per thread)
+template <typename RT>
 __host__ __device__ constexpr int tile_elems() {
-    return kTileBytes / (int)sizeof(typename RowTerm<V>::P);
+    return RT::kTileBytes / (int)sizeof(typename RT::P);
 }
 
 // Rows of a tile: as many as fill the product buffer with average rows, fewer when D is so small
-// that blocks would be idle (half of them while the tiles are fewer than two per SM).
-template <typename V>
+// that blocks would be idle (half of them while the tiles are fewer than two per SM).  Real products that
+// take two values fill the buffer sooner, and where their rows are long (kLongRow elements on average)
+// the dense rows of a sample, which stand together, would keep a few blocks busy with many passes after
+// the others: such tiles fill four fifths and are at least eight per SM (low-energy samples of a
+// 28-qubit molecule, 40,000 rows of 32 elements, float64 CONN 306 us with 64 rows a tile and 122 with 16,
+// float32 CSR 38 and 22 with 32; 24,000 uniform rows of 22, float64 CSR, 12.9 us with 8, 8.9 with 16).
+constexpr double kLongRow = 12.;
+template <typename RT>
 inline int tile_rows(int64_t D, int64_t nnz, int sms) {
-    int r = kTileRows;
     const double avg = (double)nnz / (double)D;
-    while (r > 16 && (r * avg > tile_elems<V>() || (D + r - 1) / r < 2 * sms)) r >>= 1;
+    const bool cut = RT::kPair && avg > kLongRow;
+    const double fill = (cut ? 0.8 : 1.) * tile_elems<RT>();
+    int r = kTileRows;
+    while (r > (cut ? 8 : 16) && (r * avg > fill || (D + r - 1) / r < (cut ? 8 : 2) * sms)) r >>= 1;
     return r;
 }
 
@@ -153,17 +210,19 @@ inline int tile_rows(int64_t D, int64_t nnz, int sms) {
 // precedes the elements of row i, done(i, acc) stores.  All threads of the block call it.  With
 // `split` elements of more than kShortTerms terms (terms(e) of them) wait for a second round, where
 // they stand together: a warp's additions cost what its longest group costs (molecules: 2 to 24
-// terms, most of them 2 or 4; 36 qubits, 150,001 rows, float64: 941 -> 738 us).
+// terms, most of them 2 or 4; 36 qubits, 150,001 rows, float64: 941 -> 738 us).  RT: RowTerm<V>, or
+// CsrTerm<V> for elements without groups.
 constexpr int kShortTerms = 4;
-template <typename V, typename E, typename N, typename F, typename S>
+template <typename V, typename RT, typename E, typename N, typename F, typename S>
 __device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, int nr, bool split, E &&elem,
                                              N &&terms, F &&first, S &&done) {
-    using RT = RowTerm<V>;
-    constexpr int kT = tile_elems<V>();
+    constexpr int kT = tile_elems<RT>();
+    constexpr bool kGroups = std::is_same<RT, RowTerm<V>>::value;
     __shared__ int rp[kTileRows + 1];
-    __shared__ __align__(16) unsigned char buf[kTileBytes];
-    __shared__ uint16_t late[kT];
+    __shared__ __align__(16) unsigned char buf[RT::kTileBytes];
+    __shared__ uint16_t late[kGroups ? kT : 1];
     __shared__ int nlate;
+    if (!kGroups) split = false;
     if (threadIdx.x == 0) nlate = 0;
     typename RT::P *prod = reinterpret_cast<typename RT::P *>(buf);
     const int64_t base = __ldg(rowptr + r0);
@@ -187,7 +246,7 @@ __device__ __forceinline__ void tile_product(const int64_t *rowptr, int64_t r0, 
             __syncthreads();
             if (threadIdx.x == 0) nlate = 0;  // (two barriers before the next pass adds to it)
         }
-        for (int k = max(a - t0, 0); k < min(b - t0, m); ++k) acc.add(prod[k]);
+        for (int k = max(a - t0, 0); k < min(b - t0, m); ++k) RT::add(acc, prod[k]);
         __syncthreads();
     }
     if (own) done(r0 + threadIdx.x, acc);

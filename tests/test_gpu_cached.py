@@ -156,3 +156,36 @@ def test_binary_search_lists_do_not_read_a_line_filter():
             assert np.array_equal(a, b)
         if mode == 'csr':
             assert torch.equal(got.val, ref.val)
+
+
+# rows shorter than one element, tiles of average rows, several passes over the product buffer
+@pytest.mark.parametrize('n,K,D', [(18, 200, 700), (16, 200, 700), (12, 300, 1500), (10, 1500, 300)])
+def test_real_products_are_not_rounded_before_the_sum(n, K, D):
+    """Real products: each element's product enters its row's sum exactly.  In 64 bits that is a fused
+    multiply-add per element in list order, bit for bit; in 32 bits the error of a row of m elements stays
+    within its own rounding plus what compensated sums leave, 2 m (m + 2) 2^-48 of the summed magnitudes
+    (a rounded product alone leaves 2^-25 of itself)."""
+    import torch
+    from fractions import Fraction
+    ops = _operators(n, K, D, True, 7 * n)
+    x = torch.randn(D, dtype=torch.float64, device='cuda', generator=torch.Generator('cuda').manual_seed(D))
+    rowptr, col, _ = ops[2].connectivity()
+    val, diag = ops[2].val.cpu().numpy(), ops[2].diag0.cpu().numpy() if ops[2].diag0 is not None else np.zeros(D)
+    assert (rowptr[-1] < D) == (n == 18)
+    xh = x.cpu().numpy()
+    y = np.zeros(D)
+    for i in range(D):
+        s = Fraction(float(diag[i])) * Fraction(float(xh[i]))
+        for e in range(rowptr[i], rowptr[i + 1]):
+            s = Fraction(float(s)) + Fraction(float(val[e])) * Fraction(float(xh[col[e]]))
+        y[i] = float(s)
+    for op in ops:
+        assert np.array_equal(op.matvec(x).cpu().numpy(), y)
+    x32 = x.float()
+    v32, d32, xf = val.astype(np.float32).astype(float), diag.astype(np.float32).astype(float), x32.cpu().numpy().astype(float)
+    got = ops[2].matvec(x32).cpu().numpy().astype(float)
+    for i in range(D):
+        p = np.append(v32[rowptr[i]:rowptr[i + 1]] * xf[col[rowptr[i]:rowptr[i + 1]]], d32[i] * xf[i])
+        exact = float(sum(map(Fraction, p)))  # (products of 24-bit factors are exact in 64 bits)
+        m = len(p)
+        assert abs(got[i] - exact) <= 2. ** -23 * abs(exact) + 2 * m * (m + 2) * 2. ** -48 * np.abs(p).sum(), i
