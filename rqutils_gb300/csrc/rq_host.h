@@ -59,27 +59,40 @@ inline int64_t *scratch_scan(void *scratch) {
 
 int vtype_size(int32_t vtype);
 
-// Launch settings of one kernel: the dynamic shared memory it has been opted into and its
+// Launch settings of one kernel: whether it has been opted into dynamic shared memory and its
 // occupancy at one shared-memory size.  Each launcher keeps one entry per host thread and device
-// (cache_slot), so threads never share an entry and devices with different SM counts or
-// attributes never see each other's values.
+// (cache_slot), so threads never share an entry and devices with different SM counts never see each
+// other's occupancy.
 struct KernelLaunchCache {
-    size_t configured = 0;
+    bool opted = false;
     size_t occ_smem = ~size_t(0);
     int occ_blocks = 1;
 };
 constexpr int kMaxCachedDevices = 64;
 
-// Opt kern into smem bytes of dynamic shared memory (a kernel with static shared memory can need
-// the opt-in below 48 KB of dynamic memory too) and return its resident blocks per SM at `block`
-// threads, querying the runtime only when `c` does not hold the answer yet (the occupancy query
-// is also reached while a stream is being captured, where only stream work should be issued).
+// Opt kern into all the dynamic shared memory that the current device allows beside its static part.  The
+// runtime keeps one limit per kernel and device for all threads, and a later call can lower it, so every
+// call sets the same one: a thread's launch never depends on what another has asked for since.  (The
+// limit is no allocation; the launch's own size decides the occupancy.)
+template <typename KernT>
+int opt_into_shared(KernT kern, KernelLaunchCache &c) {
+    if (c.opted) return RQ_OK;
+    cudaFuncAttributes a{};
+    int dev = 0, most = 0;
+    RQ_CUDA(cudaFuncGetAttributes(&a, kern));
+    RQ_CUDA(cudaGetDevice(&dev));
+    RQ_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+    c.opted = true;
+    return RQ_OK;
+}
+
+// The same, and kern's resident blocks per SM at `block` threads and smem bytes of dynamic shared memory,
+// querying the runtime only when `c` does not hold the answer yet (the occupancy query is also reached
+// while a stream is being captured, where only stream work should be issued).
 template <typename KernT>
 int configure_kernel(KernT kern, KernelLaunchCache &c, size_t smem, int block, int *per_sm) {
-    if (smem > c.configured) {
-        RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        c.configured = smem;
-    }
+    RQ_TRY(opt_into_shared(kern, c));
     if (c.occ_smem != smem) {
         int per = 0;
         RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));

@@ -1367,10 +1367,7 @@ int launch_persist(const PersistArgs<V> &args, int grid, size_t dyn, cudaStream_
     KernelLaunchCache *c = nullptr;
     RQ_TRY(cache_slot(table, &c));
     auto kern = k_persist<V, FAST>;
-    if (dyn > c->configured) {
-        RQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-        c->configured = dyn;
-    }
+    RQ_TRY(opt_into_shared(kern, *c));
     int per = 0;
     RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPersistThreads, dyn));
     *fits = per >= 1;

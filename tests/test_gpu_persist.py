@@ -57,3 +57,36 @@ def test_persistent_kernel_equals_graph_loop(name, D, cache_level, real, variant
     r = torch.linalg.vector_norm(op.matvec(x1) - e1 * x1)
     if i1['converged']:
         assert r <= 1.01e-9 * abs(e1)
+
+
+@pytest.mark.parametrize('variant', ['fast', 'reference'])
+def test_threads_with_different_sizes(variant):
+    """A thread's large solve and products run after another thread's small ones (the runtime keeps one
+    shared-memory limit per kernel for all threads): large, small on a second thread, large again."""
+    import threading
+    import torch
+    from rqutils_gb300.ground_locg import lobpcg_solve
+    from rqutils_gb300 import workloads
+    from rqutils_gb300.device import DeviceOperator, DeviceSubspace, DeviceTerms
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    large, small = _operator('dense', 8192, (1, 0), False), _operator('dense', 40, (1, 0), False)
+    rng = np.random.default_rng(1)
+    many, few = (PauliSumXZ.from_paulisum(workloads.random_pauli_masks(rng, 16, k, locality=(1, 16)), force_real=True,
+                                          add_padding=True) for k in (6000, 2500))  # both above 2,048 X groups
+    S = np.sort(rng.choice(1 << 16, size=500, replace=False)).astype(np.uint64)
+    free = [DeviceOperator(DeviceTerms(h), DeviceSubspace(S, num_qubits=16), mode='free') for h in (many, few)]
+
+    def run(op, free_op):
+        dt = torch.float64 if op.is_real else torch.complex128
+        x0 = torch.randn(op.D, dtype=dt, device='cuda', generator=torch.Generator('cuda').manual_seed(op.D))
+        x = torch.ones(500, dtype=torch.complex128, device='cuda')
+        return lobpcg_solve(op, x0, variant=variant, maxiter=20)[0], free_op.matvec(x)
+
+    first = run(large, free[0])
+    other = []
+    t = threading.Thread(target=lambda: other.append(run(small, free[1])))
+    t.start()
+    t.join()
+    assert other
+    again = run(large, free[0])
+    assert again[0] == first[0] and torch.equal(again[1], first[1])
