@@ -392,7 +392,10 @@ typedef struct rq_mlp {
     uint16_t *w2tb;       /* [256][256] BF16 copy of W2 transposed                               */
 } rq_mlp_t;
 
-/* Device workspace of rq_mlp_fwd / rq_mlp_bwd for `rows` rows (activations kept for bwd). */
+/* Device workspace of rq_mlp_fwd / rq_mlp_bwd for `rows` rows (activations kept for bwd).  It begins
+ * with two int32 error flags that a kernel sets when a bounded wait runs out, its results being
+ * incomplete: the first is cleared by every rq_mlp_fwd, rq_mlp_infer and rq_mlp_train, the second by no
+ * call, so that a caller who zeroes it once can queue many steps and read it after the last. */
 int rq_mlp_workspace_size(int64_t rows, size_t *bytes);
 /* Refresh the BF16 weight copies from params. */
 int rq_mlp_sync(const rq_mlp_t *m, void *stream);

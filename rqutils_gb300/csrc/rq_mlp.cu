@@ -10,7 +10,7 @@
 // Inference (k_infer) and a training step (k_train, k_wgrad: rq_mlp_train.cuh) have fused kernels.
 //
 // Every mbarrier wait is bounded (about one second of clock cycles); on expiry the kernel records
-// RQ_E_CUDA in the error flag, skips the remaining work, frees its TMEM and returns.
+// RQ_E_CUDA in the error flags, skips the remaining work, frees its TMEM and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -71,6 +71,12 @@ __device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatil
         }
     }
     return true;
+}
+
+// the workspace's two flags (rqsqd.h): of this call, and of all calls
+__device__ __forceinline__ void report_error(int *err) {
+    atomicExch(err, RQ_E_CUDA);
+    atomicExch(err + 1, RQ_E_CUDA);
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
@@ -618,7 +624,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
                 wait_bar(&full[s], (uint32_t)((it / S) & 1), nullptr);
             }
             if (BRES && !bwait_s) wait_bar(&bfull, 0u, nullptr);
-            if (g.err) atomicExch(g.err, RQ_E_CUDA);
+            if (g.err) report_error(g.err);
         }
         if (warp == 1) {
             if (lane == 0) mma_commit(&fin);
@@ -755,7 +761,7 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
     const uint32_t sbase = smem_u32(smem);
     constexpr uint32_t kIdesc = make_idesc(kTileM, kHid);
     if ((sbase & 1023u) != 0u) {
-        if (threadIdx.x == 0) atomicExch(g.err, RQ_E_CUDA);
+        if (threadIdx.x == 0) report_error(g.err);
         return;
     }
     if (threadIdx.x == 0) {
@@ -948,7 +954,7 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
         if (threadIdx.x == 0) {
             if (sh.consumed < sh.issued) wait_bar(&sh.afull, (uint32_t)((sh.issued - 1) & 1), nullptr);
             if (!sh.wwait) wait_bar(&sh.wfull, 0u, nullptr);
-            atomicExch(g.err, RQ_E_CUDA);
+            report_error(g.err);
         }
         if (warp == 1) {
             if (lane == 0) mma_commit(&sh.fin);

@@ -142,7 +142,7 @@ k_train(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sbase = smem_u32(smem);
     if ((sbase & 1023u) != 0u) {
-        if (threadIdx.x == 0) atomicExch(g.err, RQ_E_CUDA);
+        if (threadIdx.x == 0) report_error(g.err);
         return;
     }
     if (threadIdx.x == 0) {
@@ -509,7 +509,7 @@ k_train(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
         if (threadIdx.x == 0) {
             if (sh.consumed < sh.issued) wait_bar(&sh.xfull, (uint32_t)((sh.issued - 1) & 1), nullptr);
             if (!sh.wwait) wait_bar(&sh.wfull, 0u, nullptr);
-            atomicExch(g.err, RQ_E_CUDA);
+            report_error(g.err);
         }
         if (warp == 1) {
             if (lane == 0) mma_commit(&sh.fin);
@@ -701,7 +701,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tma_h1, const __grid_constant__ CUte
         // let the copies and MMAs already issued land before the memory is released
         if (threadIdx.x == 0) {
             for (long long it = consumed_s; it < issued_s; ++it) wait_bar(&full[it % S], (uint32_t)((it / S) & 1), nullptr);
-            atomicExch(g.err, RQ_E_CUDA);
+            report_error(g.err);
         }
         if (warp == 1) {
             if (lane == 0) mma_commit(&fin);

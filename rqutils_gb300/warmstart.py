@@ -71,7 +71,12 @@ class WarmStartMLP:
         n = ctypes.c_size_t()
         L.check(L.lib().rq_mlp_workspace_size(int(rows), ctypes.byref(n)), 'rq_mlp_workspace_size')
         if self._ws is None or self._ws.numel() < n.value:
-            self._ws = torch.empty(int(n.value), dtype=torch.uint8, device=self.device)
+            ws = torch.empty(int(n.value), dtype=torch.uint8, device=self.device)
+            if self._ws is None:
+                ws[:8].zero_()
+            else:
+                ws[:8].copy_(self._ws[:8])  # the error flags
+            self._ws = ws
         return self._ws
 
     def forward(self, x, out=None, stream=None):
@@ -128,9 +133,13 @@ class WarmStartMLP:
                                     float(beta2), float(eps), L.stream_ptr(stream)), 'rq_mlp_step')
 
     def check_errors(self):
+        """Raise if a kernel of any call since the last check reported an error (a wait that ran out:
+        its results, and the steps taken from them, are incomplete)."""
         if self._ws is not None:
-            flag = int(self._ws[:4].view(torch.int32).item())
+            sticky = self._ws[4:8].view(torch.int32)
+            flag = int(sticky.item())
             if flag:
+                sticky.zero_()
                 raise L.RqError(flag, 'an MLP kernel reported an error')
 
     # ------------------------------------------------------------------------------------------
@@ -164,7 +173,8 @@ class WarmStartMLP:
         return logged
 
     def predict(self, states, U, out=None):
-        """Network outputs (D, 2) on every state for one U."""
+        """Network outputs (D, 2) on every state for one U.  Nothing is waited for: check_errors()
+        tells afterwards whether a kernel gave up."""
         dev = self.device
         S = states if isinstance(states, torch.Tensor) else _u64_tensor(states, dev)
         D = S.numel()
@@ -174,7 +184,8 @@ class WarmStartMLP:
         return self.infer(x, out)
 
     def warm_start(self, states, U, dtype=torch.float64):
-        """Start vector sign * exp(log-amplitude) on every state for one U."""
+        """Start vector sign * exp(log-amplitude) on every state for one U (check_errors() as for
+        predict)."""
         out = self.predict(states, U)
         D = out.shape[0]
         x0 = torch.empty(D, dtype=dtype, device=self.device)
@@ -268,6 +279,7 @@ def evaluate_starts(model, S, Us, Lx=4, Ly=4, t=1.0, periodic=True, target_rel=1
                                       variant=variant, mixed=mixed, jacobi=jacobi)
             torch.cuda.synchronize()
             dt = time.perf_counter() - t0
+            model.check_errors()
             ax = op.matvec(x)
             rel = float(torch.linalg.vector_norm(ax - e * x) / abs(e))
             ov = None

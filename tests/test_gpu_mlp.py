@@ -309,3 +309,24 @@ def test_training_step_over_tile_counts(tiles):
     assert torch.equal(m.grads, gb)
     for a, b in [(0, OFF_B1), (OFF_B1, OFF_W2), (OFF_W2, OFF_B2), (OFF_B2, NPARAMS)]:
         assert (gb[a:b] - ga[a:b]).norm().item() < 1e-2 * ga[a:b].norm().item(), (a, b)
+
+
+def test_errors_of_earlier_steps_are_reported():
+    """A flag left by one step (the word that a kernel whose wait ran out sets beside the call's own)
+    outlasts later steps, inference and a larger workspace, and is reported once."""
+    import torch
+    from rqutils_gb300 import _lib as L
+    from rqutils_gb300.warmstart import WarmStartMLP
+    m = WarmStartMLP(seed=1)
+    x = _features(256, 3)
+    tgt = torch.ones((256, 3), device='cuda')
+    m.train_step(x, x.T.contiguous(), tgt)
+    m.check_errors()
+    m.workspace(256)[4:8].view(torch.int32).fill_(L.E_CUDA)
+    m.step(1e-3)
+    m.train_step(x, x.T.contiguous(), tgt)
+    m.infer(x.repeat(9, 1))
+    with pytest.raises(L.RqError):
+        m.check_errors()
+    m.infer(x)
+    m.check_errors()
