@@ -73,6 +73,12 @@ __device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatil
     return true;
 }
 
+// the same for a whole warp, with one answer for its lanes: one that gave up alone would miss the
+// others' next __syncwarp or tcgen05.ld, which wait for all 32
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort) {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort)) != 0;
+}
+
 // the workspace's two flags (rqsqd.h): of this call, and of all calls
 __device__ __forceinline__ void report_error(int *err) {
     atomicExch(err, RQ_E_CUDA);
@@ -530,7 +536,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
         for (int64_t u = blockIdx.x; u < units && !bad; u += gridDim.x) {
             for (int64_t c = 0; c < g.nchunks; ++c, ++it) {
                 const int s = (int)(it % S);
-                if (it >= S && !wait_bar(&empty[s], (uint32_t)((it / S - 1) & 1), abort_p)) {
+                if (it >= S && !warp_wait(&empty[s], (uint32_t)((it / S - 1) & 1), abort_p)) {
                     bad = true;
                     break;
                 }
@@ -545,17 +551,17 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
             }
         }
     } else if (warp == 1) {  // ---- MMA issuer
-        bool bad = BRES && !wait_bar(&bfull, 0u, abort_p);
+        bool bad = BRES && !warp_wait(&bfull, 0u, abort_p);
         if (BRES && !bad && lane == 0) bwait_s = 1;
         long long it = 0, t = 0;
         for (int64_t u = blockIdx.x; u < units && !bad; u += gridDim.x, ++t) {
             const int b = (int)(t & 1);
-            if (t >= 2 && !wait_bar(&tempty[b], (uint32_t)((t / 2 - 1) & 1), abort_p)) break;
+            if (t >= 2 && !warp_wait(&tempty[b], (uint32_t)((t / 2 - 1) & 1), abort_p)) break;
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)(b * N);
             for (int64_t c = 0; c < g.nchunks; ++c, ++it) {
                 const int s = (int)(it % S);
-                if (!wait_bar(&full[s], (uint32_t)((it / S) & 1), abort_p)) {
+                if (!warp_wait(&full[s], (uint32_t)((it / S) & 1), abort_p)) {
                     bad = true;
                     break;
                 }
@@ -594,7 +600,7 @@ k_gemm(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtens
         long long t = 0;
         for (int64_t u = blockIdx.x; u < units; u += gridDim.x, ++t) {
             const int b = (int)(t & 1);
-            const bool ok = wait_bar(&tfull[b], (uint32_t)((t >> 1) & 1), abort_p);
+            const bool ok = warp_wait(&tfull[b], (uint32_t)((t >> 1) & 1), abort_p);
             if (named_bar_or(kEpiBar, kEpiThreads, !ok || *abort_p != 0)) {  // the same answer in every epilogue thread
                 broke = true;
                 break;
@@ -796,7 +802,7 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
         }
         int64_t it = 0;
         for (int64_t u = blockIdx.x; u < g.tiles; u += gridDim.x, ++it) {
-            if (it >= 1 && !wait_bar(&sh.aempty, (uint32_t)((it - 1) & 1), abort_p)) break;
+            if (it >= 1 && !warp_wait(&sh.aempty, (uint32_t)((it - 1) & 1), abort_p)) break;
             if (lane == 0) {
                 mbar_expect_tx(&sh.afull, kTileABytes);
                 tma_load_2d(sbase + kInfA, &tma_x, 0, (int)(u * kTileM), &sh.afull);
@@ -805,12 +811,12 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
             __syncwarp();
         }
     } else if (warp == 1) {  // ---- MMA issuer
-        bool ok = wait_bar(&sh.wfull, 0u, abort_p);
+        bool ok = warp_wait(&sh.wfull, 0u, abort_p);
         if (ok && lane == 0) sh.wwait = 1;
         int64_t it = 0, hq = 0;
         for (int64_t u = blockIdx.x; u < g.tiles && ok; u += gridDim.x, ++it) {
-            ok = wait_bar(&sh.afull, (uint32_t)(it & 1), abort_p) &&
-                 (it < 1 || wait_bar(&sh.d1empty, (uint32_t)((it - 1) & 1), abort_p));
+            ok = warp_wait(&sh.afull, (uint32_t)(it & 1), abort_p) &&
+                 (it < 1 || warp_wait(&sh.d1empty, (uint32_t)((it - 1) & 1), abort_p));
             if (!ok) break;
             tc_fence_after();
             if (lane == 0) {
@@ -823,10 +829,10 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
                 sh.consumed = it + 1;
             }
             __syncwarp();
-            if (it >= 1 && !wait_bar(&sh.d2empty, (uint32_t)((it - 1) & 1), abort_p)) break;
+            if (it >= 1 && !warp_wait(&sh.d2empty, (uint32_t)((it - 1) & 1), abort_p)) break;
             for (int q = 0; q < 4; ++q, ++hq) {
                 const int s = (int)(hq & 1);
-                ok = wait_bar(&sh.hfull[s], (uint32_t)((hq >> 1) & 1), abort_p);
+                ok = warp_wait(&sh.hfull[s], (uint32_t)((hq >> 1) & 1), abort_p);
                 if (!ok) break;
                 tc_fence_after();
                 if (lane == 0) {
@@ -854,12 +860,12 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
         named_bar_sync(kEpiBar, kThreadsE);
         int64_t it = 0, hq = 0;
         for (int64_t u = blockIdx.x; u < g.tiles; u += gridDim.x, ++it) {
+            // a wait that gives up changes nothing until the vote below, when the tile is dropped: lanes that
+            // left the path alone would miss what waits for all 32 of them
             bool ok = wait_bar(&sh.d1full, (uint32_t)(it & 1), abort_p);
             tc_fence_after();
             for (int q = 0; q < 4; ++q, ++hq) {  // H1 quarter by quarter; this warp's 16 columns of it
                 const int s = (int)(hq & 1);
-                ok = ok && (hq < 2 || wait_bar(&sh.hempty[s], (uint32_t)(((hq >> 1) - 1) & 1), abort_p));
-                if (!ok) continue;
                 const int c0 = 64 * q + 16 * cq;
                 float z[16];
                 tmem_ld16(lanes + (uint32_t)c0, z);
@@ -877,6 +883,7 @@ k_infer(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
                 }
                 // 16-byte chunk c of row r sits at chunk c ^ (r mod 8) of the row's 128 bytes
                 unsigned char *dst = smem + kInfH + kTileABytes * (uint32_t)s + row * 128;
+                if (hq >= 2 && !wait_bar(&sh.hempty[s], (uint32_t)(((hq >> 1) - 1) & 1), abort_p)) ok = false;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
                     *reinterpret_cast<uint4 *>(dst + (((2 * cq + j) ^ (row & 7)) << 4)) = reinterpret_cast<const uint4 *>(o)[j];

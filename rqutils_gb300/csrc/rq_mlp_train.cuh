@@ -162,9 +162,7 @@ k_train(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUten
     tc_fence_after();
     const uint32_t tmem = sh.tmem;
     volatile int *abort_p = &sh.abort;
-    auto wait = [&](uint64_t *bar, uint32_t parity) {  // the same answer in every lane
-        return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_p)) != 0;
-    };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return warp_wait(bar, parity, abort_p); };
     // every barrier completes once per tile: phase it & 1 of the CTA's tile `it`
 
     if (warp == 0) {  // ---- TMA: X in, H1, dZ2 and dZ1 out
@@ -608,9 +606,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tma_h1, const __grid_constant__ CUte
         c0 = sp * g.chunks / n;
         c1 = (sp + 1) * g.chunks / n;
     };
-    auto wait = [&](uint64_t *bar, uint32_t parity) {  // the same answer in every lane
-        return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_p)) != 0;
-    };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return warp_wait(bar, parity, abort_p); };
 
     if (warp == 0) {  // ---- TMA producer
         long long it = 0;
