@@ -57,8 +57,10 @@ __device__ __forceinline__ bool sector_pass(K t, K fa, K fbm, int pa0, int pb0) 
 //   and FP64 instructions, which cost a warp the same however few lanes are active, run full;
 //   groups of more than kShortTerms terms go to a second queue, so that short ones do not wait;
 // * the owner lane of a row adds its products from the queue in group order, as the cached products do.
-// Hubbard 4x4, complex64, against a loop of each lane over its own hits (48 warps per SM instead of
-// 32): 2^20 rows 75 us against 78, 2^18 low-energy rows 47 against 59.
+// Hubbard 4x4, complex64, against a loop of each lane over its own hits: 2^20 rows 75 us against 78, 2^18
+// low-energy rows 47 against 59.
+// QUEUE = false: that loop (own_hits).  It needs fewer registers (48 warps per SM instead of 32), and where
+// every lane has about as many hits as its neighbours no lane waits for another.
 constexpr int kQueueSlots = 128;  // hits resolved together
 
 template <typename V>
@@ -80,8 +82,8 @@ __host__ __device__ constexpr size_t line_key_bytes() { return FM != kFiltNone ?
 // molecule above), and the entries past the last group
 constexpr int kPart = 64;
 
-template <typename V, int BLOCK>
-__host__ __device__ constexpr size_t line_work_bytes() { return (BLOCK / 32) * sizeof(WarpWork<V>); }
+template <typename V, int BLOCK, bool QUEUE = true>
+__host__ __device__ constexpr size_t line_work_bytes() { return QUEUE ? (BLOCK / 32) * sizeof(WarpWork<V>) : 0; }
 
 constexpr size_t kLineSmem = 216 * 1024;  // shared memory of a block with many groups (one per SM)
 template <typename V, int FM, int BLOCK>
@@ -101,20 +103,21 @@ __device__ __forceinline__ uint32_t line_word(uint32_t h, uint32_t hpre, const r
 // sees for each row: start(i, s, own) -- own: the lane that sums the row -- then for each hit
 // resolve(W, q, g, s, m) on some lane of the warp (queue slot q, group g, row state s, source m;
 // true: call late() for it in the second round), take(W, q, g) on the owner in list order, and
-// finish(i).  A warp takes the 32 >> lw rows from `first` + a multiple of `stride` while some row of
-// the block's turn lies below `end`; the caller has filled hk_htab (and hk_fb), and every thread of
-// the block calls.
-template <typename V, int KB, int FM, int BLOCK, typename C>
+// finish(i).  Without a queue: hit(g, s, m) on the owner.  A warp takes the 32 >> lw rows from
+// `first` + a multiple of `stride` while some row of the block's turn lies below `end`; the caller
+// has filled hk_htab (and hk_fb), and every thread of the block calls.
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE = true, typename C>
 __device__ __forceinline__ void line_rows(const rq_subspace_t &S, const rq_terms_t &T, int *err, int lw, int kt,
                                           int64_t first, int64_t turn, int64_t stride, int64_t end, C &use) {
     using K = typename KeyWidth<KB>::K;
     constexpr int NB = KeyWidth<KB>::kNbytes;
-    constexpr int U = FM != kFiltNone ? 8 : 16;  // probes in flight per lane: what 64 registers hold
+    // probes in flight per lane: what 64 (QUEUE) and 40 registers hold
+    constexpr int U = FM != kFiltNone ? 8 : QUEUE ? 16 : KB == 32 ? 32 : 8;
     const int skip = T.diag_group;
     const int nres = T.J - (skip >= 0 ? 1 : 0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WarpWork<V> &W = reinterpret_cast<WarpWork<V> *>(hk_dyn)[warp];
-    uint2 *gk = reinterpret_cast<uint2 *>(hk_dyn + line_work_bytes<V, BLOCK>());  // [kt + kPart]
+    WarpWork<V> &W = reinterpret_cast<WarpWork<V> *>(hk_dyn)[QUEUE ? warp : 0];
+    uint2 *gk = reinterpret_cast<uint2 *>(hk_dyn + line_work_bytes<V, BLOCK, QUEUE>());  // [kt + kPart]
     uint64_t *gx = reinterpret_cast<uint64_t *>(gk + kt + kPart);                       // the same, FM only
     auto load_keys = [&](int c0, int n) {
         for (int c = threadIdx.x; c < n + kPart; c += blockDim.x) {
@@ -179,6 +182,16 @@ __device__ __forceinline__ void line_rows(const rq_subspace_t &S, const rq_terms
                     hot |= (uint64_t)hb << k0;
                 }
                 hot &= en >= 64 ? ~0ULL : (1ULL << en) - 1ULL;
+                if constexpr (!QUEUE) {
+                    while (hot) {
+                        const int e = e0 + __ffsll((long long)hot) - 1, c = t0 + e, gg = c + (skip >= 0 && c >= skip);
+                        hot &= hot - 1ULL;
+                        const int m = lookup_hash_at<KB>(S, s64 ^ __ldg(T.xmask + gg), (hs ^ gk[e].x) >> shift, err);
+                        if (m >= 0) use.hit(gg, s64, m);
+                    }
+                    __syncwarp();  // re-converge before the next probes
+                    continue;
+                }
                 // resolve the hits of the warp, kQueueSlots at a time
                 const int cnt = __popcll(hot);
                 int incl = cnt;
@@ -248,7 +261,7 @@ __device__ __forceinline__ void line_rows(const rq_subspace_t &S, const rq_terms
 
 // The tables and the calling warp's place for a kernel that walks the whole subspace: neighbouring
 // tiles of 32 >> lw rows to the same block, or (spread) to different SMs.
-template <typename V, int KB, int FM, int BLOCK, typename C>
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE = true, typename C>
 __device__ __forceinline__ void line_subspace(const rq_operator_t &op, int *err, int lw, int kt, int spread, C &use) {
     copy_hash_tables(hk_htab, KeyWidth<KB>::kNbytes);
     if (FM == kFiltSet)
@@ -257,7 +270,7 @@ __device__ __forceinline__ void line_subspace(const rq_operator_t &op, int *err,
     const int64_t rows = 32 >> lw, stride = (int64_t)gridDim.x * (BLOCK / 32) * rows;
     const int64_t first =
         (spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * (BLOCK / 32) + warp) * rows;
-    line_rows<V, KB, FM, BLOCK>(op.sub, op.terms, err, lw, kt, first, 0, stride, op.sub.D, use);
+    line_rows<V, KB, FM, BLOCK, QUEUE>(op.sub, op.terms, err, lw, kt, first, 0, stride, op.sub.D, use);
 }
 
 // ---- launch rules -----------------------------------------------------------------------------
@@ -294,6 +307,17 @@ inline int line_lanes_log2(const rq_subspace_t &S, int J, int sms) {
 // in tiles above what fits) one 1024-thread block
 template <int FM>
 inline bool line_small(int J) { return J * line_key_bytes<FM>() <= 16 * 1024; }
+
+// Whether the lanes resolve their own hits, in 32-bit arithmetic: dense subspaces with more rows than are
+// resident with the queue.  Their rows have many hits each, and about as many as their neighbours.  The
+// prefix shift tells them, as above: shift b is about 2^(lwbits - 5) states among 2^b neighbours.  complex64,
+// queue against own hits: 20 qubits, 157,000 rows (shift 5) 131 us against 86; 23 qubits, 676,000 rows
+// (6) 514 against 435; 24 qubits, 500,000 rows (7) 126 against 121, 250,000 (8) 50 against 54; 32 qubits,
+// 400,000 low-energy rows (13) 69 against 92; 21 qubits, 120,000 rows, all resident, 51 against 53.
+constexpr int kOwnHitsShift = 7;  // for lines of 2^8 bits
+inline bool own_hits(const rq_subspace_t &S, int J, int sms) {
+    return S.D > (int64_t)sms * kLineThreads && S.lshift <= kOwnHitsShift + S.lwbits - 8 && line_small<kFiltNone>(J);
+}
 
 // whether there is a line filter (rq_subspace_build fills it for hash lookups only, whatever lmap holds
 // otherwise) and it stays in L2 beside the other tables

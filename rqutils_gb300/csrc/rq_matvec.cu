@@ -184,6 +184,7 @@ struct UseProduct {  // y = H x
         if (op.diag0 && skip >= 0) RT::add(acc, RT::scaled((R)op.diag0[i], x, i));
         else if (skip >= 0) RT::add(acc, RT::product(op.terms, skip, s, x, i));
     }
+    __device__ __forceinline__ void hit(int g, uint64_t s, int m) { RT::add(acc, RT::product(op.terms, g, s, x, m)); }
     __device__ __forceinline__ bool resolve(WarpWork<V> &W, int q, int g, uint64_t s, int m) {
         if (group_terms(op.terms, g) > kShortTerms) return true;
         W.prod[q] = RT::product(op.terms, g, s, x, m);
@@ -196,13 +197,13 @@ struct UseProduct {  // y = H x
     __device__ __forceinline__ void finish(int64_t i) { RT::store(y, i, acc); }
 };
 
-template <typename V, int KB, int FM, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : 4)
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
+__global__ void __launch_bounds__(BLOCK, BLOCK == 1024 ? 1 : QUEUE ? 4 : 6)
 k_matvec_line(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y, int *err, int lw, int kt,
               int spread, const int *gate, const int *gate2) {
     if (gate && (*gate == 0 || (gate2 && *gate2 == 0))) return;
     UseProduct<V> use{op, x, y, {}};
-    line_subspace<V, KB, FM, BLOCK>(op, err, lw, kt, spread, use);
+    line_subspace<V, KB, FM, BLOCK, QUEUE>(op, err, lw, kt, spread, use);
 }
 
 // ---- probes of the key buckets ----------------------------------------------------------------
@@ -796,15 +797,15 @@ int launch_hash_block(const rq_operator_t &op, const void *x, void *y, int *err,
     return RQ_OK;
 }
 
-template <typename V, int KB, int FM, int BLOCK>
+template <typename V, int KB, int FM, int BLOCK, bool QUEUE>
 int launch_line_block(const rq_operator_t &op, int lw, const void *x, void *y, int *err, cudaStream_t st,
                       const int *gate, const int *gate2) {
-    auto kern = k_matvec_line<V, KB, FM, BLOCK>;
+    auto kern = k_matvec_line<V, KB, FM, BLOCK, QUEUE>;
     const int nres = op.terms.J - (op.terms.diag_group >= 0 ? 1 : 0);
     constexpr int kMaxTile = line_tile_groups<V, FM, BLOCK>();
     static_assert(kMaxTile <= 65536, "a queue entry holds 16 bits of group");
     const int kt = nres < kMaxTile ? std::max(nres, 1) : kMaxTile;
-    const size_t smem = line_work_bytes<V, BLOCK>() + (size_t)(kt + kPart) * line_key_bytes<FM>();
+    const size_t smem = line_work_bytes<V, BLOCK, QUEUE>() + (size_t)(kt + kPart) * line_key_bytes<FM>();
     thread_local KernelLaunchCache table[kMaxCachedDevices];
     KernelLaunchCache *c = nullptr;
     int per_sm = 1;
@@ -831,9 +832,12 @@ int launch_hash(const rq_operator_t &op, const void *x, void *y, int *err, cudaS
     // fits): one 1024-thread block
     if (op.sub.lmap) {
         const int lw = line_lanes_log2(op.sub, op.terms.J, sm_count());
+        if constexpr (KB == 32 && FM == kFiltNone && sizeof(typename VT<V>::R) == 4)
+            if (lw == 0 && own_hits(op.sub, op.terms.J, sm_count()))
+                return launch_line_block<V, KB, FM, 256, false>(op, lw, x, y, err, st, gate, gate2);
         return line_small<FM>(op.terms.J)
-                   ? launch_line_block<V, KB, FM, 256>(op, lw, x, y, err, st, gate, gate2)
-                   : launch_line_block<V, KB, FM, 1024>(op, lw, x, y, err, st, gate, gate2);
+                   ? launch_line_block<V, KB, FM, 256, true>(op, lw, x, y, err, st, gate, gate2)
+                   : launch_line_block<V, KB, FM, 1024, true>(op, lw, x, y, err, st, gate, gate2);
     }
     const bool small = op.terms.J <= max_resident_groups<KB>() &&
                        group_key_bytes<KB>(op.terms.J) <= 16 * 1024;

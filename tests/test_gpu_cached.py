@@ -189,3 +189,34 @@ def test_real_products_are_not_rounded_before_the_sum(n, K, D):
         exact = float(sum(map(Fraction, p)))  # (products of 24-bit factors are exact in 64 bits)
         m = len(p)
         assert abs(got[i] - exact) <= 2. ** -23 * abs(exact) + 2 * m * (m + 2) * 2. ** -48 * np.abs(p).sum(), i
+
+
+# one row more than the queue's resident rows and fewer, most of a space and all of it; groups around the
+# 64 that a lane probes between two resolutions
+@pytest.mark.parametrize('D', [155648, 155649, 262144])
+@pytest.mark.parametrize('groups', [63, 64, 65, 129])
+@pytest.mark.parametrize('dtype', ['float32', 'complex64'])
+def test_dense_subspaces_equal_bits(D, groups, dtype):
+    """Dense subspaces, whose lanes resolve their own hits, against the product without a line filter."""
+    import torch
+    from rqutils_gb300.device import DeviceOperator, DeviceSubspace, DeviceTerms
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    rng = np.random.default_rng(groups)
+    masks = rng.choice(np.arange(1, 1 << 18), size=groups, replace=False)
+    labels, coeffs = ['I' * 18, 'Z' * 18], [0.3, 0.7]
+    for m in masks:
+        x = ''.join('X' if m >> (17 - k) & 1 else 'I' for k in range(18))
+        z = ''.join('Z' if c == 'I' and rng.random() < 0.5 else c for c in x)
+        labels += [x, z] if x != z else [x]
+        coeffs += list(rng.normal(size=2 if x != z else 1))
+    if dtype == 'complex64':  # an odd number of Y: a term with an imaginary part
+        labels = [s.replace('X', 'Y', 1) if k % 3 == 2 else s for k, s in enumerate(labels)]
+    ham = PauliSumXZ.from_paulisum((labels, np.array(coeffs)), force_real=True, add_padding=True)
+    S = np.sort(rng.choice(1 << 18, size=D, replace=False)).astype(np.uint64)
+    terms, sub = DeviceTerms(ham), DeviceSubspace(S, num_qubits=18)
+    assert terms.J == groups + 1 and sub.c.lshift <= 7
+    x = torch.randn(D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(D))
+    y = DeviceOperator(terms, DeviceSubspace(S, num_qubits=18, line_filter=False), mode='free').matvec(x)
+    op = DeviceOperator(terms, sub, mode='free')
+    assert torch.equal(op.matvec(x), y)
+    op.check_errors()
