@@ -471,15 +471,23 @@ int scan_row_counts(int64_t *rowptr_plus1, int64_t D, int64_t *bsum, cudaStream_
 template <typename V>
 int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cudaStream_t st,
                        const int *gate, int64_t gstride, const int *gate2) {
-    if (B.mode == RQ_MODE_FREE && B.lmap) {
+    // lanes per row (log2): the most with which all rows are resident at once
+    int lw = 0;
+    while (lw < 5 && B.D << (lw + 1) <= (int64_t)sm_count() * kLineThreads) ++lw;
+    // A tile of more than kTileProblems problems on average goes row by row, a thread each, as without a
+    // line filter: problem by problem most of a block's lanes would have no row, and every problem costs
+    // two barriers and a load of its group keys (complex64, 100,000 rows: problems of 20 rows 58 us against
+    // 30, of 50 37 against 30, of 80 27 against 32).
+    constexpr int kTileProblems = 4;
+    const bool small_problems = (int64_t)(kThreads >> lw) * B.P > kTileProblems * B.D;
+    if (B.mode == RQ_MODE_FREE && B.lmap && !small_problems) {
         auto kern = k_batch_matvec_line<V>;
         const size_t smem = line_work_bytes<V, kThreads>() + (kBatchLineGroups + kPart) * line_key_bytes<kFiltNone>();
         thread_local KernelLaunchCache table[kMaxCachedDevices];
         KernelLaunchCache *c = nullptr;
-        int per_sm = 1, lw = 0;
+        int per_sm = 1;
         RQ_TRY(cache_slot(table, &c));
         RQ_TRY(configure_kernel(kern, *c, smem, kThreads, &per_sm));
-        while (lw < 5 && B.D << (lw + 1) <= (int64_t)sm_count() * kLineThreads) ++lw;
         const int64_t tiles = (B.D + (kThreads >> lw) - 1) / (kThreads >> lw);
         // four times the resident blocks: a block that ends early makes room (2.0 M rows in 40 problems,
         // complex64: 607 us with one walk per resident block, 547 with four)

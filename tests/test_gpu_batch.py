@@ -273,3 +273,29 @@ def test_batch_products_agree_bit_for_bit(seed, P, d_range, dtype):
         b.check_errors()
     line.check_errors()
     assert (line.D > 2 ** 20) == (P == 30)
+
+
+@pytest.mark.parametrize('dtype', ['float32', 'float64', 'complex64', 'complex128'])
+@pytest.mark.parametrize('P,rows', [(1, 3), (700, 1), (2000, 6), (2600, 60), (2400, 64), (2300, 70)])
+def test_batches_of_small_problems_agree_bit_for_bit(P, rows, dtype):
+    """Many problems of a few rows (a thread per row behind the line filter) up to where tiles of few problems
+    begin: the same bits with and without the filter."""
+    import torch
+    from rqutils_gb300.batch import BatchedSQD
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    from rqutils_gb300.workloads import random_pauli_masks
+    rng = np.random.default_rng(P + rows)
+    hams = []
+    for _ in range(8):
+        labels, coeffs = random_pauli_masks(rng, 9, 80)
+        if dtype.startswith('float'):
+            labels = [s if s.count('Y') % 2 == 0 else s.replace('Y', 'X') for s in labels]
+        hams.append(PauliSumXZ.from_paulisum((labels, coeffs), force_real=True, add_padding=True))
+    hams = [hams[p % 8] for p in range(P)]
+    states = [np.sort(rng.choice(512, size=rows, replace=False)).astype(np.uint64) for _ in range(P)]
+    line = BatchedSQD(hams, states)
+    x = torch.randn(line.D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(P))
+    y = line.matvec(x)
+    plain = BatchedSQD(hams, states, line_filter=False, presence=False)
+    assert torch.equal(plain.matvec(x), y)
+    line.check_errors()
