@@ -480,7 +480,9 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
     // 30, of 50 37 against 30, of 80 27 against 32).
     constexpr int kTileProblems = 4;
     const bool small_problems = (int64_t)(kThreads >> lw) * B.P > kTileProblems * B.D;
-    if (B.mode == RQ_MODE_FREE && B.lmap && !small_problems) {
+    // (line_rows computes a filter word's index in 32 bits; rq_batch_build takes larger filters too)
+    const bool narrow = B.lbits + B.lwbits <= 37;
+    if (B.mode == RQ_MODE_FREE && B.lmap && narrow && !small_problems) {
         auto kern = k_batch_matvec_line<V>;
         const size_t smem = line_work_bytes<V, kThreads>() + (kBatchLineGroups + kPart) * line_key_bytes<kFiltNone>();
         thread_local KernelLaunchCache table[kMaxCachedDevices];

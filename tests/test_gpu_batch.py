@@ -299,3 +299,23 @@ def test_batches_of_small_problems_agree_bit_for_bit(P, rows, dtype):
     plain = BatchedSQD(hams, states, line_filter=False, presence=False)
     assert torch.equal(plain.matvec(x), y)
     line.check_errors()
+
+
+def test_batch_line_filter_beyond_32_bit_word_indices():
+    """rq_batch_build takes line filters of more than 2^32 words (lbits + lwbits > 37: 32 GB here): every
+    hit is found."""
+    import ctypes
+    import torch
+    from rqutils_gb300 import _lib as L
+    from rqutils_gb300.batch import BatchedSQD
+    hams, states, ns = _random_problems(51, 4, n_range=(12, 12), d_range=(2000, 3000))
+    b = BatchedSQD(hams, states)
+    x = torch.randn(b.D, dtype=torch.complex128, device='cuda', generator=torch.Generator('cuda').manual_seed(1))
+    y = b.matvec(x)
+    lmap = torch.empty(1 << 33, dtype=torch.int32, device='cuda')
+    b.c.lmap, b.c.lbits, b.c.lwbits = L.ptr(lmap), 28, 10
+    L.check(L.lib().rq_batch_build(ctypes.byref(b.c), L.ptr(b.scratch), L.stream_ptr()), 'rq_batch_build')
+    assert torch.equal(b.matvec(x), y)
+    b.check_errors()
+    del lmap
+    torch.cuda.empty_cache()
