@@ -438,11 +438,33 @@ k_batch_matvec_conn(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
     }
 }
 
-// A thread per row, for 32-bit values and more than kConnRowsD rows: 2.03 M rows of 40 problems,
-// complex64: 134 us against 181 with tiles, whose height fits the average problem and not the few with
-// long rows (780,729 rows of 48 problems: 20.8 against 21.1; complex128 wants tiles at any size: its
-// additions are what counts, 262 us against 351).
-constexpr int64_t kConnRowsD = int64_t(1) << 20;
+// A thread per row, for 32-bit values where tiles cost more than they gain (complex64, against tiles):
+// * rows that stream from HBM (2.03 M rows of 40 problems: 134 us against 181), from 2^19 rows on where
+//   they have less than an element on average and differ between large problems (780,729 rows of 48
+//   problems, 0.35 elements: 17.2 against 18.4);
+// * problems of a few rows and elements (100,000 rows of 5,000 problems: 4.7 against 5.4).
+// (complex128 wants tiles at any size: its additions are what counts, 262 us against 351.)
+inline bool batch_conn_rows(const rq_batch_t &B) {
+    return B.D > (int64_t(1) << 20) || B.D < 64 * (int64_t)B.P ||
+           (B.D > (int64_t(1) << 19) && B.nnz < B.D && B.D >= 4096 * (int64_t)B.P);
+}
+
+// Rows of a tile of 32-bit values.  Problems differ in their rows' lengths; where they are large, the tiles
+// of a dense problem stand together and keep their blocks busy after the others, so tiles are at most 128
+// rows and three eighths of a full buffer, and at least four per SM (complex64: 16 problems, 195,270 rows of
+// 4 elements 52 us with 256 rows, 32 with 128; 40 problems, 592,748 rows of 8 176 with 256, 117 with 64; a
+// thread per row 45 and 123).  Small problems even out: 2,000 of 300 rows 14 us with 256, 20 with 128.
+constexpr int64_t kLargeProblem = 2048;
+template <typename V>
+inline int batch_tile_rows(const rq_batch_t &B, int sms) {
+    using RT = RowTerm<V>;
+    if (sizeof(typename VT<V>::R) == 8 || B.D < kLargeProblem * B.P) return tile_rows<RT>(B.D, B.nnz, sms);
+    const double avg = (double)B.nnz / (double)B.D;
+    int r = kTileRows / 2;
+    while (r > 16 && (r * avg > 0.375 * tile_elems<RT>() || (B.D + r - 1) / r < 4 * sms)) r >>= 1;
+    return r;
+}
+
 template <typename V>
 __global__ void __launch_bounds__(kThreads)
 k_batch_matvec_conn_rows(const rq_batch_t B, const V *__restrict__ x, V *__restrict__ y,
@@ -501,13 +523,13 @@ int batch_matvec_typed(const rq_batch_t &B, const void *x, void *y, int *err, cu
     } else if (B.mode == RQ_MODE_CONN) {
         if (!B.rowptr || (B.nnz > 0 && (!B.col || !B.grp)))
             return fail(RQ_E_ARG, "rq_batch_matvec: RQ_MODE_CONN needs rowptr, col and grp");
-        if (sizeof(typename VT<V>::R) == 4 && B.D > kConnRowsD) {
+        if (sizeof(typename VT<V>::R) == 4 && batch_conn_rows(B)) {
             k_batch_matvec_conn_rows<V><<<grid_rows(B.D), kThreads, 0, st>>>(
                 B, static_cast<const V *>(x), static_cast<V *>(y), gate, gstride, gate2);
             RQ_CUDA(cudaGetLastError());
             return RQ_OK;
         }
-        const int rows = tile_rows<RowTerm<V>>(B.D, B.nnz, sm_count());
+        const int rows = batch_tile_rows<V>(B, sm_count());
         const int64_t tiles = (B.D + rows - 1) / rows;
         k_batch_matvec_conn<V><<<(int)std::min<int64_t>(tiles, 0x7FFFFFFF), kThreads, 0, st>>>(
             B, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gstride, gate2);

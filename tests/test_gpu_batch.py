@@ -319,3 +319,27 @@ def test_batch_line_filter_beyond_32_bit_word_indices():
     b.check_errors()
     del lmap
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize('dtype', ['float32', 'complex64'])
+@pytest.mark.parametrize('P,rows', [(1, 1), (3, 2047), (3, 2048), (2, 9001), (20, 2048), (70, 2050), (65, 63), (64, 64)])
+def test_batched_connectivity_at_its_rules_agrees_with_lookups(P, rows, dtype):
+    """32-bit cached products at the edges of their rules (problems of 64 and 2,048 rows, few and many tiles),
+    dense and sparse problems side by side: the bits of the matrix-free product."""
+    import torch
+    from rqutils_gb300.batch import BatchedSQD
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    from rqutils_gb300.workloads import random_pauli_masks
+    rng = np.random.default_rng(10 * P + rows)
+    hams, states = [], []
+    for n in (max(6, int(np.ceil(np.log2(rows + 1)))), 20):
+        labels, coeffs = random_pauli_masks(rng, n, 150)
+        if dtype == 'float32':
+            labels = [s if s.count('Y') % 2 == 0 else s.replace('Y', 'X') for s in labels]
+        hams.append((n, PauliSumXZ.from_paulisum((labels, coeffs), force_real=True, add_padding=True)))
+    pick = [hams[p % 2] for p in range(P)]
+    states = [np.sort(rng.choice(1 << n, size=rows, replace=False)).astype(np.uint64) for n, _ in pick]
+    conn = BatchedSQD([h for _, h in pick], states, cache_level=(1, 0))
+    free = BatchedSQD([h for _, h in pick], states)
+    x = torch.randn(conn.D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(P))
+    assert torch.equal(conn.matvec(x), free.matvec(x))
