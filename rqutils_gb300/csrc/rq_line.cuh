@@ -308,15 +308,22 @@ inline int line_lanes_log2(const rq_subspace_t &S, int J, int sms) {
 template <int FM>
 inline bool line_small(int J) { return J * line_key_bytes<FM>() <= 16 * 1024; }
 
-// Whether the lanes resolve their own hits, in 32-bit arithmetic: dense subspaces with more rows than are
-// resident with the queue.  Their rows have many hits each, and about as many as their neighbours.  The
-// prefix shift tells them, as above: shift b is about 2^(lwbits - 5) states among 2^b neighbours.  complex64,
+// Dense subspaces, whose rows have many hits each and about as many as their neighbours.  The prefix shift
+// tells them, as above: shift b is about 2^(lwbits - 5) states among 2^b neighbours.
+constexpr int kDenseShift = 7;  // for lines of 2^8 bits
+inline bool dense(const rq_subspace_t &S) {
+    return S.lookup == RQ_LOOKUP_HASH && S.lmap && S.lshift <= kDenseShift + S.lwbits - 8;
+}
+
+// more of them than are resident with the queue
+inline bool even_rows(const rq_subspace_t &S, int sms) { return S.D > (int64_t)sms * kLineThreads && dense(S); }
+
+// Whether the lanes resolve their own hits, in 32-bit arithmetic.  complex64,
 // queue against own hits: 20 qubits, 157,000 rows (shift 5) 131 us against 86; 23 qubits, 676,000 rows
 // (6) 514 against 435; 24 qubits, 500,000 rows (7) 126 against 121, 250,000 (8) 50 against 54; 32 qubits,
 // 400,000 low-energy rows (13) 69 against 92; 21 qubits, 120,000 rows, all resident, 51 against 53.
-constexpr int kOwnHitsShift = 7;  // for lines of 2^8 bits
 inline bool own_hits(const rq_subspace_t &S, int J, int sms) {
-    return S.D > (int64_t)sms * kLineThreads && S.lshift <= kOwnHitsShift + S.lwbits - 8 && line_small<kFiltNone>(J);
+    return even_rows(S, sms) && line_small<kFiltNone>(J);
 }
 
 // whether there is a line filter (rq_subspace_build fills it for hash lookups only, whatever lmap holds

@@ -713,8 +713,9 @@ k_matvec_csr(const rq_operator_t op, const V *__restrict__ x, V *__restrict__ y,
 // A thread per row, for 64-bit rows that are many: a row's owner adds them one by one either way, and with
 // full warps of owners the FP64 pipe does more a cycle than in tiles.  float64: 400,000 rows of 4 elements
 // 15.2 us against 18.2 with tiles (28.6 with each product rounded before its addition), 700,000 rows of 7
-// 40 against 42; 20,000 rows of 34 44 against 26.  complex128, long rows only (150,001 of 83: 750 us
-// against 805 with tiles, whose buffer a dozen rows fill).
+// 40 against 42; 20,000 rows of 34 44 against 26.  complex128, long rows only, whose tiles are low:
+// 150,001 of 83 750 us against 805 with tiles, 352,000 of 39 in a dense subspace 236 against 274 (150,000 of
+// 40 that differ 282 against 213).
 constexpr int64_t kCsrRowsD = int64_t(1) << 15;
 template <typename V, typename VV>
 __global__ void __launch_bounds__(kThreads)
@@ -744,10 +745,10 @@ void run_csr(const rq_operator_t &op, const V *x, V *y, cudaStream_t st, const i
     const bool many = std::is_same<V, double>::value && D >= kCsrRowsD;
     if (rows_short(D, op.nnz) && !many) {
         k_matvec_csr<V, VV, true><<<grid_short(D), kThreads, 0, st>>>(op, x, y, 0, gate, gate2);
-    } else if (many || (sizeof(V) == 16 && avg > 48. && D > 65536)) {
+    } else if (many || (sizeof(V) == 16 && D > 65536 && avg > (dense(op.sub) ? 32. : 48.))) {
         k_matvec_csr_rows<V, VV><<<grid_rows(D), kThreads, 0, st>>>(op, x, y, gate, gate2);
     } else {
-        const int rows = tile_rows<CsrTerm<V>>(D, op.nnz, sm_count());
+        const int rows = tile_rows<CsrTerm<V>>(D, op.nnz, sm_count(), even_rows(op.sub, sm_count()));
         k_matvec_csr<V, VV, false><<<grid_tiles(D, rows), kThreads, 0, st>>>(op, x, y, rows, gate, gate2);
     }
 }
@@ -903,7 +904,7 @@ int matvec_typed(const rq_operator_t &op, const void *x, void *y, void *scratch,
                 k_matvec_conn<V, true><<<grid_short(op.sub.D), kThreads, 0, st>>>(
                     op, static_cast<const V *>(x), static_cast<V *>(y), 0, gate, gate2);
             } else {
-                const int rows = tile_rows<RowTerm<V>>(op.sub.D, op.nnz, sm_count());
+                const int rows = tile_rows<RowTerm<V>>(op.sub.D, op.nnz, sm_count(), even_rows(op.sub, sm_count()));
                 k_matvec_conn<V, false><<<grid_tiles(op.sub.D, rows), kThreads, 0, st>>>(
                     op, static_cast<const V *>(x), static_cast<V *>(y), rows, gate, gate2);
             }

@@ -97,6 +97,7 @@ struct RowTerm<V, true> {  // the complex product
     using A = CAcc<R>;
     static constexpr int kTileBytes = 16 * 1024;  // products of one pass over a tile (below)
     static constexpr bool kPair = false;          // a product takes two values
+    static constexpr int kEvenElems = 0;          // with kPair: elements of a tile of even rows
     static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const V *x, int64_t m) {
         const cx<R> d = group_diag<R>(T, g, s), v = VT<V>::ld(x, m);
         // a real diagonal times a finite value: the products with zero change nothing
@@ -121,6 +122,7 @@ struct RowTerm<float, false> {  // the product, rounded on its own
     // a 28-qubit molecule, 40 each: 525 against 188; 200,000 Hubbard rows of 2: 9.5 against 8.5)
     static constexpr int kTileBytes = 8 * 1024;
     static constexpr bool kPair = false;
+    static constexpr int kEvenElems = 0;
     static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const float *x, int64_t m) {
         return mul_rn(group_diag_re<float>(T, g, s), x[m]);
     }
@@ -137,6 +139,7 @@ struct RowTerm<double, false> {  // both factors: the row's owner adds their exa
     using A = Acc<double>;
     static constexpr int kTileBytes = 16 * 1024;
     static constexpr bool kPair = true;
+    static constexpr int kEvenElems = 2048;
     static __device__ __forceinline__ P product(const rq_terms_t &T, int g, uint64_t s, const double *x, int64_t m) {
         return {group_diag_re<double>(T, g, s), x[m]};
     }
@@ -162,6 +165,7 @@ struct CsrTerm<float> {
     using A = Acc<float>;
     static constexpr int kTileBytes = 16 * 1024;
     static constexpr bool kPair = true;
+    static constexpr int kEvenElems = 4096;
     static __device__ __forceinline__ P of(float d, float x) {
         const float p = mul_rn(d, x);
         return {p, fmaf(d, x, -p)};
@@ -197,13 +201,14 @@ __host__ __device__ constexpr int tile_elems() {
 // the dense rows of a sample, which stand together, would keep a few blocks busy with many passes after
 // the others: such tiles fill four fifths and are at least eight per SM (low-energy samples of a
 // 28-qubit molecule, 40,000 rows of 32 elements, float64 CONN 306 us with 64 rows a tile and 122 with 16,
-// float32 CSR 38 and 22 with 32; 24,000 uniform rows of 22, float64 CSR, 12.9 us with 8, 8.9 with 16).
+// float32 CSR 38 and 22 with 32).  `even` rows (large dense subspaces) take two passes instead, for full warps of
+// row owners (23 qubits, 676,000 rows of 56, float64 CONN: 759 us with 8 rows a tile, 533 with 32).
 constexpr double kLongRow = 12.;
 template <typename RT>
-inline int tile_rows(int64_t D, int64_t nnz, int sms) {
+inline int tile_rows(int64_t D, int64_t nnz, int sms, bool even = false) {
     const double avg = (double)nnz / (double)D;
-    const bool cut = RT::kPair && avg > kLongRow;
-    const double fill = (cut ? 0.8 : 1.) * tile_elems<RT>();
+    const bool cut = RT::kPair && avg > kLongRow && !even;
+    const double fill = RT::kPair && even ? RT::kEvenElems : (cut ? 0.8 : 1.) * tile_elems<RT>();
     int r = kTileRows;
     while (r > (cut ? 8 : 16) && (r * avg > fill || (D + r - 1) / r < (cut ? 8 : 2) * sms)) r >>= 1;
     return r;
