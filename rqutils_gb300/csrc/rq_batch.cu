@@ -451,7 +451,7 @@ inline bool batch_conn_rows(const rq_batch_t &B) {
 
 // Rows of a tile of 32-bit values.  Problems differ in their rows' lengths; where they are large, the tiles
 // of a dense problem stand together and keep their blocks busy after the others, so tiles are at most 128
-// rows and three eighths of a full buffer, and at least four per SM (complex64: 16 problems, 195,270 rows of
+// rows and 768 elements, and at least four per SM (complex64: 16 problems, 195,270 rows of
 // 4 elements 52 us with 256 rows, 32 with 128; 40 problems, 592,748 rows of 8 176 with 256, 117 with 64; a
 // thread per row 45 and 123).  Small problems even out: 2,000 of 300 rows 14 us with 256, 20 with 128.
 constexpr int64_t kLargeProblem = 2048;
@@ -461,7 +461,7 @@ inline int batch_tile_rows(const rq_batch_t &B, int sms) {
     if (sizeof(typename VT<V>::R) == 8 || B.D < kLargeProblem * B.P) return tile_rows<RT>(B.D, B.nnz, sms);
     const double avg = (double)B.nnz / (double)B.D;
     int r = kTileRows / 2;
-    while (r > 16 && (r * avg > 0.375 * tile_elems<RT>() || (B.D + r - 1) / r < 4 * sms)) r >>= 1;
+    while (r > 16 && (r * avg > 768. || (B.D + r - 1) / r < 4 * sms)) r >>= 1;
     return r;
 }
 
