@@ -412,7 +412,7 @@ int rq_mlp_sample(const uint64_t *states, int64_t D, const double *U, const floa
 int rq_mlp_fwd(const rq_mlp_t *m, int64_t rows, const uint16_t *x, float *out, void *ws,
                void *stream);
 /* out[rows][2] = f(x) without keeping the activations for rq_mlp_bwd (inference: one kernel, which
- * writes only its error flag to ws). */
+ * writes only the error flags to ws: 16 bytes are enough). */
 int rq_mlp_infer(const rq_mlp_t *m, int64_t rows, const uint16_t *x, float *out, void *ws,
                  void *stream);
 /* dout[rows][2] of the weighted loss mean_i w_i ((o0 - a_i)^2 + softplus(-s_i o1)); the loss

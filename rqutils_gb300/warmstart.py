@@ -59,6 +59,7 @@ class WarmStartMLP:
         L.check(L.lib().rq_mlp_sync(ctypes.byref(self.c), L.stream_ptr()), 'rq_mlp_sync')
         self.t = 0
         self._ws = None
+        self._infer_ws = torch.zeros(16, dtype=torch.uint8, device=dev)  # the error flags alone
 
     # ------------------------------------------------------------------------------------------
     def views(self):
@@ -90,9 +91,10 @@ class WarmStartMLP:
         return out
 
     def infer(self, x, out=None, stream=None):
-        """out (rows, 2) FP32 for BF16 features x (rows, 64), keeping no activations."""
+        """out (rows, 2) FP32 for BF16 features x (rows, 64), keeping no activations (and needing
+        no workspace for them: 0.7 GB for 2^18 rows)."""
         rows = x.shape[0]
-        ws = self.workspace(rows)
+        ws = self._infer_ws
         if out is None:
             out = torch.empty((rows, 2), dtype=torch.float32, device=self.device)
         L.check(L.lib().rq_mlp_infer(ctypes.byref(self.c), rows, L.ptr(x), L.ptr(out), L.ptr(ws),
@@ -135,12 +137,13 @@ class WarmStartMLP:
     def check_errors(self):
         """Raise if a kernel of any call since the last check reported an error (a wait that ran out:
         its results, and the steps taken from them, are incomplete)."""
-        if self._ws is not None:
-            sticky = self._ws[4:8].view(torch.int32)
-            flag = int(sticky.item())
-            if flag:
-                sticky.zero_()
-                raise L.RqError(flag, 'an MLP kernel reported an error')
+        for ws in (self._infer_ws, self._ws):
+            if ws is not None:
+                sticky = ws[4:8].view(torch.int32)
+                flag = int(sticky.item())
+                if flag:
+                    sticky.zero_()
+                    raise L.RqError(flag, 'an MLP kernel reported an error')
 
     # ------------------------------------------------------------------------------------------
     def fit(self, states, U, psi, steps=2000, batch=65536, lr=2e-3, lr_min=1e-4, seed=1,

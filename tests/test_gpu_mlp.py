@@ -330,3 +330,26 @@ def test_errors_of_earlier_steps_are_reported():
         m.check_errors()
     m.infer(x)
     m.check_errors()
+
+
+def test_inference_needs_no_training_workspace():
+    """predict() on many states holds its features and outputs, not the activations of a training step
+    (five rows x 256 BF16 arrays), and its error flag is reported."""
+    import torch
+    from rqutils_gb300 import _lib as L
+    from rqutils_gb300.warmstart import WarmStartMLP
+    m = WarmStartMLP(seed=1)
+    rows = 1 << 18
+    s = torch.arange(rows, dtype=torch.int64, device='cuda')
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    m.predict(s, 4.)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before <= rows * (128 + 8) + (1 << 22)
+    m.check_errors()
+    m._infer_ws[4:8].view(torch.int32).fill_(L.E_CUDA)
+    m.predict(s, 4.)
+    with pytest.raises(L.RqError):
+        m.check_errors()
+    m.check_errors()
