@@ -343,3 +343,38 @@ def test_batched_connectivity_at_its_rules_agrees_with_lookups(P, rows, dtype):
     free = BatchedSQD([h for _, h in pick], states)
     x = torch.randn(conn.D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(P))
     assert torch.equal(conn.matvec(x), free.matvec(x))
+
+
+@pytest.mark.parametrize('dtype', ['float32', 'complex64', 'complex128'])
+@pytest.mark.parametrize('rows', [300, 9000])
+def test_batches_stream_their_group_keys(rows, dtype):
+    """Problems of 1023, 1024, 1025 and 2100 groups without the x = 0 group (their keys pass through shared
+    memory 1,024 at a time) with small ones beside them in the same tiles."""
+    import torch
+    from oracle.paulis import from_paulisum as o_from
+    from oracle.sqd import matvec_nocache
+    from rqutils_gb300.batch import BatchedSQD
+    from rqutils_gb300.paulis.symplectic import PauliSumXZ
+    rng = np.random.default_rng(rows)
+    n, hams, states = 14, [], []
+    for p, J in enumerate((3, 1023, 1024, 7, 1025, 2100, 1)):
+        masks = rng.choice(np.arange(1, 1 << n), size=J, replace=False)
+        labels = ['I' * n] if p % 2 else []
+        for m in masks:
+            x = ['XY'[rng.integers(2)] if m >> (n - 1 - k) & 1 else 'IZ'[rng.integers(2)] for k in range(n)]
+            if dtype == 'float32' and x.count('Y') % 2:
+                x[x.index('Y')] = 'X'
+            labels.append(''.join(x))
+        hams.append((labels, rng.normal(size=len(labels))))
+        states.append(np.sort(rng.choice(1 << n, size=rows - 7 * p, replace=False)).astype(np.uint64))
+    ps = [PauliSumXZ.from_paulisum(h, force_real=True, add_padding=True) for h in hams]
+    b = BatchedSQD(ps, states)
+    assert [int(j) for j in np.diff(b.gofs_host)] == [3, 1024, 1024, 8, 1025, 2101, 1]
+    x = torch.randn(b.D, dtype=getattr(torch, dtype), device='cuda', generator=torch.Generator('cuda').manual_seed(rows))
+    y = b.matvec(x)
+    b.check_errors()
+    assert torch.equal(BatchedSQD(ps, states, line_filter=False, presence=False).matvec(x), y)
+    if dtype == 'complex128' and rows == 300:
+        for p in range(b.P):
+            ref = matvec_nocache(x[b.rows(p)].cpu().numpy(), o_from(hams[p], force_real=True), states[p])
+            np.testing.assert_allclose(y[b.rows(p)].cpu().numpy(), ref, rtol=1e-11, atol=1e-11)
