@@ -771,10 +771,6 @@ template <typename R>
 __device__ __forceinline__ double s_round(double a) { return (double)(R)a; }
 template <typename R>
 __device__ __forceinline__ double2 s_round(double2 a) { return make_double2((double)(R)a.x, (double)(R)a.y); }
-template <typename R>
-__device__ __forceinline__ cx<R> s_coef(double a) { return {(R)a, (R)0}; }
-template <typename R>
-__device__ __forceinline__ cx<R> s_coef(double2 a) { return {(R)a.x, (R)a.y}; }
 template <typename S>
 __device__ __forceinline__ S s_of(double re);
 template <>

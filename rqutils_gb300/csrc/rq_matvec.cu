@@ -469,9 +469,6 @@ k_conn_count(const rq_operator_t op, int64_t *__restrict__ rowcnt, int *err) {
     }
 }
 
-// Diagonal of group g for state s from the global term arrays (CONN mode and CSR values).
-
-
 template <typename V, int LK, int KB>
 __global__ void __launch_bounds__(kThreads)
 k_conn_fill(const rq_operator_t op, const int64_t *__restrict__ rowptr, int32_t *__restrict__ col,

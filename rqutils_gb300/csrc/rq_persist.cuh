@@ -491,7 +491,9 @@ struct Coef {
 
 // Gram pass and Rayleigh-Ritz: <y,Ax> <p,Ax> <p,Ay> <x,Ax> <y,Ay> <p,Ap> <x,p> <y,p> |p|^2, then the
 // coefficients of x' = riu (k0 x + s) and y' = rit (s k0 / |s| - x |s|), s = k1 y + k2 p, as two
-// combinations of (x, y, p); their norms follow from the products at hand.
+// combinations of (x, y, p); their norms follow from the products at hand.  Nothing cancels in them: x, y
+// and p are orthonormal to rounding (a zero y or p carries no weight: then ss = 0, and 1 / 0 as with sums
+// of squares), so |s|^2 = ss is a sum of squares and |t|^2, |u|^2 are |k0|^2 + ss to rounding, and |k| = 1.
 template <typename V, bool FAST>
 __device__ __forceinline__ bool gram_step(const PSeg &seg, const Vecs<V> &v) {
     using R = typename VT<V>::R;
