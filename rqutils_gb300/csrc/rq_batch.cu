@@ -308,8 +308,8 @@ k_batch_matvec_free(const rq_batch_t B, const V *__restrict__ x, V *__restrict__
 // The same with a line filter, through line_rows (rq_line.cuh): a block takes a tile of consecutive
 // rows, problem by problem, with that problem's group keys in shared memory, probes every group (the
 // sector stage above costs more than the probes it spares, also when the filter does not fit in L2) and
-// resolves hits through the warp's queue.  complex64: 48 problems, 780,729 rows: 486 -> 189 us; 256
-// problems, 10.2 M rows (filter of 268 MB): 7.25 -> 3.34 ms.
+// resolves hits through the warp's queue.  complex64: 48 problems, 780,729 rows: 486 -> 187 us; 256
+// problems, 10.2 M rows (filter of 268 MB), L2 flushed before each product: 10.1 -> 4.74 ms.
 template <typename V>
 struct UseBatchProduct {
     using RT = RowTerm<V>;
